@@ -330,6 +330,130 @@ def run(s):
     return dict(out=out.detach(), dq=dq, dk=dk, dv=dv)
 
 
+# ---------------------------------------------------------------- the results in 64 bits --
+
+def _attend(q, k, v, blocks, tok, dout=None):
+    """Attention of query blocks over lists of key blocks, in 64 bits: q (g, n, 16, 128) of n tokens at
+    positions tok (g, n), k / v (l, 128), blocks (g, m) with -1 for unused.  Returns the outputs and,
+    with dout, (dq, dk, dv) as well."""
+    g, n = tok.shape
+    pos = (blocks[:, :, None] * BLOCK + torch.arange(BLOCK, device=DEV)).flatten(1)             # (g, m * 64)
+    real = (blocks >= 0).repeat_interleave(BLOCK, 1) & (pos < k.shape[0])
+    pos = pos.clamp(0, k.shape[0] - 1).long()
+    kg, vg = k[pos], v[pos]
+    scale = D ** -0.5
+    s = (q.reshape(g, n * GROUP, D) @ kg.mT).mul_(scale).view(g, n, GROUP, -1)
+    seen = real[:, None, :] & (pos[:, None, :] <= tok[:, :, None])
+    p = s.masked_fill_(~seen[:, :, None, :], -math.inf).softmax(-1).nan_to_num_(0.0).view(g, n * GROUP, -1)
+    out = p @ vg
+    if dout is None:
+        return out.view_as(q), None
+    do = dout.reshape(g, n * GROUP, D)
+    ds = (do @ vg.mT).sub_((do * out).sum(-1, keepdim=True)).mul_(p).mul_(scale)
+    dk, dv = torch.zeros_like(k), torch.zeros_like(v)
+    dk.index_add_(0, pos.flatten(), (ds.mT @ q.reshape(g, n * GROUP, D)).flatten(0, 1))
+    dv.index_add_(0, pos.flatten(), (p.mT @ do).flatten(0, 1))
+    return out.view_as(q), ((ds @ kg).view_as(q), dk, dv)
+
+
+def _exact_packed(s, grads):
+    """Block-sparse (s["idx"], shared by the tokens of a query block) or dense attention of packed
+    sequences: out (and dq, dk, dv)."""
+    q, k, v = (s[n].detach().double() for n in "qkv")
+    dout = s["dout"].double() if grads else None
+    out, dq, dk, dv = (torch.zeros_like(t) for t in (q, q, k, v))
+    base = 0
+    for l in s["lens"]:
+        n_blk = (l + BLOCK - 1) // BLOCK
+        for h in range(k.shape[1]):
+            heads = slice(h * GROUP, (h + 1) * GROUP)
+            part = max(1, 65536 // (s["idx"].shape[-1] * BLOCK if "idx" in s else n_blk * BLOCK))
+            for b0 in range(0, n_blk, part):
+                full = (min(b0 + part, n_blk) if l % BLOCK == 0 else min(b0 + part, n_blk - 1)) - b0
+                spans = [(b0, full, BLOCK)] if full > 0 else []
+                if b0 + full < min(b0 + part, n_blk):
+                    spans.append((n_blk - 1, 1, l % BLOCK))                 # the ragged last query block
+                for first, g, n in spans:
+                    rows = slice(base + first * BLOCK, base + first * BLOCK + g * n)
+                    tok = torch.arange(first * BLOCK, first * BLOCK + g * n, device=DEV).view(g, n)
+                    if "idx" in s:
+                        blocks = s["idx"][h, rows][::n].long()
+                    else:
+                        blocks = torch.arange(first + g, device=DEV).expand(g, -1)
+                    o, d = _attend(q[rows, heads].view(g, n, GROUP, D), k[base:base + l, h], v[base:base + l, h], blocks, tok,
+                                   dout[rows, heads].view(g, n, GROUP, D) if grads else None)
+                    out[rows, heads] = o.view(g * n, GROUP, D)
+                    if grads:
+                        dq[rows, heads] = d[0].view(g * n, GROUP, D)
+                        dk[base:base + l, h] += d[1]
+                        dv[base:base + l, h] += d[2]
+        base += l
+    return dict(out=out, dq=dq, dk=dk, dv=dv) if grads else dict(out=out)
+
+
+def _exact_kvcache(s):
+    """Append at the end, rotation of the query and of the new key, attention over the listed blocks."""
+    page, out = s["k_cache"].shape[1], []
+
+    def rotate(x, cos, sin):                        # neighbouring pairs
+        a, b = x[..., 0::2], x[..., 1::2]
+        return torch.stack([a * cos - b * sin, a * sin + b * cos], -1).flatten(-2)
+    for i, n in enumerate(s["lens"].tolist()):
+        cos, sin = s["cos"][n].double(), s["sin"][n].double()
+        pages = s["table"][i, :n // page + 1].long()
+        k, v = (s[c][pages].flatten(0, 1)[:n + 1].double() for c in ("k_cache", "v_cache"))
+        k[n], v[n] = rotate(s["k"][i, 0].double(), cos, sin), s["v"][i, 0].double()
+        q = rotate(s["q"][i, 0].double(), cos, sin).view(-1, 1, 1, GROUP, D)
+        tok = torch.full((1, 1), n, device=DEV)
+        out.append(torch.cat([_attend(q[h], k[:, h], v[:, h], s["idx"][i, h].long(), tok)[0].view(GROUP, D)
+                              for h in range(k.shape[1])]))
+    return dict(out=torch.stack(out)[:, None], k=None, v=None)
+
+
+def _exact_scores(s):
+    """Probabilities of the compressed keys, normalised over the visible keys of the row sums and summed
+    over the heads of a group."""
+    def visible(l, keys, stride):
+        t = torch.arange(1, l + 1, device=DEV)
+        off = keys - (l - stride + 1) // stride if l >= stride - 1 else keys
+        return (t.div(stride, rounding_mode="floor") - 1 + off).clamp(0, keys)
+    hk = s["kc"].shape[1]
+    scores = torch.zeros(hk, s["q"].shape[0], _windows(s["max_len"]), device=DEV, dtype=torch.float64)
+    base = 0
+    cu_c, cu_v = s["cu_c"].tolist(), s["cu_v"].tolist()
+    for i, l in enumerate(s["lens"]):
+        kc, kv = s["kc"][cu_c[i]:cu_c[i + 1]].double(), s["kv"][cu_v[i]:cu_v[i + 1]].double()
+        see = visible(l, len(kc), 16)
+        see_v = visible(l, len(kv), 16 if len(kv) == len(kc) else 64)
+        for h in range(hk):
+            for t0 in range(0, l, 1024):
+                rows = slice(t0, min(t0 + 1024, l))
+                q = s["q"][base + t0:base + rows.stop, h * GROUP:(h + 1) * GROUP].double() * D ** -0.5
+                hid = torch.arange(len(kc), device=DEV) >= see[rows, None]
+                hid_v = torch.arange(len(kv), device=DEV) >= see_v[rows, None]
+                lse = (q @ kv[:, h].mT).masked_fill_(hid_v[:, None], -math.inf).logsumexp(-1, keepdim=True)
+                p = (q @ kc[:, h].mT).sub_(lse).exp_().nan_to_num_(0.0, 0.0, 0.0).masked_fill_(hid[:, None], 0.0)
+                scores[h, base + t0:base + rows.stop, :len(kc)] = p.sum(1)
+        base += l
+    return dict(scores=scores, pooled=None, idx=None, mask=None)
+
+
+def exact(case, seed):
+    """What `run` returns, in 64 bits.  None for the calls whose attention follows from block lists that
+    they choose themselves, and for integers and copied rows."""
+    kind = case["kind"]
+    dense = kind in ("prefill", "train_layer") and max(_lens(case)) <= case["dense_len"]
+    if kind not in ("train", "kvcache", "select") and not dense:
+        return None
+    s = prepare(case, seed)
+    if kind == "kvcache":
+        return _exact_kvcache(s)
+    if kind == "select":
+        return _exact_scores(s)
+    got = _exact_packed(s, kind != "prefill")
+    return dict(got, k=None, v=None, kc=None, seqlens=None, n_comp=None) if kind == "prefill" else got
+
+
 # ----------------------------------------------------------------------- work and tolerance --
 
 def _pairs(start, end, topk):
