@@ -1,5 +1,6 @@
 // Selection kernels: 1-D max-pool of stage-1 scores to 64-token block scores, and per-query
-// top-k of block scores.  Both are HBM-bound: one warp per row, 16-byte loads, warp shuffles.
+// top-k of block scores.  One warp per row, 16-byte loads, warp shuffles; the pool is bound by HBM, the
+// top-k by instruction issue.
 #include "common.cuh"
 
 namespace ifv2 {
@@ -157,7 +158,8 @@ int launch_pool(const PoolParams& p, cudaStream_t st) {
 // of 8 elements, so element index order is (iteration, lane, slot)).  The k-th largest value is
 // found by bisection over the 16-bit ordered key space; each probe counts `x >= candidate`
 // with native packed compares.  Entries above the threshold are all taken, entries equal to it
-// are taken lowest index first, and output slots come from one packed warp prefix scan.
+// are taken lowest index first; only ties and block lists need a warp prefix scan (byte counters,
+// four iterations to a register).
 
 struct TopkParams {
   const void* score;
@@ -187,10 +189,6 @@ template <> struct Pack<__nv_bfloat16> {
   static __device__ __forceinline__ T2 splat(uint16_t bits) {
     return __halves2bfloat162(__ushort_as_bfloat16(bits), __ushort_as_bfloat16(bits));
   }
-  static __device__ __forceinline__ T2 zero() { return __float2bfloat162_rn(0.f); }
-  static __device__ __forceinline__ int hsum(T2 v) {
-    return (int)(__bfloat162float(v.x) + __bfloat162float(v.y));
-  }
   // 0xFFFF in the half of the word whose comparison holds
   static __device__ __forceinline__ uint32_t ge_mask(T2 a, T2 b) { return __hge2_mask(a, b); }
   static __device__ __forceinline__ uint32_t gt_mask(T2 a, T2 b) { return __hgt2_mask(a, b); }
@@ -201,36 +199,46 @@ template <> struct Pack<__half> {
   static __device__ __forceinline__ T2 splat(uint16_t bits) {
     return __halves2half2(__ushort_as_half(bits), __ushort_as_half(bits));
   }
-  static __device__ __forceinline__ T2 zero() { return __float2half2_rn(0.f); }
-  static __device__ __forceinline__ int hsum(T2 v) {
-    return (int)(__half2float(v.x) + __half2float(v.y));
-  }
   static __device__ __forceinline__ uint32_t ge_mask(T2 a, T2 b) { return __hge2_mask(a, b); }
   static __device__ __forceinline__ uint32_t gt_mask(T2 a, T2 b) { return __hgt2_mask(a, b); }
   static __device__ __forceinline__ uint32_t eq_mask(T2 a, T2 b) { return __heq2_mask(a, b); }
 };
 
-// Output stores are guarded by the capacity of the row: a slot outside [0, k) is never written
-// (-DIFV2_TOPK_CHECK additionally reports such a slot).
-#ifdef IFV2_TOPK_CHECK
-#define IFV2_TOPK_STORE(pos, val)                                                               \
-  do {                                                                                          \
-    if (o != nullptr && (unsigned)(pos) < (unsigned)k_cap) o[(pos)] = (val);                    \
-    else if (o != nullptr) printf("topk: slot %d outside [0,%d) lane %d k_sel %d need %d exact %d bq %d\n", (int)(pos), k_cap, \
-                lane, k_sel, need, (int)exact, bq);                                             \
-  } while (0)
-#else
-#define IFV2_TOPK_STORE(pos, val)                                  \
-  do {                                                             \
-    if (o != nullptr && (unsigned)(pos) < (unsigned)k_cap) o[(pos)] = (val);   \
-  } while (0)
-#endif
+// Bits of the packed 0xFFFF / 0 masks of one iteration's four pairs, slot order.
+__device__ __forceinline__ uint32_t slot_bits(uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+  const uint32_t t = (m0 & 0x00020001u) | (m1 & 0x00080004u) | (m2 & 0x00200010u) | (m3 & 0x00800040u);
+  return (t | (t >> 16)) & 0xFFu;
+}
+
+// Exclusive prefix over the lanes of kRegs registers of four byte counters (at most 8 each, so the
+// largest prefix, 31 * 8, fits its byte); totals[i] is the warp's sum of counter i.
+template <int kRegs, int kCount>
+__device__ __forceinline__ void scan_bytes(uint32_t (&c)[kRegs], int (&totals)[kCount], int lane) {
+#pragma unroll
+  for (int r = 0; r < kRegs; ++r) {
+    const uint32_t mine = c[r];
+    uint32_t e = __shfl_up_sync(0xFFFFFFFFu, mine, 1);
+    if (lane == 0) e = 0u;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, e, d);
+      if (lane >= d) e += up;
+    }
+    const uint32_t e31 = __shfl_sync(0xFFFFFFFFu, e, 31), m31 = __shfl_sync(0xFFFFFFFFu, mine, 31);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (4 * r + i < kCount)
+        totals[4 * r + i] = (int)(((e31 >> (8 * i)) & 0xFFu) + ((m31 >> (8 * i)) & 0xFFu));
+    c[r] = e;
+  }
+}
 
 // Selection over the first kIts iterations (256 entries each) of a row held in registers; the
 // iteration count is a template parameter so that the probe and emit loops are straight-line
-// code.  Returns the number of entries emitted, or -1 when a restricted selection turns out not
-// to be equivalent to the full one.
-template <typename T, int kPairs, int kIts>
+// code.  kList: the block list is written as well, which needs an output slot per entry; the mask
+// alone needs no prefix scan unless entries tie at the threshold.  Returns the number of entries
+// taken, or -1 when a restricted selection turns out not to be equivalent to the full one.
+template <typename T, int kPairs, int kIts, bool kList>
 __device__ __forceinline__ int topk_row(const typename Pack<T>::T2 (&v)[kPairs],
                                         typename Pack<T>::T2 tail2, bool restricted, int k_sel,
                                         int bq, int lane, int32_t* o, int k_cap,
@@ -241,23 +249,23 @@ __device__ __forceinline__ int topk_row(const typename Pack<T>::T2 (&v)[kPairs],
   // ---- bisection for the k_sel-th largest value over ordered keys [-inf, +inf]
   uint32_t lo = bits_to_ordered(N::kNegInf), hi = bits_to_ordered(N::kPosInf) + 1u;
   bool exact = false;                     // count(x >= val(lo)) == k_sel: no tie handling needed
+  int above = 0;                          // entries known to lie at or above val(hi)
   while (hi - lo > 1u) {
     const uint32_t mid = (lo + hi) >> 1;
     const T2 c = P::splat(ordered_to_bits(mid));
-    T2 acc = P::zero();
+    // every comparison gives 0xFFFF per half that holds, and the sum of the words keeps both counts:
+    // low * 0xFFFF - high * 0x10000 = (low - high) * 0x10000 - low
+    uint32_t acc = 0u;
 #pragma unroll
-    for (int it = 0; it < kIts; ++it) {
-      if (it < kIts) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc = __hadd2(acc, __hge2(v[it * 4 + j], c));
-      }
-    }
-    const int cnt = __reduce_add_sync(0xFFFFFFFFu, P::hsum(acc));
+    for (int j = 0; j < kIts * 4; j += 2) acc += P::ge_mask(v[j], c) + P::ge_mask(v[j + 1], c);
+    const int low = (int)((0u - acc) & 0xFFFFu);
+    const int cnt = __reduce_add_sync(0xFFFFFFFFu, 2 * low - ((int)(acc + (uint32_t)low) >> 16));
     if (cnt >= k_sel) {
       lo = mid;
       if (cnt == k_sel) { exact = true; break; }
     } else {
       hi = mid;
+      above = cnt;
     }
   }
   const T2 thr = P::splat(ordered_to_bits(lo));
@@ -267,99 +275,110 @@ __device__ __forceinline__ int topk_row(const typename Pack<T>::T2 (&v)[kPairs],
     const bool bad = tm > N::to_f(thr.x);
     if (__any_sync(0xFFFFFFFFu, bad)) return -1;        // redo over the full width
   }
-  int need = 0;                           // how many entries equal to the threshold to take
-  if (!exact) {
-    T2 acc = P::zero();
+
+  // ---- slots taken, one byte per iteration
+  uint32_t taken[kIts];
+  if (exact) {
+#pragma unroll
+    for (int it = 0; it < kIts; ++it)
+      taken[it] = slot_bits(P::ge_mask(v[it * 4], thr), P::ge_mask(v[it * 4 + 1], thr),
+                            P::ge_mask(v[it * 4 + 2], thr), P::ge_mask(v[it * 4 + 3], thr));
+  } else {
+    // entries equal to the threshold are taken lowest index first until k_sel are there; the
+    // bisection ended with hi = lo + 1, so `above` counts the entries above the threshold
+    const int need = k_sel - above;
+    constexpr int kRegs = (kIts + 3) / 4;
+    uint32_t excl[kRegs];
+    int totals[kIts];
+#pragma unroll
+    for (int r = 0; r < kRegs; ++r) excl[r] = 0u;
+    uint32_t tie[kIts];
 #pragma unroll
     for (int it = 0; it < kIts; ++it) {
-      if (it < kIts) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc = __hadd2(acc, __hgt2(v[it * 4 + j], thr));
-      }
+      taken[it] = slot_bits(P::gt_mask(v[it * 4], thr), P::gt_mask(v[it * 4 + 1], thr),
+                            P::gt_mask(v[it * 4 + 2], thr), P::gt_mask(v[it * 4 + 3], thr));
+      tie[it] = slot_bits(P::eq_mask(v[it * 4], thr), P::eq_mask(v[it * 4 + 1], thr),
+                          P::eq_mask(v[it * 4 + 2], thr), P::eq_mask(v[it * 4 + 3], thr));
+      excl[it >> 2] |= (uint32_t)__popc(tie[it]) << (8 * (it & 3));
     }
-    need = k_sel - __reduce_add_sync(0xFFFFFFFFu, P::hsum(acc));
+    scan_bytes<kRegs, kIts>(excl, totals, lane);
+    int base = 0;
+#pragma unroll
+    for (int it = 0; it < kIts; ++it) {
+      int left = need - base - (int)((excl[it >> 2] >> (8 * (it & 3))) & 0xFFu);
+      uint32_t t = tie[it];
+      if (left < __popc(t)) {               // only the first `left` of this lane's ties
+        uint32_t rest = t;
+        for (; left > 0; --left) rest &= rest - 1u;
+        t ^= rest;
+      }
+      taken[it] |= t;
+      base += totals[it];
+    }
   }
 
-  // ---- emit in index order
-  int base_gt = 0, base_tie = 0;          // counts over all earlier iterations
+  // ---- packed mask: four lanes own the 32 entries of one half word; entries past the query's own
+  // block are taken (they fill list slots) but invisible
+  if (mw != nullptr) {
+    uint32_t* mh = reinterpret_cast<uint32_t*>(mw);
 #pragma unroll
-  for (int it = 0; it < kIts; ++it) {
-    if (it < kIts) {
-      uint32_t gt_bits = 0, tie_bits = 0;   // bit s: slot s of this lane's 8 elements
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const T2 pr = v[it * 4 + j];
-        const uint32_t mg = exact ? P::ge_mask(pr, thr) : P::gt_mask(pr, thr);
-        gt_bits |= ((mg & 1u) | ((mg >> 15) & 2u)) << (2 * j);
-        if (!exact) {
-          const uint32_t me = P::eq_mask(pr, thr);
-          tie_bits |= ((me & 1u) | ((me >> 15) & 2u)) << (2 * j);
-        }
-      }
-      // packed inclusive scan over lanes: low 16 bits = taken-for-sure, high 16 = ties
-      const uint32_t mine = (uint32_t)__popc(gt_bits) | ((uint32_t)__popc(tie_bits) << 16);
-      uint32_t scan = mine;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, scan, d);
-        if (lane >= d) scan += up;
-      }
-      const uint32_t total = __shfl_sync(0xFFFFFFFFu, scan, 31);
-      const uint32_t excl = scan - mine;
-      int gt_before = base_gt + (int)(excl & 0xFFFFu);
-      int tie_before = base_tie + (int)(excl >> 16);
+    for (int it = 0; it < kIts; ++it) {
       const int e0 = (it * 32 + lane) * 8;
-      // slots of this lane that the query may see (index <= bq): only those reach the mask
-      const uint32_t vis_bits = (bq >= e0 + 7) ? 0xFFu : ((bq < e0) ? 0u : ((2u << (bq - e0)) - 1u));
-      uint32_t taken = gt_bits;           // slots selected in this iteration
-      if (tie_bits == 0u) {               // the common case: walk the few set bits
-        int pos = gt_before + min(tie_before, need);
-        uint32_t sel = gt_bits;
-        while (sel) {
-          const int s = __ffs(sel) - 1;
-          sel &= sel - 1u;
-          const int idx = e0 + s;
-          IFV2_TOPK_STORE(pos, (idx <= bq) ? idx : -1);
-          ++pos;
-        }
-      } else {
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-          const bool g = (gt_bits >> s) & 1u, t = (tie_bits >> s) & 1u;
-          if (g || (t && tie_before < need)) {
-            const int pos = gt_before + min(tie_before, need);
-            const int idx = e0 + s;
-            IFV2_TOPK_STORE(pos, (idx <= bq) ? idx : -1);
-            taken |= 1u << s;
-          }
-          gt_before += g;
-          tie_before += t;
-        }
-      }
-      if (mw != nullptr) {
-        // eight lanes own the 64 consecutive entries of one mask word: OR their bytes together
-        unsigned long long wv = (unsigned long long)(taken & vis_bits) << (8 * (lane & 7));
-        wv |= __shfl_xor_sync(0xFFFFFFFFu, wv, 1);
-        wv |= __shfl_xor_sync(0xFFFFFFFFu, wv, 2);
-        wv |= __shfl_xor_sync(0xFFFFFFFFu, wv, 4);
-        const int w = it * 4 + (lane >> 3);
-        if ((lane & 7) == 0 && w < mask_words) mw[w] = wv;
-      }
-      base_gt += (int)(total & 0xFFFFu);
-      base_tie += (int)(total >> 16);
+      const uint32_t vis = (bq >= e0 + 7) ? 0xFFu : ((bq < e0) ? 0u : ((2u << (bq - e0)) - 1u));
+      uint32_t wv = (taken[it] & vis) << (8 * (lane & 3));
+      wv |= __shfl_xor_sync(0xFFFFFFFFu, wv, 1);
+      wv |= __shfl_xor_sync(0xFFFFFFFFu, wv, 2);
+      const int w = it * 8 + (lane >> 2);
+      if ((lane & 3) == 0 && w < 2 * mask_words) mh[w] = wv;
     }
   }
-  return base_gt + min(base_tie, need);
+
+  // ---- block list, in index order
+  int total = 0;
+  if (kList) {
+    constexpr int kRegs = (kIts + 3) / 4;
+    uint32_t excl[kRegs];
+    int totals[kIts];
+#pragma unroll
+    for (int r = 0; r < kRegs; ++r) excl[r] = 0u;
+#pragma unroll
+    for (int it = 0; it < kIts; ++it) excl[it >> 2] |= (uint32_t)__popc(taken[it]) << (8 * (it & 3));
+    scan_bytes<kRegs, kIts>(excl, totals, lane);
+#pragma unroll
+    for (int it = 0; it < kIts; ++it) {
+      const int e0 = (it * 32 + lane) * 8;
+      int pos = total + (int)((excl[it >> 2] >> (8 * (it & 3))) & 0xFFu);
+      uint32_t sel = taken[it];
+      while (sel) {
+        const int idx = e0 + __ffs(sel) - 1;
+        sel &= sel - 1u;
+        // (guarded by the capacity of the row: a slot outside [0, k) is never written)
+        if ((unsigned)pos < (unsigned)k_cap) o[pos] = (idx <= bq) ? idx : -1;
+        ++pos;
+      }
+      total += totals[it];
+    }
+  }
+  return total;
 }
 
-template <typename T, int kIters>
-__global__ void __launch_bounds__(kThreads, (kIters <= 8) ? 2 : 1) topk_select_kernel(const TopkParams p) {
+// Floor of x / d for a position x (rounded towards zero if negative): 32-bit wherever it fits, a
+// 64-bit division costs as many instructions as a probe of the bisection.
+__device__ __forceinline__ int block_of(int64_t x, int d) {
+  return (x == (int64_t)(int)x) ? (int)x / d : (int)(x / d);
+}
+
+// Bound by instruction issue and by the latency of the probes (a row is read once, everything else
+// happens in registers).  Over 1 M rows of 2048 blocks, mask only: 6.88 -> 2.28 ms against a form that
+// scanned the lanes once per 256 entries, counted in bf16 and walked the taken entries even where no list
+// was wanted; with the list, 65536 rows of 512 blocks: 0.112 -> 0.101 ms.
+template <typename T, int kIters, bool kList>
+__global__ void __launch_bounds__(kThreads, (kIters <= 8) ? 3 : 1) topk_select_kernel(const TopkParams p) {
   using N = Num<T>;
   using P = Pack<T>;
   using T2 = typename P::T2;
   constexpr int kPairs = kIters * 4;          // packed registers per lane
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t rows = (int64_t)p.heads * p.total_q;
   const T* score = static_cast<const T*>(p.score);
   const int n = p.n_blocks;
   const int k_eff = min(p.k, n);
@@ -367,19 +386,21 @@ __global__ void __launch_bounds__(kThreads, (kIters <= 8) ? 2 : 1) topk_select_k
   const T2 pad2 = P::splat(N::kNegInf);
   const T ninf = N::from_bits(N::kNegInf);
 
-  for (int64_t row = (int64_t)blockIdx.x * kWarps + warp; row < rows;
-       row += (int64_t)gridDim.x * kWarps) {
-    const int64_t q = row % p.total_q;
+  // (heads are an axis of the grid: splitting a row number into head and token is a 64-bit division)
+  for (int64_t head_row = (int64_t)blockIdx.y * p.total_q; head_row < p.heads * p.total_q;
+       head_row += (int64_t)gridDim.y * p.total_q)
+  for (int64_t q = (int64_t)blockIdx.x * kWarps + warp; q < p.total_q; q += (int64_t)gridDim.x * kWarps) {
+    const int64_t row = head_row + q;
     int bq;
     if (p.cu_q != nullptr) {
       const int b = find_sequence(p.cu_q, p.batch, (int)q);
       const int cl = p.cache_lens ? p.cache_lens[b] : p.cache_len;
-      bq = (int)((q - p.cu_q[b] + cl) / p.block_size);
+      bq = block_of(q - p.cu_q[b] + cl, p.block_size);
     } else {
-      bq = (int)((q + p.cache_len) / p.block_size);
+      bq = block_of(q + p.cache_len, p.block_size);
     }
     const T* x = score + row * p.row_stride;
-    int32_t* o = p.out ? p.out + row * p.k : nullptr;
+    int32_t* o = kList ? p.out + row * p.k : nullptr;
     unsigned long long* mw = p.mask ? p.mask + row * p.mask_words : nullptr;
 
     // Entries past the query's own block only ever come out as -1.  When none of them beats the
@@ -420,7 +441,13 @@ __global__ void __launch_bounds__(kThreads, (kIters <= 8) ? 2 : 1) topk_select_k
 #pragma unroll
         for (int it = 0; it < kIters; ++it) {
           const int nh = width - (it * 32 + lane) * 8;      // entries of this lane that take part
-          if (nh < 8) {
+          if (nh <= 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              tail2 = __hmax2(tail2, v[it * 4 + j]);
+              v[it * 4 + j] = pad2;
+            }
+          } else if (nh < 8) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               T2 pr = v[it * 4 + j], tl = pad2;
@@ -442,14 +469,14 @@ __global__ void __launch_bounds__(kThreads, (kIters <= 8) ? 2 : 1) topk_select_k
 #define IFV2_TOPK_CASE(I)                                                                \
         case I:                                                                          \
           if constexpr (I <= kIters)                                                     \
-            got = topk_row<T, kPairs, I>(v, tail2, restricted, k_sel, bq, lane, o, p.k,  \
-                                         mw, p.mask_words);                              \
+            got = topk_row<T, kPairs, I, kList>(v, tail2, restricted, k_sel, bq, lane, o, p.k,  \
+                                                mw, p.mask_words);                       \
           break;
         IFV2_TOPK_CASE(2) IFV2_TOPK_CASE(4) IFV2_TOPK_CASE(6)
 #undef IFV2_TOPK_CASE
         default:
-          got = topk_row<T, kPairs, kIters>(v, tail2, restricted, k_sel, bq, lane, o, p.k, mw,
-                                            p.mask_words);
+          got = topk_row<T, kPairs, kIters, kList>(v, tail2, restricted, k_sel, bq, lane, o, p.k, mw,
+                                                   p.mask_words);
           break;
       }
       if (got < 0) continue;
@@ -462,29 +489,38 @@ __global__ void __launch_bounds__(kThreads, (kIters <= 8) ? 2 : 1) topk_select_k
       break;
     }
     // unused tail (k > entries that took part, or NaN scores that no probe counts)
-    if (o != nullptr)
+    if (kList)
       for (int i = emitted + lane; i < p.k; i += 32) o[i] = -1;
   }
 }
 
+template <typename T, int kIters>
+void launch_topk_iters(const TopkParams& p, cudaStream_t st) {
+  const int64_t gy = p.heads < 65535 ? p.heads : 65535;
+  const int64_t cap = ceil_div64((int64_t)kNumSMs * 8, gy);
+  int64_t gx = ceil_div64(p.total_q, kWarps);
+  if (gx > cap) gx = cap;
+  const dim3 grid((unsigned)gx, (unsigned)gy);
+  if (p.out != nullptr)
+    topk_select_kernel<T, kIters, true><<<grid, kThreads, 0, st>>>(p);
+  else
+    topk_select_kernel<T, kIters, false><<<grid, kThreads, 0, st>>>(p);
+}
+
 template <typename T>
 int launch_topk(const TopkParams& p, cudaStream_t st) {
-  const int64_t rows = (int64_t)p.heads * p.total_q;
-  int64_t blocks = ceil_div64(rows, kWarps);
-  const int64_t cap = (int64_t)kNumSMs * 8;
-  if (blocks > cap) blocks = cap;
   if (p.n_blocks <= 256)
-    topk_select_kernel<T, 1><<<(int)blocks, kThreads, 0, st>>>(p);
+    launch_topk_iters<T, 1>(p, st);
   else if (p.n_blocks <= 512)
-    topk_select_kernel<T, 2><<<(int)blocks, kThreads, 0, st>>>(p);
+    launch_topk_iters<T, 2>(p, st);
   else if (p.n_blocks <= 1024)
-    topk_select_kernel<T, 4><<<(int)blocks, kThreads, 0, st>>>(p);
+    launch_topk_iters<T, 4>(p, st);
   else if (p.n_blocks <= 2048)
-    topk_select_kernel<T, 8><<<(int)blocks, kThreads, 0, st>>>(p);
+    launch_topk_iters<T, 8>(p, st);
   else if (p.n_blocks <= 4096)
-    topk_select_kernel<T, 16><<<(int)blocks, kThreads, 0, st>>>(p);
+    launch_topk_iters<T, 16>(p, st);
   else
-    topk_select_kernel<T, 32><<<(int)blocks, kThreads, 0, st>>>(p);
+    launch_topk_iters<T, 32>(p, st);
   return check_launch("topk_select");
 }
 

@@ -267,3 +267,25 @@ def test_topk_mask_varlen_and_attention_takes_the_mask():
     a = infllm_v2.infllmv2_attn_varlen_func(q, k, v, cu1, cu1, L, L, causal=True, topk_idx=idx)
     b = infllm_v2.infllmv2_attn_varlen_func(q, k, v, cu1, cu1, L, L, causal=True, block_mask=m)
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("n", [1, 31, 256, 257, 1025, 2048, 5000, 8192])
+@pytest.mark.parametrize("k", [1, 7, 64, 300])
+def test_topk_ties_are_taken_lowest_index_first(n, k):
+    """Rows in which the threshold value occurs far more often than it can be taken, so that the last tie
+    falls inside one lane's run of entries, with 0, 1 or many entries above it; list and mask."""
+    t = 6
+    y = torch.zeros(1, t, n)
+    y[0, 1] = float("-inf")                                  # all entries tie at -inf
+    y[0, 2, n // 2] = 1.0                                    # one above the ties
+    y[0, 3, ::5] = 2.0                                       # many, in every lane
+    y[0, 4, n // 3:] = -1.0                                  # ties at a second value once the first runs out
+    y[0, 5, : n // 2] = float("inf")
+    y = y.to(torch.bfloat16)
+    exp = oracle.topk_select(y, k, torch.full((t,), n - 1))
+    got = infllm_v2.infllmv2_topk(y.to(DEV), k, cache_len=64 * (n - 1))
+    assert torch.equal(got.cpu(), exp)
+    mask, _, idx = infllm_v2.infllmv2_topk_mask(y.to(DEV), k, 64 * n, cache_len=64 * (n - 1), return_idx=True)
+    only, _ = infllm_v2.infllmv2_topk_mask(y.to(DEV), k, 64 * n, cache_len=64 * (n - 1))
+    words = torch.from_numpy(oracle.topk_to_uint64(exp.numpy(), 64 * n, 64)[0])
+    assert torch.equal(idx.cpu(), exp) and torch.equal(mask.cpu(), words) and torch.equal(only.cpu(), words)
