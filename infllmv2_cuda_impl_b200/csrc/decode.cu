@@ -114,34 +114,66 @@ __global__ void decode_append_kernel(__nv_bfloat16* k_cache, __nv_bfloat16* v_ca
   }
 }
 
-// index of the j-th (0-based) block of the selection, scanning the mask words upward
+// The selected blocks of one (sequence, KV head), lowest first, looked up by a whole warp that takes
+// every kWarps-th of them: lane l fetches mask word 32 c + l of a chunk of words, a warp scan gives
+// the selected blocks before it, and lane i of the warp finds the i-th next block of the warp by two
+// short bisections, so that 32 look-ups cost one trip to memory.  (One thread walking the words paid a
+// chain of a load per word, 33 of them at 131072 tokens, for the count and again for every block.)
+// Every lane must make the calls and gets the same answers.
 struct BlockList {
   const unsigned long long* words;   // null = every block below nblk
   int nwords, nblk;
+  int cached;                        // lane i: block of look-up 32 n + i
   __device__ unsigned long long word(int w) const {
+    if (w >= nwords) return 0ull;
     unsigned long long x = __ldg(words + w);
     const int first = w * 64;
     if (nblk - first < 64) x &= (nblk > first) ? ((1ull << (nblk - first)) - 1ull) : 0ull;
     return x;
   }
-  __device__ int count() const {
+  __device__ int count(int lane) const {
     if (words == nullptr) return nblk;
     int n = 0;
-    for (int w = 0; w < nwords; ++w) n += __popcll(word(w));
-    return n;
+    for (int w = lane; w < nwords; w += 32) n += __popcll(word(w));
+    return __reduce_add_sync(0xFFFFFFFFu, n);
   }
-  __device__ int nth(int j) const {
-    if (words == nullptr) return j;
-    for (int w = 0; w < nwords; ++w) {
-      unsigned long long x = word(w);
-      const int c = __popcll(x);
-      if (j < c) {
-        for (int i = 0; i < j; ++i) x &= x - 1;      // drop the j lowest set bits
-        return w * 64 + __ffsll((long long)x) - 1;
+  // blocks number j, j + kWarps, ... (0-based), one per lane; -1 past the end of the mask
+  __device__ void refill(int j, int lane) {
+    const int target = j + lane * kWarps;
+    cached = -1;
+    int before = 0;
+    for (int c = 0; c * 32 < nwords && before <= j + 31 * kWarps; ++c) {
+      const unsigned long long mine = word(c * 32 + lane);
+      const int cnt = __popcll(mine);
+      int incl = cnt;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int up = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= d) incl += up;
       }
-      j -= c;
+      const int excl = incl - cnt, total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+      const bool here = target >= before && target < before + total;
+      const int r = here ? target - before : 0;
+      int src = 0;                               // last word that starts at or below block r
+#pragma unroll
+      for (int d = 16; d >= 1; d >>= 1)
+        if (__shfl_sync(0xFFFFFFFFu, excl, src + d) <= r) src += d;
+      unsigned long long x = __shfl_sync(0xFFFFFFFFu, mine, src);
+      int rank = r - __shfl_sync(0xFFFFFFFFu, excl, src), pos = 0;
+#pragma unroll
+      for (int d = 32; d >= 1; d >>= 1) {        // position of the set bit with `rank` set bits below it
+        const int low = __popcll(x & ((1ull << d) - 1ull));
+        if (rank >= low) { rank -= low; pos += d; x >>= d; }
+      }
+      if (here) cached = (c * 32 + src) * 64 + pos;
+      before += total;
     }
-    return -1;
+  }
+  // the warp's look-up number i, of block j = first + i * kWarps; look-ups come in order
+  __device__ int nth(int i, int j, int lane) {
+    if (words == nullptr) return j;
+    if ((i & 31) == 0) refill(j, lane);
+    return __shfl_sync(0xFFFFFFFFu, cached, i & 31);
   }
 };
 
@@ -175,8 +207,8 @@ decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
   const int len = (int)max(end - pad, (int64_t)0);
   const int slot = p.cache_batch_idx ? p.cache_batch_idx[b] : b;
   BlockList list{p.mask ? p.mask + ((int64_t)b * p.heads_k + h) * p.mask_words : nullptr, p.mask_words,
-                 (len + kBlockN - 1) / kBlockN};
-  const int n = list.count();
+                 (len + kBlockN - 1) / kBlockN, -1};
+  const int n = list.count(lane);
   const int per_split = (n + p.splits - 1) / p.splits;
   const int j_begin = split * per_split, j_end = min(n, j_begin + per_split);
 
@@ -251,8 +283,8 @@ decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
 
   // The warp streams its blocks as 32-key units (two per block), so that the K tile of the next
   // unit is already in flight while this unit's softmax and P.V run.
-  int j = j_begin + warp, half = 0;
-  int blk = (j < j_end) ? list.nth(j) : -1;
+  int j = j_begin + warp, half = 0, lookups = 0;
+  int blk = (j < j_end) ? list.nth(lookups++, j, lane) : -1;
   int key0 = blk * kBlockN;
   auto advance = [&](int& jj, int& hh, int& bb) -> int {          // next unit; returns its first key or -1
     if (hh == 0 && bb * kBlockN + kUnit < len) {
@@ -261,7 +293,7 @@ decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     }
     jj += kWarps;
     hh = 0;
-    bb = (jj < j_end) ? list.nth(jj) : -1;
+    bb = (jj < j_end) ? list.nth(lookups++, jj, lane) : -1;
     return bb >= 0 ? bb * kBlockN : -1;
   };
   if (blk >= 0) {

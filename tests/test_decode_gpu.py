@@ -215,3 +215,32 @@ def test_decode_full_cache_and_lengths_beyond_the_capacity():
     beyond = infllm_v2.infllmv2_attn_with_kvcache(q, kc, vc, cache_seqlens=torch.tensor(
         [cap + 1000, cap + 1, 101], dtype=torch.int32, device=DEV))
     assert torch.equal(beyond, without)
+
+
+@pytest.mark.parametrize("n_blk,picks", [
+    (2200, "word_edges"), (2200, "all"), (2100, "last"), (2049, "sparse"), (64, "all"), (65, "all"), (40, "none"),
+])
+def test_decode_block_lists(n_blk, picks):
+    """Masks of one and of several 32-word chunks, more look-ups per warp than one batch holds, empty
+    words and no block at all: the given list against the same blocks gathered into a short cache."""
+    hk, d, length = 2, 128, n_blk * 64 - 5
+    sel = {"word_edges": [0, 63, 64, 127, 1983, 1984, 2047, 2048, 2111, n_blk - 1], "all": list(range(n_blk)),
+           "last": [n_blk - 1], "sparse": list(range(3, n_blk, 101)), "none": []}[picks]
+    g = torch.Generator(device=DEV).manual_seed(n_blk)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV, dtype=torch.bfloat16)
+    q, k, v = rand(1, 1, 16 * hk, d), rand(1, n_blk * 64, hk, d), rand(1, n_blk * 64, hk, d)
+    bits = torch.zeros((n_blk + 63) // 64 * 64, dtype=torch.bool, device=DEV)
+    bits[sel] = True
+    words, _ = infllm_v2.blockmask_to_uint64(bits.expand(1, hk, 1, -1)[..., :n_blk])
+    out, lse = infllm_v2.infllmv2_attn_with_kvcache(q, k, v, cache_seqlens=length, block_mask=words, return_softmax_lse=True)
+    if not sel:
+        assert out.abs().max() == 0 and torch.isinf(lse).all()
+        return
+    pos = (torch.tensor(sel, device=DEV)[:, None] * 64 + torch.arange(64, device=DEV)).flatten()
+    pos = pos[pos < length]
+    kf, vf = k[0, pos].float(), v[0, pos].float()
+    s = torch.einsum("hgd,nhd->hgn", q.view(hk, 16, d).float(), kf) * d ** -0.5
+    ref = torch.einsum("hgn,nhd->hgd", s.softmax(-1), vf).view(1, 1, 16 * hk, d)
+    mx, mr = err_stats(out, ref)
+    assert mx <= MAX_ABS and mr <= MEAN_REL, (mx, mr)
+    assert (lse.view(hk, 16) - s.logsumexp(-1)).abs().max() < 2e-2
