@@ -86,6 +86,12 @@ int ifv2_compress_keys(const void* k, void* kc, const int32_t* cu_seqlens_k,
                        const int32_t* cu_seqlens_c, int batch, int64_t total_k, int64_t total_c,
                        int heads_k, int head_dim, int kernel_size, int kernel_stride, void* stream);
 
+/* Cumulative number of compressed keys per sequence: cu_seqlens_c[0] = 0 and cu_seqlens_c[b+1] -
+ * cu_seqlens_c[b] = (len_b - kernel)/stride + 1 full windows, 0 when len_b < kernel.  Both tables are
+ * (batch+1) int32 on the device (calc_chunks_with_stride of tests/test_stage1_compressed_lse.py:11-55). */
+int ifv2_compressed_lengths(const int32_t* cu_seqlens_k, int32_t* cu_seqlens_c, int batch, int kernel_size,
+                            int kernel_stride, void* stream);
+
 /* Decode-time update of a compressed-key cache after one token was appended to every sequence:
  * a sequence whose new length L satisfies L >= kernel and (L - kernel) % stride == 0 has completed
  * window j = (L - kernel)/stride, and kc_cache[b, j] is written; other sequences are untouched.

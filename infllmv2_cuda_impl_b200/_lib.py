@@ -28,6 +28,7 @@ SIGNATURES = {
     "ifv2_transpose_blockmask": [c_void_p, c_void_p, c_int, c_int64, c_int, c_void_p],
     "ifv2_compress_keys": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int64, c_int, c_int,
                            c_int, c_int, c_void_p],
+    "ifv2_compressed_lengths": [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "ifv2_compress_keys_append": [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int64, c_int, c_int,
                                   c_int, c_int, c_void_p],
     "ifv2_max_pooling_1d": [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int64, c_int, c_int,

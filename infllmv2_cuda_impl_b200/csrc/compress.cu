@@ -74,6 +74,39 @@ __global__ void __launch_bounds__(kThreads) compress_keys_kernel(const CompressP
   }
 }
 
+// Cumulative number of full windows per sequence, one CTA: every round of kThreads sequences is
+// scanned over the warps and then over the CTA.  Latency-bound; it stands in for a dozen launches of
+// elementwise and scan operators, which took about 50 us of a short prefill.
+__global__ void __launch_bounds__(kThreads) compressed_lengths_kernel(const int32_t* __restrict__ cu_k,
+                                                                      int32_t* __restrict__ cu_c, int batch,
+                                                                      int kernel, int stride) {
+  __shared__ long long warp_sum[kThreads / 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  long long before = 0;                        // windows of all earlier rounds
+  if (threadIdx.x == 0) cu_c[0] = 0;
+  for (int b0 = 0; b0 < batch; b0 += kThreads) {
+    const int b = b0 + threadIdx.x;
+    const long long len = b < batch ? (long long)(cu_k[b + 1] - cu_k[b]) : 0;
+    long long n = len >= kernel ? (len - kernel) / stride + 1 : 0;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const long long up = __shfl_up_sync(0xFFFFFFFFu, n, d);
+      if (lane >= d) n += up;
+    }
+    if (lane == 31) warp_sum[warp] = n;
+    __syncthreads();
+    long long total = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) {
+      if (w < warp) n += warp_sum[w];
+      total += warp_sum[w];
+    }
+    if (b < batch) cu_c[b + 1] = (int32_t)(before + n);
+    before += total;
+    __syncthreads();                           // warp_sum is free again
+  }
+}
+
 struct AppendParams {
   const __nv_bfloat16* k_cache;   // (batch, cap, heads, 128)
   __nv_bfloat16* kc_cache;        // (batch, c_cap, heads, 128)
@@ -138,6 +171,16 @@ extern "C" int ifv2_compress_keys(const void* k, void* kc, const int32_t* cu_seq
   if (blocks > cap) blocks = cap;
   compress_keys_kernel<<<(int)blocks, kThreads, 0, (cudaStream_t)stream>>>(p);
   return check_launch("compress_keys");
+}
+
+extern "C" int ifv2_compressed_lengths(const int32_t* cu_seqlens_k, int32_t* cu_seqlens_c, int batch,
+                                       int kernel_size, int kernel_stride, void* stream) {
+  IFV2_REQUIRE(batch >= 0 && kernel_size >= 1 && kernel_stride >= 1, IFV2_ERR_INVALID_ARG,
+               "compressed_lengths: bad size");
+  IFV2_REQUIRE(cu_seqlens_k && cu_seqlens_c, IFV2_ERR_INVALID_ARG, "compressed_lengths: null pointer");
+  compressed_lengths_kernel<<<1, kThreads, 0, (cudaStream_t)stream>>>(cu_seqlens_k, cu_seqlens_c, batch, kernel_size,
+                                                                      kernel_stride);
+  return check_launch("compressed_lengths");
 }
 
 extern "C" int ifv2_compress_keys_append(const void* k_cache, void* kc_cache,

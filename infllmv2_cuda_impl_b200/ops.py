@@ -265,6 +265,14 @@ def compressed_lengths(cu_seqlens_k: torch.Tensor, kernel_size: int = 32,
     """Cumulative number of compressed keys per sequence (int32, same device, no host sync):
     a sequence of length L has (L - kernel_size) // kernel_stride + 1 full windows, none when
     L < kernel_size (tests/test_stage1_compressed_lse.py:11-55, calc_chunks_with_stride)."""
+    if (cu_seqlens_k.is_cuda and cu_seqlens_k.dtype == torch.int32 and cu_seqlens_k.dim() == 1
+            and cu_seqlens_k.numel() >= 1 and kernel_size >= 1 and kernel_stride >= 1):
+        cu_seqlens_k = cu_seqlens_k.contiguous()
+        cu_c = torch.empty_like(cu_seqlens_k)
+        with torch.cuda.device(cu_c.device):
+            _lib.call("ifv2_compressed_lengths", cu_seqlens_k.data_ptr(), cu_c.data_ptr(), cu_c.numel() - 1,
+                      kernel_size, kernel_stride, _stream(cu_c.device))
+        return cu_c
     lens = (cu_seqlens_k[1:] - cu_seqlens_k[:-1]).to(torch.int64)
     n = torch.where(lens >= kernel_size, (lens - kernel_size) // kernel_stride + 1,
                     torch.zeros_like(lens))

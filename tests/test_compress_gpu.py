@@ -94,3 +94,16 @@ def test_compress_append_equals_recompute():
         full, _ = oracle.compress_keys(kcache[i, :int(lens[i])].cpu(), [0, int(lens[i])])
         assert torch.equal(kc_cache[i, :full.shape[0]].cpu(), full)
         assert (kc_cache[i, full.shape[0]:] == 0).all()
+
+
+@pytest.mark.parametrize("batch", [1, 255, 256, 257, 1000])
+@pytest.mark.parametrize("kernel,stride", [(32, 16), (128, 64), (5, 3)])
+def test_compressed_lengths(batch, kernel, stride):
+    lens = torch.randint(0, 300, (batch,), generator=torch.Generator().manual_seed(batch)).tolist()
+    got = infllm_v2.compressed_lengths(cu(lens, DEV), kernel, stride)
+    assert got.dtype == torch.int32
+    exp = [0]
+    for l in lens:
+        exp.append(exp[-1] + ((l - kernel) // stride + 1 if l >= kernel else 0))
+    assert got.cpu().tolist() == exp
+    assert infllm_v2.compressed_lengths(cu(lens), kernel, stride).tolist() == exp      # a host table
