@@ -107,11 +107,20 @@ class SparseAttention:
     def select(self, q, kc, cu_seqlens_q, cu_seqlens_c, max_seqlen_q, max_c, kc2=None,
                cu_seqlens_c2=None, cache_len: int = 0):
         """Block selection of packed sequences: int32 (Hk, total_q, topk), ascending, -1 padded."""
+        pooled = self._block_scores(q, kc, cu_seqlens_q, cu_seqlens_c, max_seqlen_q, max_c, kc2, cu_seqlens_c2, cache_len)
+        return ops.infllmv2_topk(pooled, self.config.topk, cache_len=cache_len, cu_seqlens_q=cu_seqlens_q)
+
+    @torch.no_grad()
+    def _select_mask(self, q, kc, cu_seqlens, cu_seqlens_c, max_seqlen, max_c, kc2, cu_seqlens_c2):
+        """`select`, packed into the mask that the attention takes: no block list is written and read."""
+        pooled = self._block_scores(q, kc, cu_seqlens, cu_seqlens_c, max_seqlen, max_c, kc2, cu_seqlens_c2)
+        return ops.infllmv2_topk_mask(pooled, self.config.topk, max_seqlen, cu_seqlens_q=cu_seqlens)[0]
+
+    def _block_scores(self, q, kc, cu_seqlens_q, cu_seqlens_c, max_seqlen_q, max_c, kc2, cu_seqlens_c2, cache_len=0):
         c = self.config
-        pooled = infllmv2_stage1_block_scores(q, kc, cu_seqlens_q, cu_seqlens_c, max_seqlen_q, max_c,
-                                              c.local_blocks, c.init_blocks, cache_len=cache_len,
-                                              lse_keys=kc2, cu_seqlens_v=cu_seqlens_c2)
-        return ops.infllmv2_topk(pooled, c.topk, cache_len=cache_len, cu_seqlens_q=cu_seqlens_q)
+        return infllmv2_stage1_block_scores(q, kc, cu_seqlens_q, cu_seqlens_c, max_seqlen_q, max_c,
+                                            c.local_blocks, c.init_blocks, cache_len=cache_len,
+                                            lse_keys=kc2, cu_seqlens_v=cu_seqlens_c2)
 
     # ------------------------------------------------------------------ prefill / training
     def prefill(self, q, k, v, cu_seqlens, max_seqlen: int, seqlens: Optional[Sequence[int]] = None,
@@ -128,11 +137,11 @@ class SparseAttention:
             kc, cu_c = self.compress(k.detach(), cu_seqlens, seqlens)
             if c.coarse_lse:
                 kc2, cu_c2 = self.compress(k.detach(), cu_seqlens, seqlens, coarse=True)
-        idx = None
+        mask = None
         if max_seqlen > c.dense_len and max_c > 0:
-            idx = self.select(q.detach(), kc, cu_seqlens, cu_c, max_seqlen, max_c, kc2, cu_c2)
+            mask = self._select_mask(q.detach(), kc, cu_seqlens, cu_c, max_seqlen, max_c, kc2, cu_c2)
         out = infllmv2_attn_varlen_func(q, k, v, cu_seqlens, cu_seqlens, max_seqlen, max_seqlen,
-                                        softmax_scale=softmax_scale, causal=True, topk_idx=idx)
+                                        softmax_scale=softmax_scale, causal=True, block_mask=mask)
         if cache is not None:
             cache.fill(k.detach(), v.detach(), kc, cu_seqlens, cu_c, max_seqlen, kc2, cu_c2)
         return out
