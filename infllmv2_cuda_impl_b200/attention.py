@@ -14,7 +14,7 @@ from typing import Optional, Tuple, Union
 import torch
 
 from . import _lib
-from .ops import topk_to_uint64, transpose_blockmask
+from .ops import _on, _stream, topk_to_uint64, transpose_blockmask
 
 BLOCK_N = 64      # tokens per KV block (the reference's N_BLOCK_DIM)
 GROUP = 16        # query heads per KV head (the reference's m_block_dim)
@@ -46,10 +46,6 @@ def check_device_status(device=None) -> None:
                 torch.cuda.synchronize(idx)
                 _lib.call("ifv2_check_status", _status[idx].data_ptr(),
                           torch.cuda.current_stream(idx).cuda_stream)
-
-
-def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
 
 
 def maybe_contiguous(x):
@@ -152,13 +148,13 @@ def infllmv2_attn_stage1(
         lib = _lib.load()
         ws_bytes = int(lib.ifv2_stage1_decode_workspace_bytes(batch, nheads_k, max_seqlen_k))
         ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-        with torch.cuda.device(q.device):
+        with _on(q.device):
             _lib.call("ifv2_stage1_decode_scores", q.data_ptr(), k.data_ptr(), buf.data_ptr(),
                       cu_seqlens_k.contiguous().data_ptr(), used_ptr, batch, k.shape[0], nheads,
                       nheads_k, q.shape[-1], max_seqlen_k, row_stride, float(softmax_scale), int(bool(causal)),
                       ws.data_ptr(), ws_bytes, _stream(q.device))
         return buf[:, :, :max_seqlen_k]
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         _lib.call("ifv2_stage1_scores", q.data_ptr(), k.data_ptr(),
                   lse_keys.data_ptr() if lse_keys is not None else None, buf.data_ptr(),
                   cu_seqlens_q.contiguous().data_ptr(), cu_seqlens_k.contiguous().data_ptr(),
@@ -208,7 +204,7 @@ def _stage1_paged(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_
     else:
         n_blocks, cache_len, cache_lens, local_blocks, init_blocks = pool_args
         pooled = torch.empty(nheads_k, total_q, n_blocks, dtype=torch.bfloat16, device=q.device)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         _lib.call("ifv2_stage1_paged", q.data_ptr(), k.data_ptr(), buf.data_ptr() if buf is not None else None,
                   pooled.data_ptr() if pooled is not None else None, cu_seqlens_q.contiguous().data_ptr(),
                   cu_seqlens_k.contiguous().data_ptr(),
@@ -253,7 +249,7 @@ def infllmv2_stage1_decode_select(q, k, cu_seqlens_k, positions, max_seqlen_k, c
     lib = _lib.load()
     ws_bytes = int(lib.ifv2_stage1_decode_workspace_bytes(batch, nheads_k, max_seqlen_k))
     ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device=q.device)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         _lib.call("ifv2_stage1_decode_select", q.data_ptr(), k.data_ptr(), cu_seqlens_k.contiguous().data_ptr(),
                   seqused_k.data_ptr() if seqused_k is not None else None, positions.contiguous().data_ptr(),
                   mask.data_ptr(), idx.data_ptr() if idx is not None else None, batch, k.shape[0], nheads,
@@ -323,7 +319,7 @@ def infllmv2_stage1_block_scores(q, k, cu_seqlens_q, cu_seqlens_k, max_seqlen_q,
     if return_scores:
         row_stride = max(round_multiple(max_seqlen_k, 128), 128)
         buf = torch.empty(nheads_k, total_q, row_stride, dtype=torch.bfloat16, device=q.device)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         _lib.call("ifv2_stage1_block_scores", q.data_ptr(), k.data_ptr(),
                   lse_keys.data_ptr() if lse_keys is not None else None,
                   buf.data_ptr() if buf is not None else None, pooled.data_ptr(),
@@ -364,7 +360,7 @@ def _fwd(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softma
                 assert t.dtype == torch.int32 and t.numel() == batch, f"{name} must be (batch,) int32"
         nheads_k = k.shape[1]
         lse = torch.empty(nheads_k, total_q * GROUP, dtype=torch.float32, device=q.device)
-        with torch.cuda.device(q.device):
+        with _on(q.device):
             _lib.call("ifv2_sparse_attn_fwd_paged", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
                       lse.data_ptr(), fwd_mask.data_ptr() if fwd_mask is not None else None,
                       fwd_mask.shape[-1] if fwd_mask is not None else 0,
@@ -377,7 +373,7 @@ def _fwd(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softma
         return out, lse
     nheads_k = k.shape[1]
     lse = torch.empty(nheads_k, total_q * GROUP, dtype=torch.float32, device=q.device)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         _lib.call("ifv2_sparse_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(),
                   lse.data_ptr(), fwd_mask.data_ptr() if fwd_mask is not None else None,
                   fwd_mask.shape[-1] if fwd_mask is not None else 0,
@@ -396,7 +392,7 @@ def _bwd(dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_
     lib = _lib.load()
     ws_bytes = int(lib.ifv2_sparse_attn_bwd_workspace_bytes(total_q, nheads, d))
     ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         _lib.call("ifv2_sparse_attn_bwd", dout.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(),
                   out.data_ptr(), lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                   fwd_mask.data_ptr() if fwd_mask is not None else None,
@@ -410,13 +406,19 @@ def _bwd(dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_
     return dq, dk, dv
 
 
-@torch.library.custom_op("infllmv2_attn::_infllmv2_attn_varlen_forward", mutates_args=(),
-                         device_types="cuda")
-def _infllmv2_attn_varlen_forward(
-    q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens_q: torch.Tensor,
-    cu_seqlens_k: torch.Tensor, max_seqlen_q: int, max_seqlen_k: int, softmax_scale: float,
-    causal: bool, topk_idx: Optional[torch.Tensor] = None, block_mask: Optional[torch.Tensor] = None,
-) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+def _plain_eager(*tensors) -> bool:
+    """True when nothing watches the operators that are called: no compilation or trace, no dispatch
+    mode, no function transform, no tensor subclass.  The bodies of the two registered operators below
+    are then called as they are; going through the registration costs 50-70 us of host time per call,
+    more than the kernels of a short prefill."""
+    return (not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and torch._C._len_torch_dispatch_stack() == 0
+            and torch._C._functorch.peek_interpreter_stack() is None
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors if t is not None))
+
+
+def _varlen_forward(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softmax_scale,
+                    causal, topk_idx=None, block_mask=None):
     """Returns (out, softmax_lse (nheads_k, total_q*16), fwd_blockmask int64 or an empty tensor)."""
     q, k, v = [_dense(maybe_contiguous(x)) for x in (q, k, v)]
     if block_mask is not None:
@@ -438,6 +440,18 @@ def _infllmv2_attn_varlen_forward(
     return out, lse, fwd_mask
 
 
+@torch.library.custom_op("infllmv2_attn::_infllmv2_attn_varlen_forward", mutates_args=(),
+                         device_types="cuda")
+def _infllmv2_attn_varlen_forward(
+    q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cu_seqlens_q: torch.Tensor,
+    cu_seqlens_k: torch.Tensor, max_seqlen_q: int, max_seqlen_k: int, softmax_scale: float,
+    causal: bool, topk_idx: Optional[torch.Tensor] = None, block_mask: Optional[torch.Tensor] = None,
+) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """`_varlen_forward` as a registered operator."""
+    return _varlen_forward(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softmax_scale, causal,
+                           topk_idx, block_mask)
+
+
 @_infllmv2_attn_varlen_forward.register_fake
 def _(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softmax_scale, causal,
       topk_idx=None, block_mask=None):
@@ -448,14 +462,8 @@ def _(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softmax_s
             q.new_empty((k.shape[1], q.shape[0] * GROUP), dtype=torch.float32), mask)
 
 
-@torch.library.custom_op("infllmv2_attn::_infllmv2_attn_varlen_backward", mutates_args=(),
-                         device_types="cuda")
-def _infllmv2_attn_varlen_backward(
-    dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor,
-    softmax_lse: torch.Tensor, cu_seqlens_q: torch.Tensor, cu_seqlens_k: torch.Tensor,
-    max_seqlen_q: int, max_seqlen_k: int, softmax_scale: float, causal: bool,
-    fwd_blockmask: torch.Tensor,
-) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+def _varlen_backward(dout, q, k, v, out, softmax_lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
+                     softmax_scale, causal, fwd_blockmask):
     dout = _dense(maybe_contiguous(dout))
     fwd_mask = bwd_mask = None
     if fwd_blockmask.numel() > 0:
@@ -465,6 +473,19 @@ def _infllmv2_attn_varlen_backward(
     return _bwd(dout, q, k, v, out, softmax_lse, cu_seqlens_q.contiguous(),
                 cu_seqlens_k.contiguous(), max_seqlen_q, max_seqlen_k, softmax_scale, causal,
                 fwd_mask, bwd_mask)
+
+
+@torch.library.custom_op("infllmv2_attn::_infllmv2_attn_varlen_backward", mutates_args=(),
+                         device_types="cuda")
+def _infllmv2_attn_varlen_backward(
+    dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tensor,
+    softmax_lse: torch.Tensor, cu_seqlens_q: torch.Tensor, cu_seqlens_k: torch.Tensor,
+    max_seqlen_q: int, max_seqlen_k: int, softmax_scale: float, causal: bool,
+    fwd_blockmask: torch.Tensor,
+) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
+    """`_varlen_backward` as a registered operator."""
+    return _varlen_backward(dout, q, k, v, out, softmax_lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
+                            softmax_scale, causal, fwd_blockmask)
 
 
 @_infllmv2_attn_varlen_backward.register_fake
@@ -482,7 +503,9 @@ class Infllmv2AttnVarlenFunc(torch.autograd.Function):
                       "infllmv2_attn_varlen_func")
         if softmax_scale is None:
             softmax_scale = q.shape[-1] ** (-0.5)
-        out, lse, fwd_mask = _infllmv2_attn_varlen_forward(
+        forward = (_varlen_forward if _plain_eager(q, k, v, cu_seqlens_q, cu_seqlens_k, topk_idx, block_mask)
+                   else _infllmv2_attn_varlen_forward)
+        out, lse, fwd_mask = forward(
             q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softmax_scale, causal,
             topk_idx, block_mask)
         if block_mask is not None:
@@ -495,7 +518,9 @@ class Infllmv2AttnVarlenFunc(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout, *args):
         q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, fwd_mask = ctx.saved_tensors
-        dq, dk, dv = _infllmv2_attn_varlen_backward(
+        backward = (_varlen_backward if _plain_eager(dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, fwd_mask)
+                    else _infllmv2_attn_varlen_backward)
+        dq, dk, dv = backward(
             dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, ctx.max_seqlen_q,
             ctx.max_seqlen_k, ctx.softmax_scale, ctx.causal, fwd_mask)
         if _CHECK_STATUS:
@@ -640,7 +665,7 @@ def infllmv2_attn_with_kvcache(
                              "(seqlen_ro, rotary_dim / 2) in the dtype of q")
         k2 = k.reshape(batch, nheads_k, d).contiguous()
         q_rot, k_rot = torch.empty_like(q2), torch.empty_like(k2)
-        with torch.cuda.device(q.device):
+        with _on(q.device):
             _lib.call("ifv2_decode_rotary", q2.data_ptr(), k2.data_ptr(), q_rot.data_ptr(), k_rot.data_ptr(),
                       rotary_cos.contiguous().data_ptr(), rotary_sin.contiguous().data_ptr(),
                       cache_seqlens.data_ptr(), batch, nheads, nheads_k, d, 2 * rotary_cos.shape[1],
@@ -652,7 +677,7 @@ def infllmv2_attn_with_kvcache(
     max_blocks = (cap + BLOCK_N - 1) // BLOCK_N
     ws_bytes = int(lib.ifv2_decode_workspace_bytes(batch, nheads, d, max_blocks))
     ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device=q.device)
-    with torch.cuda.device(q.device):
+    with _on(q.device):
         _lib.call("ifv2_decode_paged", q2.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
                   k.contiguous().data_ptr() if k is not None else None,
                   v.contiguous().data_ptr() if v is not None else None, out.data_ptr(),

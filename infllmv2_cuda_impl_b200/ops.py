@@ -6,6 +6,7 @@ the CUDA library through the C ABI on the current stream.  `infllmv2_topk` and
 `transpose_blockmask` are additions (the reference leaves top-k to its caller and builds the
 backward mask through a bool round trip).
 """
+import contextlib
 from typing import Optional, Tuple
 
 import torch
@@ -14,7 +15,15 @@ from . import _lib
 
 
 def _stream(device) -> int:
-    return torch.cuda.current_stream(device).cuda_stream
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+_AS_IT_IS = contextlib.nullcontext()
+
+
+def _on(device):
+    """Context in which `device` is the current one; nothing to switch (2-3 us of a call) if it is."""
+    return _AS_IT_IS if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def _require_cuda(t: torch.Tensor, name: str):
@@ -46,7 +55,7 @@ def topk_to_uint64(topk_idx: torch.Tensor, max_seqlen_k: int, block_size: int,
         result = memory_buffer
     else:
         result = torch.empty(out_shape, dtype=torch.int64, device=topk_idx.device)
-    with torch.cuda.device(topk_idx.device):
+    with _on(topk_idx.device):
         _lib.call("ifv2_topk_to_uint64", topk_idx.data_ptr(), result.data_ptr(), rows,
                   topk_idx.shape[-1], k_blocks, words, _stream(topk_idx.device))
     return result, k_blocks
@@ -63,7 +72,7 @@ def blockmask_to_uint64(blockmask: torch.Tensor) -> Tuple[torch.Tensor, int]:
     rows = int(torch.Size(blockmask.shape[:-1]).numel())
     result = torch.empty(tuple(blockmask.shape[:-1]) + (words,), dtype=torch.int64,
                          device=blockmask.device)
-    with torch.cuda.device(blockmask.device):
+    with _on(blockmask.device):
         _lib.call("ifv2_blockmask_to_uint64", blockmask.data_ptr(), result.data_ptr(), rows, last,
                   words, _stream(blockmask.device))
     return result, last
@@ -79,7 +88,7 @@ def uint64_to_bool(uint64_array: torch.Tensor, last_dim_size: int) -> torch.Tens
     rows = int(torch.Size(uint64_array.shape[:-1]).numel())
     result = torch.empty(tuple(uint64_array.shape[:-1]) + (last_dim_size,), dtype=torch.bool,
                          device=uint64_array.device)
-    with torch.cuda.device(uint64_array.device):
+    with _on(uint64_array.device):
         _lib.call("ifv2_uint64_to_bool", uint64_array.data_ptr(), result.data_ptr(), rows,
                   last_dim_size, words, _stream(uint64_array.device))
     return result
@@ -98,7 +107,7 @@ def transpose_blockmask(fwd_mask: torch.Tensor, k_blocks: int) -> torch.Tensor:
     if words != (k_blocks + 63) // 64:
         raise ValueError(f"fwd_mask has {words} words per row, k_blocks={k_blocks} needs {(k_blocks + 63) // 64}")
     out = torch.empty(hk, k_blocks, (t + 63) // 64, dtype=torch.int64, device=fwd_mask.device)
-    with torch.cuda.device(fwd_mask.device):
+    with _on(fwd_mask.device):
         _lib.call("ifv2_transpose_blockmask", fwd_mask.data_ptr(), out.data_ptr(), hk, t, k_blocks,
                   _stream(fwd_mask.device))
     return out
@@ -128,7 +137,7 @@ def max_pooling_1d(input: torch.Tensor, cache_len: int, local_blocks: int, init_
     num_heads, q_len, k_len = input.shape
     out_len = (q_len + cache_len + block_size - 1) // block_size
     output = torch.empty(num_heads, q_len, out_len, device=input.device, dtype=input.dtype)
-    with torch.cuda.device(input.device):
+    with _on(input.device):
         _lib.call("ifv2_max_pooling_1d", input.data_ptr(), output.data_ptr(),
                   int(input.dtype == torch.bfloat16), num_heads, q_len, k_len, row_stride, out_len,
                   cache_len, kernel_size, pool_stride, padding, block_size, local_blocks,
@@ -164,7 +173,7 @@ def max_pooling_1d_varlen(input: torch.Tensor, cu_seqlens_q: torch.Tensor,
         max_cache_len = int(cache_lens.max().item())
     out_len = (max_seqlen_q + max_cache_len + block_size - 1) // block_size
     output = torch.empty(num_heads, total_q, out_len, device=input.device, dtype=input.dtype)
-    with torch.cuda.device(input.device):
+    with _on(input.device):
         _lib.call("ifv2_max_pooling_1d_varlen", input.data_ptr(), output.data_ptr(),
                   cu_seqlens_q.data_ptr(), cu_seqlens_k.data_ptr(), cache_lens.data_ptr(),
                   int(input.dtype == torch.bfloat16), batch_size, num_heads, total_q, max_seqlen_k,
@@ -204,7 +213,7 @@ def infllmv2_topk(block_score: torch.Tensor, k: int, cache_len: int = 0,
             cl_ptr = cache_lens.data_ptr()
     elif cache_lens is not None:
         raise ValueError("cache_lens needs cu_seqlens_q")
-    with torch.cuda.device(block_score.device):
+    with _on(block_score.device):
         _lib.call("ifv2_topk_select", block_score.data_ptr(), out.data_ptr(),
                   int(block_score.dtype == torch.bfloat16), hk, t, n, row_stride, k, cu_ptr, cl_ptr,
                   batch, cache_len, block_size, _stream(block_score.device))
@@ -247,7 +256,7 @@ def infllmv2_topk_mask(block_score: torch.Tensor, k: int, max_seqlen_k: int, cac
             cl_ptr = cache_lens.data_ptr()
     elif cache_lens is not None:
         raise ValueError("cache_lens needs cu_seqlens_q")
-    with torch.cuda.device(dev):
+    with _on(dev):
         _lib.call("ifv2_topk_select_mask", block_score.data_ptr(), idx.data_ptr() if idx is not None else None,
                   mask.data_ptr(), col.data_ptr() if col is not None else None,
                   int(block_score.dtype == torch.bfloat16), hk, t, n, row_stride, k, k_blocks, cu_ptr, cl_ptr,
@@ -269,7 +278,7 @@ def compressed_lengths(cu_seqlens_k: torch.Tensor, kernel_size: int = 32,
             and cu_seqlens_k.numel() >= 1 and kernel_size >= 1 and kernel_stride >= 1):
         cu_seqlens_k = cu_seqlens_k.contiguous()
         cu_c = torch.empty_like(cu_seqlens_k)
-        with torch.cuda.device(cu_c.device):
+        with _on(cu_c.device):
             _lib.call("ifv2_compressed_lengths", cu_seqlens_k.data_ptr(), cu_c.data_ptr(), cu_c.numel() - 1,
                       kernel_size, kernel_stride, _stream(cu_c.device))
         return cu_c
@@ -312,7 +321,7 @@ def compress_keys(k: torch.Tensor, cu_seqlens_k: Optional[torch.Tensor] = None, 
             total_c = int(cu_seqlens_c[-1].item())
         cu_k_ptr, cu_c_ptr = cu_seqlens_k.data_ptr(), cu_seqlens_c.data_ptr()
     kc = torch.empty(total_c, hk, d, dtype=k.dtype, device=k.device)
-    with torch.cuda.device(k.device):
+    with _on(k.device):
         _lib.call("ifv2_compress_keys", k.data_ptr(), kc.data_ptr(), cu_k_ptr, cu_c_ptr, batch,
                   total_k, total_c, hk, d, kernel_size, kernel_stride, _stream(k.device))
     return kc, cu_seqlens_c
@@ -333,7 +342,7 @@ def compress_keys_append(k_cache: torch.Tensor, cache_seqlens: torch.Tensor, kc_
     b, cap, hk, d = k_cache.shape
     if kc_cache.shape[0] != b or kc_cache.shape[2] != hk or kc_cache.shape[3] != d:
         raise ValueError("kc_cache does not match k_cache")
-    with torch.cuda.device(k_cache.device):
+    with _on(k_cache.device):
         _lib.call("ifv2_compress_keys_append", k_cache.data_ptr(), kc_cache.data_ptr(),
                   cache_seqlens.contiguous().data_ptr(), b, cap, kc_cache.shape[1], hk, d,
                   kernel_size, kernel_stride, _stream(k_cache.device))
@@ -353,7 +362,7 @@ def cache_fill(src: torch.Tensor, cache: torch.Tensor, cu_seqlens: torch.Tensor,
     if seqlens_out is not None:
         assert seqlens_out.dtype == torch.int32 and seqlens_out.is_contiguous() and seqlens_out.numel() == cache.shape[0]
     src = src.contiguous()
-    with torch.cuda.device(src.device):
+    with _on(src.device):
         _lib.call("ifv2_cache_fill", src.data_ptr(), cache.data_ptr(), cu_seqlens.contiguous().data_ptr(),
                   seqlens_out.data_ptr() if seqlens_out is not None else None, cache.shape[0],
                   src.shape[0], cache.shape[1], cache.shape[2], cache.shape[3], _stream(src.device))
@@ -387,7 +396,7 @@ def decode_append(k_new: torch.Tensor, v_new: torch.Tensor, k_cache: torch.Tenso
                               or c.shape[0] != b or c.shape[2:] != k_cache.shape[2:]):
             raise ValueError("decode_append: a compressed cache must be contiguous (batch, c_capacity, heads_k, 128) bf16")
     ptr = lambda t: t.data_ptr() if t is not None else None
-    with torch.cuda.device(k_cache.device):
+    with _on(k_cache.device):
         _lib.call("ifv2_decode_append", k_new.data_ptr(), v_new.data_ptr(), k_cache.data_ptr(),
                   v_cache.data_ptr(), ptr(kc_cache), ptr(kc2_cache), cache_seqlens.data_ptr(),
                   ptr(positions), ptr(n_comp), ptr(n_comp2), b, cap,
@@ -421,7 +430,7 @@ def decode_select(score: torch.Tensor, positions: torch.Tensor, k: int, max_seql
     words = (n_blocks + 63) // 64
     mask = torch.empty(b, hk, 1, words, dtype=torch.int64, device=score.device)
     idx = torch.empty(b, hk, 1, k, dtype=torch.int32, device=score.device) if return_topk else None
-    with torch.cuda.device(score.device):
+    with _on(score.device):
         _lib.call("ifv2_decode_select", score.data_ptr(), int(score.dtype == torch.bfloat16), row_stride,
                   seqused_c.data_ptr() if seqused_c is not None else None, positions.contiguous().data_ptr(),
                   mask.data_ptr(), idx.data_ptr() if idx is not None else None, b, hk, n_c, n_blocks, words,
