@@ -13,6 +13,7 @@
 //                    the group is implicit because those heads are rows of the same tile.
 // Recomputing S and dP in both kernels costs 7 tile products instead of 5, but removes the
 // scatter of 16x128 fp32 tiles per (token, block) pair that bounds an atomics-based design.
+#include "block_walk.cuh"
 #include "tc05.cuh"
 
 namespace ifv2 {
@@ -103,23 +104,6 @@ struct MaskRowReader {
       below = j > 0 ? __ldg(row + j - 1) : 0ull;
     }
     return (cur >> (blk & 63)) & 1ull;
-  }
-};
-
-// Highest-to-lowest walk over the set bits of a tile's union mask.
-struct BlockWalk {
-  const unsigned long long* words;
-  int w;
-  unsigned long long cur;
-  __device__ BlockWalk(const unsigned long long* u, int nwords) : words(u), w(nwords), cur(0) {}
-  __device__ int next() {
-    while (cur == 0ull) {
-      if (w == 0) return -1;
-      cur = words[--w];
-    }
-    const int b = 63 - __clzll(cur);
-    cur &= ~(1ull << b);
-    return w * 64 + b;
   }
 };
 

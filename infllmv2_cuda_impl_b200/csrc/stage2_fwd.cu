@@ -13,16 +13,22 @@
 // epilogue.  K and V each have a 2-deep ring; S/P is double-buffered in TMEM so Q.K^T of the
 // next block overlaps the softmax of the current one.  TMEM: 2 x 64 (S/P) + 128 (O) = 256
 // columns, shared memory 96 KB, so two CTAs share an SM and fill each other's bubbles.
-// The running max is only raised when it grows by more than 2^8 (the accumulator then needs a
-// rescale); P stays bounded by 256 and the final 1/l normalisation makes the result exact.
-// Measured with the optional timeline below: the tensor pipe is ~70 % busy and what bounds a
-// CTA is the latency of the chain S ready -> P ready -> P.V -> next Q.K^T on each S buffer
-// while the co-resident CTA competes for the tensor pipe and the exponential unit.  Splitting a
-// row over two threads (8 softmax warps, half-row maxima exchanged through shared memory) or
-// giving each S buffer its own warp group did not shorten that chain and ran 8-12 % slower;
-// evaluating every 2nd, 3rd or 4th pair of exponentials on the FMA pipe (degree-3 polynomial)
-// ran 8, 4 and 3 % slower: the exponential unit is not what the softmax warps wait for.
+// The reference maximum of a row is raised only when a block's exponentials get large (their sum passes
+// 64 x 2^8): P is a floating-point number, so its relative precision does not depend on the reference,
+// and the final 1/l normalisation makes the result exact.  A block costs no row maximum otherwise.
+// What bounds a softmax warp (timeline of a build with clock stamps, 65536-token training batch, per
+// 64-key block): ~1000 clocks of exponentials, 2 x 64 x 8 for the two warps that share a special-function
+// unit, ~200 of waiting for the scores, ~180 of loop and selection bookkeeping, ~100 of TMEM traffic.
+// The bookkeeping was 350 clocks while every thread walked the union and its own mask row block by block
+// (block_walk.cuh does it 32 blocks at a time); that and the row maximum gone: 2.80 -> 2.50 ms at 32768
+// tokens, 2.00 -> 1.79 ms for a 4096-token chunk at 131072, 4.10 -> 3.62 ms for the training batch.
+// Measured and not taken: pairs of blocks (S with N = 128 in one buffer; 20 % fewer tensor clocks, but the
+// chain of a CTA gets longer: 10-20 % slower); a row split over two threads (8 softmax warps, half the
+// columns each, no exchange in the common case: 15-20 % slower); every 8th or 4th pair of exponentials as
+// a polynomial on the FMA pipe (3-8 % slower).
+#include "block_walk.cuh"
 #include "tc05.cuh"
+#include <limits.h>
 
 namespace ifv2 {
 namespace {
@@ -36,6 +42,7 @@ constexpr uint32_t kQHalfBytes = 128 * 128;   // 128 rows x 64 bf16
 constexpr uint32_t kKVHalfBytes = 64 * 128;   // 64 keys x 64 bf16
 constexpr uint32_t kTmemCols = 256;
 constexpr float kRescaleThreshold = 8.0f;     // log2 units
+constexpr float kSumLimit = 16384.0f;         // 64 scores, each the threshold above the reference
 
 struct FwdParams {
   __nv_bfloat16* out;
@@ -67,45 +74,7 @@ struct Smem {
   //               refill the V tile, a rescale or the epilogue may touch O.
   uint64_t q_full, k_full[2], v_full[2], qk_done[2], pv_done[2], p_ready[2];
   uint32_t tmem_base;
-  int n_blocks;
   int abort_flag;
-};
-
-// One thread's mask row, read in the order the tile's blocks are walked (highest first): the word
-// of the current 64 blocks stays in a register and the word below it is fetched ahead, so that a
-// step does not start with a round trip to global memory.
-struct MaskRowReader {
-  const unsigned long long* row;   // null: every block counts as selected
-  int wi;                          // index of the word in `cur`, -1 before the first read
-  unsigned long long cur, below;
-  __device__ explicit MaskRowReader(const unsigned long long* r) : row(r), wi(-1), cur(0ull), below(0ull) {}
-  __device__ bool selected(int blk) {
-    if (row == nullptr) return true;
-    const int j = blk >> 6;
-    if (j != wi) {
-      cur = (wi >= 0 && j == wi - 1) ? below : __ldg(row + j);
-      wi = j;
-      below = j > 0 ? __ldg(row + j - 1) : 0ull;
-    }
-    return (cur >> (blk & 63)) & 1ull;
-  }
-};
-
-// Highest-to-lowest walk over the set bits of the tile's union mask.
-struct BlockWalk {
-  const unsigned long long* words;
-  int w;
-  unsigned long long cur;
-  __device__ BlockWalk(const unsigned long long* u, int nwords) : words(u), w(nwords), cur(0) {}
-  __device__ int next() {
-    while (cur == 0ull) {
-      if (w == 0) return -1;
-      cur = words[--w];
-    }
-    const int b = 63 - __clzll(cur);
-    cur &= ~(1ull << b);
-    return w * 64 + b;
-  }
 };
 
 __global__ void __launch_bounds__(kThreads, 2)
@@ -143,7 +112,9 @@ sparse_attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q,
       if (p.mask != nullptr) {
         const unsigned long long* row =
             p.mask + ((int64_t)h * p.total_q + q0 + tok0) * p.mask_words + w;
-        for (int t = 0; t < ntok; ++t) u |= __ldg(row + (int64_t)t * p.mask_words);
+#pragma unroll
+        for (int t = 0; t < kTokPerTile; ++t)            // (all rows in flight at once)
+          if (t < ntok) u |= __ldg(row + (int64_t)t * p.mask_words);
       } else {
         u = ~0ull;
       }
@@ -172,20 +143,16 @@ sparse_attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q,
     tmem_alloc(&sm.tmem_base, kTmemCols);
     tmem_relinquish();
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int n = 0;
-    for (int w = 0; w < words; ++w) n += __popcll(sm.umask[w]);
-    sm.n_blocks = n;
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
 
-  // (read through a warp broadcast: it tells the compiler that the value is warp-uniform, so the
+  // (warp reductions and broadcasts: they tell the compiler that the values are warp-uniform, so the
   //  MMA issuer's descriptor arithmetic stays in uniform registers instead of being moved there
   //  operand by operand for every MMA)
-  const int n_blocks = __shfl_sync(0xFFFFFFFFu, sm.n_blocks, 0);
+  int n_blocks = 0;
+  for (int w = lane; w < words; w += 32) n_blocks += __popcll(sm.umask[w]);
+  n_blocks = __reduce_add_sync(0xFFFFFFFFu, n_blocks);
   const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, sm.tmem_base, 0);
   const uint32_t tmem_o = tmem + 128;
   volatile int* abort_flag = &sm.abort_flag;
@@ -286,24 +253,29 @@ sparse_attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q,
     const int tok = tok0 + tl;                       // local token index
     const bool valid = tl < ntok;
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
-    const unsigned long long* mrow =
-        (p.mask != nullptr && valid)
-            ? p.mask + ((int64_t)h * p.total_q + q0 + tok) * p.mask_words : nullptr;
+    // mask rows of the warp's two tokens
+    auto mask_row = [&](int t) -> const unsigned long long* {
+      return (p.mask != nullptr && t < ntok) ? p.mask + ((int64_t)h * p.total_q + q0 + tok0 + t) * p.mask_words : nullptr;
+    };
     const int row_limit = valid ? min(lk, p.causal ? tok + shift + 1 : lk) : 0;   // visible keys
 
     float m_ref = -INFINITY, l = 0.f;
     bool ok = true;
-    BlockWalk walk(sm.umask, words);
-    MaskRowReader mask_reader(mrow);
+    // keys that every row of the warp sees (rows past the sequence see none and do not count)
+    const int all_see = __reduce_min_sync(0xFFFFFFFFu, valid ? row_limit : INT_MAX);
+    bool no_ref = true;                              // some row of the warp has no reference maximum yet
+    WalkBatch walk;
     for (int i = 0; i < n_blocks; ++i) {
-      const int blk = walk.next();
+      if ((i & 31) == 0)
+        walk.refill(sm.umask, words, i, p.mask != nullptr, mask_row(2 * quad), mask_row(2 * quad + 1), lane);
+      const int blk = __shfl_sync(0xFFFFFFFFu, walk.blk, i & 31);
       const int s = i & 1;
       const uint32_t par = (uint32_t)((i >> 1) & 1);
-      const bool selected = valid && mask_reader.selected(blk);
+      const bool selected = valid && ((walk.sel >> (i & 31)) & 1u);
       const int lim = selected ? min(max(row_limit - blk * kBlockN, 0), kBlockN) : 0;
       // only the diagonal / ragged block needs per-element masking; a row that did not select
       // the block is handled by the row-level terms below
-      const bool partial = __any_sync(0xFFFFFFFFu, lim > 0 && lim < kBlockN);
+      const bool partial = (blk + 1) * kBlockN > all_see;
       ok = __all_sync(0xFFFFFFFFu, mbar_wait(&sm.qk_done[s], par, abort_flag, p.status, 31));
       if (!ok) break;
       tc_fence_after();
@@ -345,17 +317,15 @@ sparse_attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q,
           mx4[(c >> 1) & 3] = fmaxf(mx4[(c >> 1) & 3], fmaxf(__uint_as_float(raw[c]), __uint_as_float(raw[c + 1])));
         return (lim > 0) ? fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) : -INFINITY;
       };
-      // The reference maximum moves only when the row maximum exceeds it by more than the
-      // threshold, which after a row's first block almost never happens.  So once every row of the
-      // warp that takes part has a reference, the exponentials are started against the current one
-      // and the row maximum is computed beside them (it is off the chain S -> P); a block that does
-      // move some row's reference is redone below, with the result the in-order form would give.
+      // The reference maximum has to move only when a score exceeds it by so much that the numbers
+      // get large, which after a row's first block almost never happens: P keeps its relative
+      // precision at any reference.  So once every row of the warp that takes part has a reference,
+      // the exponentials are taken against it and no row maximum is computed at all; a block whose
+      // sum reaches the bound (or is not a number) is redone below with the maximum.
       bool done = false;
-      if (!__any_sync(0xFFFFFFFFu, lim > 0 && m_ref == -INFINITY)) {
+      if (!no_ref || !__any_sync(0xFFFFFFFFu, lim > 0 && m_ref == -INFINITY)) {
         compute_p((lim == 0) ? -INFINITY : -m_ref * p.scale_log2);
-        const float mx = row_max();
-        const bool moves = mx > m_ref && (mx - m_ref) * p.scale_log2 > kRescaleThreshold;
-        done = !__any_sync(0xFFFFFFFFu, moves);
+        done = __all_sync(0xFFFFFFFFu, sum < kSumLimit);
       }
       if (!done) {
         const float mx = row_max();
@@ -385,6 +355,7 @@ sparse_attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q,
           }
           tmem_wait_st();
         }
+        no_ref = __any_sync(0xFFFFFFFFu, valid && m_ref == -INFINITY);
         // rows that take nothing from this block get an exponent of -inf (P = 0) for every column
         compute_p((lim == 0) ? -INFINITY : -m_ref * p.scale_log2);
       }

@@ -106,3 +106,11 @@ def test_bwd_column_masks_with_long_empty_stretches():
         assert mx <= MAX_ABS * scale and mr <= MEAN_REL, (name, mx, mr, scale)
     # the rows of block 1 of the first sequence get exactly the contributions of those 73 tokens
     assert dk[64:128].abs().max() > 0 and dv[64:128].abs().max() > 0
+
+
+@pytest.mark.parametrize("n_sel", [1, 2, 3, 7])
+@pytest.mark.parametrize("len_k", [448, 461])
+def test_bwd_odd_and_even_block_counts(n_sel, len_k):
+    # the dQ kernel takes blocks in pairs and keeps up to three pairs of key tiles in flight
+    _check([24], [len_k], n_sel, True, shared=True, seed=60 + n_sel)
+    _check([13], [len_k], n_sel, False, seed=70 + n_sel)

@@ -108,3 +108,64 @@ def test_fwd_multiword_mask_eight_kv_heads():
     ref, _ = oracle.sparse_attention_fwd(q, k, v, cu(lens), cu(lens), idx, causal=True)
     mx, mr = err_stats(out[sl], ref[sl])
     assert mx <= MAX_ABS and mr <= MEAN_REL, (mx, mr)
+
+
+@pytest.mark.parametrize("n_sel", [1, 2, 3, 5])
+@pytest.mark.parametrize("len_k", [320, 333, 384])
+def test_fwd_odd_and_even_block_counts(n_sel, len_k):
+    # blocks are walked in pairs: a last single block, a ragged block as the first or second of a
+    # pair, and tokens of one tile that select different blocks of a pair
+    hq, hk, d, lq = 32, 2, 128, 21
+    q = det_tensor((lq, hq, d), 31, 0.25)
+    k = det_tensor((len_k, hk, d), 32, 0.25)
+    v = det_tensor((len_k, hk, d), 33)
+    shared = local_topk(hk, [lq], [len_k], n_sel, 34 + n_sel)[:, -1:].expand(-1, lq, -1).contiguous()
+    _check(q, k, v, cu([lq]), cu([len_k]), shared, True)
+    _check(q, k, v, cu([lq]), cu([len_k]), local_topk(hk, [lq], [len_k], n_sel, 40 + n_sel), False)
+
+
+@pytest.mark.parametrize("jump", [1, 2, 3, 4])
+def test_fwd_reference_moves_at_any_block(jump):
+    # the scores of block `jump` (counted in walking order, highest block first) exceed all before it
+    # by ~60 (natural log units): the running reference has to move at the first or second block of a pair
+    hq, hk, d, n_blk = 32, 2, 128, 6
+    q = torch.zeros(9, hq, d, dtype=torch.bfloat16)
+    q[..., 0] = 1.0
+    q[..., 1:9] = det_tensor((9, hq, 8), 51, 0.25)
+    k = det_tensor((n_blk * 64, hk, d), 52, 0.25)
+    k[..., 0] = 0.0
+    first = (n_blk - 1 - jump) * 64
+    k[first:first + 64, :, 0] = 680.0                      # 680 / sqrt(128) = 60
+    v = det_tensor((n_blk * 64, hk, d), 53)
+    _check(q, k, v, cu([9]), cu([n_blk * 64]), None, False)
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_registered_operators_are_used_when_something_traces(packed):
+    # a plain eager call runs the bodies directly; under a dispatch mode the registered operators are
+    # what the mode sees, with the same results
+    from torch.utils._python_dispatch import TorchDispatchMode
+    seen = []
+
+    class Recorder(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    hq, hk, d, n = 32, 2, 128, 200
+    idx = local_topk(hk, [n], [n], 2, 77).to(DEV)
+    sel = dict(block_mask=infllm_v2.topk_to_uint64(idx, n, 64)[0]) if packed else dict(topk_idx=idx)
+    res = []
+    for mode in (None, Recorder()):
+        q, k, v = (det_tensor((n, h, d), 78 + i, 0.25, device=DEV).requires_grad_(True) for i, h in enumerate((hq, hk, hk)))
+        def call():
+            out = infllm_v2.infllmv2_attn_varlen_func(q, k, v, cu([n], DEV), cu([n], DEV), n, n, causal=True, **sel)
+            return (out.detach(),) + torch.autograd.grad(out, (q, k, v), det_tensor((n, hq, d), 81, 0.5, device=DEV))
+        if mode is None:
+            res.append(call())
+        else:
+            with mode:
+                res.append(call())
+    assert all(torch.equal(a, b) for a, b in zip(*res))
+    assert any("_infllmv2_attn_varlen_forward" in s for s in seen)
+    # (the engine runs the backward in a thread of its own, which the mode does not cover)
