@@ -368,12 +368,16 @@ __device__ __forceinline__ int block_of(int64_t x, int d) {
   return (x == (int64_t)(int)x) ? (int)x / d : (int)(x / d);
 }
 
+// CTAs per SM the kernel is compiled for: a probe is a chain of compares, a warp reduction and a branch,
+// so what matters is how many rows are in flight.
+template <int kIters> constexpr int kTopkResident = kIters == 2 ? 5 : kIters == 4 ? 4 : kIters <= 8 ? 3 : 1;
+
 // Bound by instruction issue and by the latency of the probes (a row is read once, everything else
 // happens in registers).  Over 1 M rows of 2048 blocks, mask only: 6.88 -> 2.28 ms against a form that
 // scanned the lanes once per 256 entries, counted in bf16 and walked the taken entries even where no list
 // was wanted; with the list, 65536 rows of 512 blocks: 0.112 -> 0.101 ms.
 template <typename T, int kIters, bool kList>
-__global__ void __launch_bounds__(kThreads, (kIters <= 8) ? 3 : 1) topk_select_kernel(const TopkParams p) {
+__global__ void __launch_bounds__(kThreads, kTopkResident<kIters>) topk_select_kernel(const TopkParams p) {
   using N = Num<T>;
   using P = Pack<T>;
   using T2 = typename P::T2;
@@ -497,7 +501,12 @@ __global__ void __launch_bounds__(kThreads, (kIters <= 8) ? 3 : 1) topk_select_k
 template <typename T, int kIters>
 void launch_topk_iters(const TopkParams& p, cudaStream_t st) {
   const int64_t gy = p.heads < 65535 ? p.heads : 65535;
-  const int64_t cap = ceil_div64((int64_t)kNumSMs * 8, gy);
+  // One wave: every warp strides over the rows, so a second, partly filled wave would leave SMs idle
+  // (2048 blocks: 2.28 -> 2.22 ms of 1 M rows; 512 blocks, with 5 instead of 3 CTAs per SM: 0.101 ->
+  // 0.094 ms of 65536).  Rows of at most 256 blocks are so short that a row per warp and more CTAs than
+  // fit are better (64 blocks, 8192 rows: 12.4 us against 14.4).
+  int64_t cap = (int64_t)kNumSMs * (kIters == 1 ? 8 : kTopkResident<kIters>) / gy;
+  if (cap < 1) cap = 1;
   int64_t gx = ceil_div64(p.total_q, kWarps);
   if (gx > cap) gx = cap;
   const dim3 grid((unsigned)gx, (unsigned)gy);
