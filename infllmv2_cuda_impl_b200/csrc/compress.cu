@@ -12,6 +12,9 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kVecPerRow = kHeadDim / 8;      // 16-byte vectors per (token, head) row
+// Loads a thread has in flight: a window is a chain of kernel / kInFlight trips to memory.  131072 tokens
+// x 8 heads: 61.3 us with 4, 56.3 with 16, 57.2 with 32 (72 with 8); short prompts are the same within 5 %.
+constexpr int kInFlight = 16;
 
 __device__ __forceinline__ void add_bf16x8(float (&acc)[8], const uint4& raw) {
   const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
@@ -58,15 +61,12 @@ __global__ void __launch_bounds__(kThreads) compress_keys_kernel(const CompressP
     const int64_t row = (int64_t)p.heads * kHeadDim;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     int t = 0;
-    for (; t + 4 <= p.kernel; t += 4) {        // four loads in flight per thread
-      const uint4 a = __ldg(reinterpret_cast<const uint4*>(src + (t + 0) * row));
-      const uint4 b4 = __ldg(reinterpret_cast<const uint4*>(src + (t + 1) * row));
-      const uint4 c = __ldg(reinterpret_cast<const uint4*>(src + (t + 2) * row));
-      const uint4 d = __ldg(reinterpret_cast<const uint4*>(src + (t + 3) * row));
-      add_bf16x8(acc, a);
-      add_bf16x8(acc, b4);
-      add_bf16x8(acc, c);
-      add_bf16x8(acc, d);
+    for (; t + kInFlight <= p.kernel; t += kInFlight) {
+      uint4 v4[kInFlight];
+#pragma unroll
+      for (int i = 0; i < kInFlight; ++i) v4[i] = __ldg(reinterpret_cast<const uint4*>(src + (t + i) * row));
+#pragma unroll
+      for (int i = 0; i < kInFlight; ++i) add_bf16x8(acc, v4[i]);
     }
     for (; t < p.kernel; ++t) add_bf16x8(acc, __ldg(reinterpret_cast<const uint4*>(src + t * row)));
     *reinterpret_cast<uint4*>(p.kc + (j * p.heads + h) * kHeadDim + v * 8) =
