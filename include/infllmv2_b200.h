@@ -112,6 +112,19 @@ int ifv2_cache_fill(const void* src, void* cache, const int32_t* cu_seqlens, int
                     int batch, int64_t total, int64_t capacity, int heads_k, int head_dim,
                     void* stream);
 
+/* The same for the keys, values and compressed keys of a prefill in ONE launch: k / v (total, heads_k,
+ * 128) by cu_seqlens, kc (total_c, heads_k, 128) by cu_seqlens_c; seqlens_out / n_comp_out (may be
+ * null): min(len_b, capacity) of the keys / compressed keys. */
+int ifv2_cache_fill_kv(const void* k, const void* v, const void* kc, void* k_cache, void* v_cache, void* kc_cache,
+                       const int32_t* cu_seqlens, const int32_t* cu_seqlens_c, int32_t* seqlens_out,
+                       int32_t* n_comp_out, int batch, int64_t total, int64_t total_c, int64_t capacity,
+                       int64_t c_capacity, int heads_k, int head_dim, void* stream);
+
+/* Three device-to-device copies in one launch (16-byte aligned, sizes multiples of 16 bytes, no overlap):
+ * what a decode step hands to the input buffers of a captured graph. */
+int ifv2_copy3(const void* src0, void* dst0, int64_t bytes0, const void* src1, void* dst1, int64_t bytes1,
+               const void* src2, void* dst2, int64_t bytes2, void* stream);
+
 /* One decode step of cache bookkeeping in one launch: k_new / v_new (batch, heads_k, 128) go to
  * position cache_seqlens[b] of k_cache / v_cache (batch, capacity, heads_k, 128); a sequence whose
  * new length L completes a compression window (L >= kernel, (L - kernel) % stride == 0) gets the

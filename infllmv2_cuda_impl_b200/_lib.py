@@ -51,6 +51,8 @@ SIGNATURES = {
                                                                                c_int64, c_void_p],
     "ifv2_cache_fill": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int64, c_int, c_int,
                         c_void_p],
+    "ifv2_cache_fill_kv": [c_void_p] * 10 + [c_int, c_int64, c_int64, c_int64, c_int64, c_int, c_int, c_void_p],
+    "ifv2_copy3": [c_void_p, c_void_p, c_int64] * 3 + [c_void_p],
     "ifv2_decode_append": [c_void_p] * 10 + [c_int, c_int64, c_int64, c_int64, c_int, c_int, c_int, c_int,
                                              c_int, c_int, c_void_p],
     "ifv2_stage1_block_scores": [c_void_p] * 8 + [c_int64, c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int64, c_int,

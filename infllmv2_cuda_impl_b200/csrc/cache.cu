@@ -41,28 +41,70 @@ __host__ __device__ inline int windows(int len, int kernel, int stride) {
   return len >= kernel ? (len - kernel) / stride + 1 : 0;
 }
 
-struct FillParams {
+struct FillSegment {
   const uint4* src;            // (total, heads, 128) bf16 as 16-byte vectors
   uint4* cache;                // (batch, cap, heads, 128)
   const int32_t* cu;           // (batch + 1)
   int32_t* seqlens_out;        // (batch) or null: min(len_b, cap)
-  int batch, heads;
   int64_t total, cap;
+  int64_t blocks;              // CTAs that copy this tensor
 };
+struct FillParams {
+  FillSegment seg[3];          // up to three tensors (keys, values, compressed keys) in one launch
+  int batch, heads;
+};
+constexpr int kFillPerThread = 4;
 
+// A CTA copies kFillPerThread * kThreads consecutive vectors of one tensor; its first token costs a
+// 64-bit division, the rest is 32-bit arithmetic and all of a thread's loads are in flight together.
 __global__ void __launch_bounds__(kThreads) cache_fill_kernel(const FillParams p) {
-  const int64_t row_vecs = (int64_t)p.heads * kVecPerRow;
-  const int64_t n_vec = p.total * row_vecs;
-  for (int64_t idx = (int64_t)blockIdx.x * kThreads + threadIdx.x; idx < n_vec;
-       idx += (int64_t)gridDim.x * kThreads) {
-    const int64_t t = idx / row_vecs, r = idx % row_vecs;
-    const int b = find_sequence(p.cu, p.batch, (int)t);
-    const int64_t pos = t - p.cu[b];
-    if (pos < p.cap) p.cache[((int64_t)b * p.cap + pos) * row_vecs + r] = __ldg(p.src + idx);
+  int64_t blk = blockIdx.x;                      // (segments that are not there have no blocks)
+  FillSegment g = p.seg[0];
+  if (blk >= g.blocks) {
+    blk -= g.blocks;
+    g = p.seg[1];
+    if (blk >= g.blocks) {
+      blk -= g.blocks;
+      g = p.seg[2];
+    }
   }
-  if (p.seqlens_out != nullptr) {
-    const int64_t b = (int64_t)blockIdx.x * kThreads + threadIdx.x;
-    if (b < p.batch) p.seqlens_out[b] = (int32_t)min((int64_t)(p.cu[b + 1] - p.cu[b]), p.cap);
+  const uint32_t row_vecs = (uint32_t)p.heads * kVecPerRow;
+  const int64_t n_vec = g.total * row_vecs;
+  const int64_t base = blk * (kFillPerThread * kThreads);
+  const int64_t t0 = base / row_vecs;
+  const uint32_t r0 = (uint32_t)(base - t0 * row_vecs);
+  uint4 v[kFillPerThread];
+#pragma unroll
+  for (int i = 0; i < kFillPerThread; ++i) {
+    const int64_t idx = base + i * kThreads + threadIdx.x;
+    if (idx < n_vec) v[i] = __ldg(g.src + idx);
+  }
+#pragma unroll
+  for (int i = 0; i < kFillPerThread; ++i) {
+    if (base + i * kThreads + threadIdx.x >= n_vec) break;
+    const uint32_t off = r0 + i * kThreads + threadIdx.x;
+    const int64_t t = t0 + off / row_vecs;
+    const int b = find_sequence(g.cu, p.batch, (int)t);
+    const int64_t pos = t - g.cu[b];
+    if (pos < g.cap) g.cache[((int64_t)b * g.cap + pos) * row_vecs + off % row_vecs] = v[i];
+  }
+  if (g.seqlens_out != nullptr)
+    for (int64_t b = blk * kThreads + threadIdx.x; b < p.batch; b += g.blocks * kThreads)
+      g.seqlens_out[b] = (int32_t)min((int64_t)(g.cu[b + 1] - g.cu[b]), g.cap);
+}
+
+struct Copy3Params {
+  const uint4* src[3];
+  uint4* dst[3];
+  int64_t end[3];              // running totals of the 16-byte vectors
+};
+// The query, key and value of a decode step into a captured graph's input buffers: one launch, where
+// three copies of a few KB took three launch slots of ~2 us in front of every replay.
+__global__ void __launch_bounds__(kThreads) copy3_kernel(const Copy3Params p) {
+  for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < p.end[2]; i += (int64_t)gridDim.x * kThreads) {
+    if (i < p.end[0]) p.dst[0][i] = p.src[0][i];
+    else if (i < p.end[1]) p.dst[1][i - p.end[0]] = p.src[1][i - p.end[0]];
+    else p.dst[2][i - p.end[1]] = p.src[2][i - p.end[1]];
   }
 }
 
@@ -168,27 +210,82 @@ __global__ void __launch_bounds__(kThreads) decode_append_kernel(const AppendPar
 
 using namespace ifv2;
 
-extern "C" int ifv2_cache_fill(const void* src, void* cache, const int32_t* cu_seqlens,
-                               int32_t* seqlens_out, int batch, int64_t total, int64_t capacity,
-                               int heads_k, int head_dim, void* stream) {
-  IFV2_REQUIRE(head_dim == kHeadDim, IFV2_ERR_UNSUPPORTED,
-               "cache_fill: head_dim %d not supported (only 128)", head_dim);
-  IFV2_REQUIRE(batch >= 1 && heads_k >= 1 && total >= 0 && capacity >= 1, IFV2_ERR_INVALID_ARG,
-               "cache_fill: bad size");
+static int fill_segment(FillSegment& g, const void* src, void* cache, const int32_t* cu_seqlens, int32_t* seqlens_out,
+                        int64_t total, int64_t capacity, int heads_k) {
+  IFV2_REQUIRE(total >= 0 && capacity >= 1, IFV2_ERR_INVALID_ARG, "cache_fill: bad size");
   IFV2_REQUIRE(cu_seqlens != nullptr && cache != nullptr && (src != nullptr || total == 0),
                IFV2_ERR_INVALID_ARG, "cache_fill: null pointer");
   IFV2_REQUIRE(reinterpret_cast<uintptr_t>(src) % 16 == 0 && reinterpret_cast<uintptr_t>(cache) % 16 == 0,
                IFV2_ERR_INVALID_ARG, "cache_fill: tensors must be 16-byte aligned");
   IFV2_REQUIRE(total <= INT32_MAX, IFV2_ERR_TOO_LARGE, "cache_fill: more than 2^31-1 rows");
-  FillParams p{static_cast<const uint4*>(src), static_cast<uint4*>(cache), cu_seqlens, seqlens_out,
-               batch, heads_k, total, capacity};
-  const int64_t n_vec = total * heads_k * kVecPerRow;
-  int64_t blocks = ceil_div64(n_vec > batch ? n_vec : batch, kThreads);
-  const int64_t min_blocks = ceil_div64(batch, kThreads);     // the threads that write seqlens_out
-  const int64_t cap = (int64_t)kNumSMs * 16;
-  if (blocks > cap) blocks = cap > min_blocks ? cap : min_blocks;
-  cache_fill_kernel<<<(int)blocks, kThreads, 0, (cudaStream_t)stream>>>(p);
+  g = FillSegment{static_cast<const uint4*>(src), static_cast<uint4*>(cache), cu_seqlens, seqlens_out, total, capacity, 0};
+  g.blocks = ceil_div64(total * heads_k * kVecPerRow, kFillPerThread * kThreads);
+  if (g.blocks < 1) g.blocks = 1;              // (the lengths are written in any case)
+  return IFV2_OK;
+}
+
+static int launch_fill(const FillParams& p, void* stream) {
+  int64_t blocks = 0;
+  for (const FillSegment& g : p.seg) blocks += g.blocks;
+  IFV2_REQUIRE(blocks <= INT32_MAX, IFV2_ERR_TOO_LARGE, "cache_fill: too many rows x heads");
+  cache_fill_kernel<<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(p);
   return check_launch("cache_fill");
+}
+
+extern "C" int ifv2_cache_fill(const void* src, void* cache, const int32_t* cu_seqlens,
+                               int32_t* seqlens_out, int batch, int64_t total, int64_t capacity,
+                               int heads_k, int head_dim, void* stream) {
+  IFV2_REQUIRE(head_dim == kHeadDim, IFV2_ERR_UNSUPPORTED,
+               "cache_fill: head_dim %d not supported (only 128)", head_dim);
+  IFV2_REQUIRE(batch >= 1 && heads_k >= 1, IFV2_ERR_INVALID_ARG, "cache_fill: bad size");
+  FillParams p{};
+  p.batch = batch;
+  p.heads = heads_k;
+  int rc = fill_segment(p.seg[0], src, cache, cu_seqlens, seqlens_out, total, capacity, heads_k);
+  return rc ? rc : launch_fill(p, stream);
+}
+
+extern "C" int ifv2_cache_fill_kv(const void* k, const void* v, const void* kc, void* k_cache, void* v_cache,
+                                  void* kc_cache, const int32_t* cu_seqlens, const int32_t* cu_seqlens_c,
+                                  int32_t* seqlens_out, int32_t* n_comp_out, int batch, int64_t total,
+                                  int64_t total_c, int64_t capacity, int64_t c_capacity, int heads_k,
+                                  int head_dim, void* stream) {
+  IFV2_REQUIRE(head_dim == kHeadDim, IFV2_ERR_UNSUPPORTED,
+               "cache_fill: head_dim %d not supported (only 128)", head_dim);
+  IFV2_REQUIRE(batch >= 1 && heads_k >= 1, IFV2_ERR_INVALID_ARG, "cache_fill: bad size");
+  FillParams p{};
+  p.batch = batch;
+  p.heads = heads_k;
+  int rc = fill_segment(p.seg[0], k, k_cache, cu_seqlens, seqlens_out, total, capacity, heads_k);
+  if (rc) return rc;
+  rc = fill_segment(p.seg[1], v, v_cache, cu_seqlens, nullptr, total, capacity, heads_k);
+  if (rc) return rc;
+  rc = fill_segment(p.seg[2], kc, kc_cache, cu_seqlens_c, n_comp_out, total_c, c_capacity, heads_k);
+  return rc ? rc : launch_fill(p, stream);
+}
+
+extern "C" int ifv2_copy3(const void* src0, void* dst0, int64_t bytes0, const void* src1, void* dst1, int64_t bytes1,
+                          const void* src2, void* dst2, int64_t bytes2, void* stream) {
+  const void* src[3] = {src0, src1, src2};
+  void* dst[3] = {dst0, dst1, dst2};
+  const int64_t bytes[3] = {bytes0, bytes1, bytes2};
+  Copy3Params p;
+  int64_t n = 0;
+  for (int i = 0; i < 3; ++i) {
+    IFV2_REQUIRE(bytes[i] >= 0 && bytes[i] % 16 == 0, IFV2_ERR_INVALID_ARG, "copy3: sizes must be multiples of 16 bytes");
+    IFV2_REQUIRE((src[i] && dst[i]) || bytes[i] == 0, IFV2_ERR_INVALID_ARG, "copy3: null pointer");
+    IFV2_REQUIRE((reinterpret_cast<uintptr_t>(src[i]) | reinterpret_cast<uintptr_t>(dst[i])) % 16 == 0,
+                 IFV2_ERR_INVALID_ARG, "copy3: tensors must be 16-byte aligned");
+    p.src[i] = static_cast<const uint4*>(src[i]);
+    p.dst[i] = static_cast<uint4*>(dst[i]);
+    n += bytes[i] / 16;
+    p.end[i] = n;
+  }
+  if (n == 0) return IFV2_OK;
+  int64_t blocks = ceil_div64(n, kThreads);
+  if (blocks > (int64_t)kNumSMs * 8) blocks = (int64_t)kNumSMs * 8;
+  copy3_kernel<<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(p);
+  return check_launch("copy3");
 }
 
 extern "C" int ifv2_decode_append(const void* k_new, const void* v_new, void* k_cache, void* v_cache,

@@ -348,11 +348,7 @@ def compress_keys_append(k_cache: torch.Tensor, cache_seqlens: torch.Tensor, kc_
                   kernel_size, kernel_stride, _stream(k_cache.device))
 
 
-def cache_fill(src: torch.Tensor, cache: torch.Tensor, cu_seqlens: torch.Tensor,
-               seqlens_out: Optional[torch.Tensor] = None) -> None:
-    """Copy the packed rows of every sequence (src: (total, Hk, 128) bf16, cu_seqlens (B+1) int32)
-    to rows [0, len_b) of its slot of cache (B, capacity, Hk, 128), in place; rows past the
-    capacity are dropped.  seqlens_out (B,) int32, optional: min(len_b, capacity)."""
+def _check_fill(src, cache, cu_seqlens, seqlens_out):
     _require_cuda(src, "src")
     _require_cuda(cache, "cache")
     if (src.dtype != torch.bfloat16 or cache.dtype != torch.bfloat16 or src.dim() != 3 or cache.dim() != 4
@@ -361,11 +357,53 @@ def cache_fill(src: torch.Tensor, cache: torch.Tensor, cu_seqlens: torch.Tensor,
     assert cu_seqlens.dtype == torch.int32 and cu_seqlens.numel() == cache.shape[0] + 1
     if seqlens_out is not None:
         assert seqlens_out.dtype == torch.int32 and seqlens_out.is_contiguous() and seqlens_out.numel() == cache.shape[0]
+
+
+def cache_fill_kv(k: torch.Tensor, v: torch.Tensor, kc: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
+                  kc_cache: torch.Tensor, cu_seqlens: torch.Tensor, cu_seqlens_c: torch.Tensor,
+                  seqlens_out: Optional[torch.Tensor] = None, n_comp_out: Optional[torch.Tensor] = None) -> None:
+    """`cache_fill` of the keys, the values (both by cu_seqlens) and the compressed keys (by
+    cu_seqlens_c) of a prefill in one launch."""
+    _check_fill(k, k_cache, cu_seqlens, seqlens_out)
+    _check_fill(v, v_cache, cu_seqlens, None)
+    _check_fill(kc, kc_cache, cu_seqlens_c, n_comp_out)
+    if v.shape != k.shape or v_cache.shape != k_cache.shape or kc.shape[1:] != k.shape[1:] or kc_cache.shape[0] != k_cache.shape[0]:
+        raise ValueError("cache_fill_kv: the three tensors must agree in batch and heads, keys and values in all sizes")
+    k, v, kc = k.contiguous(), v.contiguous(), kc.contiguous()
+    ptr = lambda t: t.data_ptr() if t is not None else None
+    with _on(k.device):
+        _lib.call("ifv2_cache_fill_kv", k.data_ptr(), v.data_ptr(), kc.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
+                  kc_cache.data_ptr(), cu_seqlens.contiguous().data_ptr(), cu_seqlens_c.contiguous().data_ptr(),
+                  ptr(seqlens_out), ptr(n_comp_out), k_cache.shape[0], k.shape[0], kc.shape[0], k_cache.shape[1],
+                  kc_cache.shape[1], k_cache.shape[2], k_cache.shape[3], _stream(k.device))
+
+
+def cache_fill(src: torch.Tensor, cache: torch.Tensor, cu_seqlens: torch.Tensor,
+               seqlens_out: Optional[torch.Tensor] = None) -> None:
+    """Copy the packed rows of every sequence (src: (total, Hk, 128) bf16, cu_seqlens (B+1) int32)
+    to rows [0, len_b) of its slot of cache (B, capacity, Hk, 128), in place; rows past the
+    capacity are dropped.  seqlens_out (B,) int32, optional: min(len_b, capacity)."""
+    _check_fill(src, cache, cu_seqlens, seqlens_out)
     src = src.contiguous()
     with _on(src.device):
         _lib.call("ifv2_cache_fill", src.data_ptr(), cache.data_ptr(), cu_seqlens.contiguous().data_ptr(),
                   seqlens_out.data_ptr() if seqlens_out is not None else None, cache.shape[0],
                   src.shape[0], cache.shape[1], cache.shape[2], cache.shape[3], _stream(src.device))
+
+
+def copy3(pairs) -> None:
+    """dst.copy_(src) for three (dst, src) pairs of equally many elements.  One launch when nothing has
+    to be converted, moved between devices or gathered; `copy_` one by one otherwise."""
+    dev = pairs[0][0].device
+    if all(s.dtype == d.dtype and s.device == dev and d.device == dev and s.numel() == d.numel() and s.is_contiguous()
+           and d.is_contiguous() and not s.requires_grad and type(s) is torch.Tensor and (s.data_ptr() | d.data_ptr()) % 16 == 0
+           and s.numel() * s.element_size() % 16 == 0 for d, s in pairs):
+        args = [x for d, s in pairs for x in (s.data_ptr(), d.data_ptr(), s.numel() * s.element_size())]
+        with _on(dev):
+            _lib.call("ifv2_copy3", *args, _stream(dev))
+        return
+    for d, s in pairs:
+        d.copy_(s.reshape(d.shape))
 
 
 def decode_append(k_new: torch.Tensor, v_new: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,

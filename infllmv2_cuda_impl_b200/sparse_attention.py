@@ -77,9 +77,12 @@ class DecodeCache:
 
     def fill(self, k, v, kc, cu_seqlens, cu_seqlens_c, max_seqlen, kc2=None, cu_seqlens_c2=None):
         """Load the caches from packed prefill tensors (rows past the capacity are dropped)."""
-        ops.cache_fill(k, self.k, cu_seqlens, self.seqlens)
-        ops.cache_fill(v, self.v, cu_seqlens)
-        ops.cache_fill(kc, self.kc, cu_seqlens_c, self.n_comp)
+        if k.shape == v.shape:
+            ops.cache_fill_kv(k, v, kc, self.k, self.v, self.kc, cu_seqlens, cu_seqlens_c, self.seqlens, self.n_comp)
+        else:                                      # (rows of one tensor past the last sequence)
+            ops.cache_fill(k, self.k, cu_seqlens, self.seqlens)
+            ops.cache_fill(v, self.v, cu_seqlens)
+            ops.cache_fill(kc, self.kc, cu_seqlens_c, self.n_comp)
         if self.kc2 is not None:
             ops.cache_fill(kc2, self.kc2, cu_seqlens_c2, self.n_comp2)
         self.max_len = min(int(max_seqlen), self.capacity)
@@ -226,9 +229,7 @@ class SparseAttention:
         def step(q, k_new, v_new):
             if cache.max_len >= cache.capacity:
                 raise RuntimeError("DecodeCache is full")
-            q_in.copy_(q.reshape(q_in.shape))
-            k_in.copy_(k_new.reshape(k_in.shape))
-            v_in.copy_(v_new.reshape(v_in.shape))
+            ops.copy3(((q_in, q), (k_in, k_new), (v_in, v_new)))
             graph.replay()
             cache.max_len += 1
             return out

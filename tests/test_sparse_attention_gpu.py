@@ -299,3 +299,44 @@ def test_cache_capacity_limits():
     assert torch.equal(cache.k[0], before[0]) and torch.equal(cache.k[1, 40].cpu(), kn[1].cpu())
     with pytest.raises(RuntimeError):
         infllm_v2.SparseAttention(cfg).decode(det_tensor((2, HQ, D), 74, 0.5).to(DEV), kn, kn, cache)
+
+
+@pytest.mark.parametrize("hk", [1, 2, 3, 8])
+@pytest.mark.parametrize("lens,cap", [([1], 1), ([31, 0, 700], 400), ([64, 65, 129], 200), ([5] * 40, 5)])
+def test_cache_fill_in_one_launch(hk, lens, cap):
+    """Keys, values and compressed keys together: CTA borders inside rows (3 heads), empty sequences, no
+    compressed key at all, rows past the capacity."""
+    total = sum(lens)
+    k, v = det_tensor((total, hk, D), 1, device=DEV), det_tensor((total, hk, D), 2, device=DEV)
+    kc, cu_c = infllm_v2.compress_keys(k, cu(lens, DEV))
+    cfg = _config()
+    got, exp = (infllm_v2.DecodeCache(len(lens), cap, hk, cfg, DEV) for _ in range(2))
+    got.fill(k, v, kc, cu(lens, DEV), cu_c, max(lens))
+    for src, dst, c, n in ((k, exp.k, cu(lens).tolist(), exp.seqlens), (v, exp.v, cu(lens).tolist(), None),
+                           (kc, exp.kc, cu_c.tolist(), exp.n_comp)):
+        for b in range(len(lens)):
+            m = min(c[b + 1] - c[b], dst.shape[1])
+            dst[b, :m] = src[c[b]:c[b] + m]
+            if n is not None:
+                n[b] = m
+    for name in ("k", "v", "kc", "seqlens", "n_comp"):
+        assert torch.equal(getattr(got, name), getattr(exp, name)), name
+
+
+@pytest.mark.parametrize("form", ["plain", "fp32", "strided", "offset", "4d"])
+def test_graph_step_takes_inputs_of_any_form(form):
+    """The step's arguments reach the graph's buffers in one launch, or converted and gathered."""
+    cfg, b = _config(), 3
+    step_in = [det_tensor((b, h, D), 90 + i, 0.25, device=DEV) for i, h in enumerate((HQ, HK, HK))]
+    outs = []
+    for given in (form, "plain"):
+        cache = infllm_v2.DecodeCache(b, 300, HK, cfg, DEV)
+        k, v = det_tensor((b * 100, HK, D), 95, 0.25, device=DEV), det_tensor((b * 100, HK, D), 96, device=DEV)
+        kc, cu_c = infllm_v2.compress_keys(k, cu([100] * b, DEV))
+        cache.fill(k, v, kc, cu([100] * b, DEV), cu_c, 100)
+        step = infllm_v2.SparseAttention(cfg).capture_decode(cache)
+        x = {"plain": lambda t: t, "fp32": lambda t: t.float(), "4d": lambda t: t[:, None],
+             "strided": lambda t: t.transpose(0, 1).contiguous().transpose(0, 1),
+             "offset": lambda t: torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)}[given]
+        outs.append([step(*(x(t) for t in step_in)).clone(), cache.k.clone(), cache.v.clone()])
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
