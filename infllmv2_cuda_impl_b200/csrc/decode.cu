@@ -3,7 +3,7 @@
 // With a single token the query tile is 16 rows, far too small for a tcgen05 tile, and the work
 // is HBM-bound: every selected 64-key block is read once (K and V, 32 KB) and used by 16 rows.
 // So this kernel is built around bandwidth: the selected blocks of one (sequence, KV head) are
-// split over several CTAs (as many as fill the SMs in ONE wave, three CTAs per SM), each warp
+// split over several CTAs (as many as fill the SMs in ONE wave, two CTAs per SM), each warp
 // streams its blocks as 32-key units into swizzled shared memory (K and V of the next unit are
 // fetched as soon as the current product has consumed its tile), the 16 x 32 products run on
 // mma.sync m16n8k16 (exactly one M tile), and the per-split (max, sum, O) partials are merged by
@@ -29,10 +29,11 @@ constexpr int kMaxSplits = 16;                          // CTAs per (sequence, K
 constexpr int kWarps = 4;
 constexpr int kWarpSmem = 2 * kUnit * 256;              // one K tile + one V tile per warp
 constexpr int kThreads = kWarps * 32;
-// resident CTAs per SM the split kernel is compiled for: 3 (168 registers, 12 warps) measured 4 %
-// faster than 2 (212 registers) on the batch-64 decode step -- more copies in flight per SM
+// Resident CTAs per SM the split kernel is compiled for, and slots that the split count below fills.  Two
+// (no spills, fewer and longer CTAs) against three: batch 64 at 32k-131k tokens 121.9 us a step against
+// 124.4, batch 12 with 8 KV heads 72.5 / 74.5, paged batch 16 30.6 / 31.5, batch 1 32.4 / 33.4.
 #ifndef IFV2_DECODE_CTAS_PER_SM
-#define IFV2_DECODE_CTAS_PER_SM 3
+#define IFV2_DECODE_CTAS_PER_SM 2
 #endif
 constexpr int kPartialFloats = kHeadDim + 4;            // O row, running max (log2 units), sum, pad (16-byte rows)
 constexpr float kLog2e = 1.4426950408889634f;
@@ -463,16 +464,31 @@ __global__ void __launch_bounds__(256) decode_combine_kernel(const DecodeParams 
     mmax = fmaxf(mmax, ms[s]);
   }
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, lsum = 0.f;
+  // bound by latency: the loads of kBatch splits are issued together (one by one they were a trip to
+  // memory per split, most of this kernel's time with 13-16 splits)
+  constexpr int kBatch = 8;
 #pragma unroll
-  for (int s = 0; s < kMaxSplits; ++s) {
-    if (s >= p.splits) break;
-    const float f = (ms[s] == -INFINITY) ? 0.f : exp2f(ms[s] - mmax);
-    const float* ps = src + (size_t)s * 16 * kPartialFloats;
-    lsum += f * ps[kHeadDim + 1];
-    const float4 a = *reinterpret_cast<const float4*>(ps + c0);
-    const float4 bq = *reinterpret_cast<const float4*>(ps + c0 + 4);
-    acc[0] += f * a.x; acc[1] += f * a.y; acc[2] += f * a.z; acc[3] += f * a.w;
-    acc[4] += f * bq.x; acc[5] += f * bq.y; acc[6] += f * bq.z; acc[7] += f * bq.w;
+  for (int s0 = 0; s0 < kMaxSplits; s0 += kBatch) {
+    if (s0 >= p.splits) break;
+    float4 a[kBatch], bq[kBatch];
+    float ls[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      if (s0 + u < p.splits) {
+        const float* ps = src + (size_t)(s0 + u) * 16 * kPartialFloats;
+        a[u] = *reinterpret_cast<const float4*>(ps + c0);
+        bq[u] = *reinterpret_cast<const float4*>(ps + c0 + 4);
+        ls[u] = ps[kHeadDim + 1];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      if (s0 + u >= p.splits) break;
+      const float f = (ms[s0 + u] == -INFINITY) ? 0.f : exp2f(ms[s0 + u] - mmax);
+      lsum += f * ls[u];
+      acc[0] += f * a[u].x; acc[1] += f * a[u].y; acc[2] += f * a[u].z; acc[3] += f * a[u].w;
+      acc[4] += f * bq[u].x; acc[5] += f * bq[u].y; acc[6] += f * bq[u].z; acc[7] += f * bq[u].w;
+    }
   }
   const float inv = (lsum > 0.f) ? 1.f / lsum : 0.f;
   const int64_t qrow = (int64_t)b * p.heads_q + h * kGroup + row;
@@ -605,9 +621,10 @@ static int decode_impl(const void* q, void* k_cache, void* v_cache, const void* 
   p.cache_batch_idx = cache_batch_idx;
   p.leftpad = cache_leftpad;
   p.scale_log2 = softmax_scale * kLog2e;
-  // One wave: as many CTAs per (sequence, KV head) as still fit the SMs all at once.  A launch
-  // that spills into a second, mostly empty wave takes twice as long (measured at batch 64 x 2 KV
-  // heads, top-64: 3 splits = 384 CTAs on 444 slots 62 us, 4 splits = 512 CTAs 78 us, 8 splits 79 us).
+  // One wave: as many CTAs per (sequence, KV head) as still fit the SMs all at once.  A launch that
+  // spills into a second, mostly empty wave takes longer (a step at batch 64 x 2 KV heads, top-64: 2
+  // splits = 256 CTAs on 296 slots 122 us, 4 splits 136, 8 splits 141; batch 16: 8-10 splits 32 us, 4
+  // splits 39, 16 splits 39).
   const int64_t slots = (int64_t)kNumSMs * IFV2_DECODE_CTAS_PER_SM;
   const int64_t pairs = (int64_t)batch * heads_k;
   int splits = (int)(slots / pairs);
