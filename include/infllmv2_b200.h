@@ -436,6 +436,20 @@ int ifv2_decode_paged(const void* q, void* k_cache, void* v_cache, const void* k
                       const int32_t* cache_batch_idx, const int32_t* cache_leftpad,
                       float softmax_scale, void* workspace, int64_t workspace_bytes, void* stream);
 
+/* ifv2_decode_paged together with what goes before it, in one launch and one call: ifv2_topk_to_uint64
+ * of block lists topk_idx (batch, heads_k, topk) into mask (batch, heads_k, mask_words; at most 4096
+ * words), ifv2_decode_rotary of q into q_rotated and of the new key, and the append.  Each part is
+ * optional: topk_idx null = mask is given (or null), rotary_cos null = no rotation, k_new null = no
+ * append. */
+int ifv2_decode_prepared(const void* q, void* q_rotated, void* k_cache, void* v_cache, const void* k_new,
+                         const void* v_new, const void* rotary_cos, const void* rotary_sin, int rotary_dim,
+                         int seqlen_ro, int interleaved, const int32_t* topk_idx, int topk, void* out, float* lse,
+                         int64_t* mask, int mask_words, const int32_t* cache_seqlens, int batch, int heads_q,
+                         int heads_k, int head_dim, int64_t cache_capacity, int64_t cache_batch_stride,
+                         const int32_t* block_table, int block_table_stride, int page_size,
+                         const int32_t* cache_batch_idx, const int32_t* cache_leftpad, float softmax_scale,
+                         void* workspace, int64_t workspace_bytes, void* stream);
+
 /* ---------------------------------------------------------------- self-tests -------------- */
 /* Test infrastructure shipped in the library so that a deployment can check the tensor-core
  * building blocks on its own GPU; not part of the attention path.  No counterpart in the

@@ -82,6 +82,9 @@ SIGNATURES = {
     "ifv2_decode_paged": [c_void_p] * 8 + [c_int, c_void_p, c_int, c_int, c_int, c_int, c_int64, c_int64,
                                            c_void_p, c_int, c_int, c_void_p, c_void_p, c_float,
                                            c_void_p, c_int64, c_void_p],
+    "ifv2_decode_prepared": [c_void_p] * 8 + [c_int] * 3 + [c_void_p, c_int] + [c_void_p] * 3 +
+                            [c_int, c_void_p, c_int, c_int, c_int, c_int, c_int64, c_int64, c_void_p, c_int, c_int,
+                             c_void_p, c_void_p, c_float, c_void_p, c_int64, c_void_p],
 }
 _INT64_RETURNS = {
     "ifv2_sparse_attn_bwd_workspace_bytes": [c_int64, c_int, c_int],

@@ -645,32 +645,40 @@ def infllmv2_attn_with_kvcache(
     for c in (k_cache, v_cache):
         if c.stride(2) != d or c.stride(1) != nheads_k * d:
             raise RuntimeError("infllmv2_attn_with_kvcache: caches must be dense in (seqlen, heads, d)")
-    mask = None
+    words = ((cap + BLOCK_N - 1) // BLOCK_N + 63) // 64
+    mask = lists = None
     if block_mask is not None:
         # an already packed selection (ops.decode_select): (batch, nheads_k, [1,] words) int64
-        words = ((cap + BLOCK_N - 1) // BLOCK_N + 63) // 64
         if topk_idx is not None or block_mask.dtype != torch.int64 or block_mask.numel() != batch * nheads_k * words:
             raise ValueError("infllmv2_attn_with_kvcache: block_mask must be (batch, nheads_k, 1, "
                              f"{words}) int64 and excludes topk_idx")
         mask = block_mask.contiguous().view(batch, nheads_k, 1, words)
     elif topk_idx is not None:
         assert topk_idx.dtype == torch.int32
-        mask, _ = topk_to_uint64(topk_idx, cap, BLOCK_N)
+        n_idx = topk_idx.shape[-1] if topk_idx.dim() in (3, 4) else 0
+        if topk_idx.is_cuda and n_idx > 0 and topk_idx.numel() == batch * nheads_k * n_idx and words <= 4096:
+            lists = topk_idx.contiguous()           # packed by the launch that rotates and appends
+            mask = torch.empty(batch, nheads_k, 1, words, dtype=torch.int64, device=q.device)
+        else:
+            mask, _ = topk_to_uint64(topk_idx, cap, BLOCK_N)
     q2 = q.reshape(batch, nheads, d).contiguous()
-    if rotary_cos is not None and k is not None:
+    rotate = rotary_cos is not None and k is not None
+    if rotate:
         # as in the reference, the rotation applies to the appended key and to the query, both at
         # the position of the append; without an append nothing is rotated
         if rotary_cos.dtype != q.dtype or rotary_cos.shape != rotary_sin.shape or rotary_cos.dim() != 2:
             raise ValueError("infllmv2_attn_with_kvcache: rotary_cos / rotary_sin must be "
                              "(seqlen_ro, rotary_dim / 2) in the dtype of q")
-        k2 = k.reshape(batch, nheads_k, d).contiguous()
-        q_rot, k_rot = torch.empty_like(q2), torch.empty_like(k2)
-        with _on(q.device):
-            _lib.call("ifv2_decode_rotary", q2.data_ptr(), k2.data_ptr(), q_rot.data_ptr(), k_rot.data_ptr(),
-                      rotary_cos.contiguous().data_ptr(), rotary_sin.contiguous().data_ptr(),
-                      cache_seqlens.data_ptr(), batch, nheads, nheads_k, d, 2 * rotary_cos.shape[1],
-                      rotary_cos.shape[0], int(bool(rotary_interleaved)), _stream(q.device))
-        q2, k = q_rot, k_rot
+        if rotary_cos.shape[0] < 1:
+            raise ValueError("infllmv2_attn_with_kvcache: rotary_cos / rotary_sin hold no position")
+        rotary_cos, rotary_sin = rotary_cos.contiguous(), rotary_sin.contiguous()
+        k = k.reshape(batch, nheads_k, d)
+    q_rot = torch.empty_like(q2) if rotate else None
+    k = k.contiguous() if k is not None else None
+    v = v.contiguous() if v is not None else None
+    cache_batch_idx = cache_batch_idx.contiguous() if cache_batch_idx is not None else None
+    cache_leftpad = cache_leftpad.contiguous() if cache_leftpad is not None else None
+    ptr = lambda t: t.data_ptr() if t is not None else None
     out = torch.empty_like(q2)
     lse = torch.empty(batch, nheads, dtype=torch.float32, device=q.device)
     lib = _lib.load()
@@ -678,14 +686,12 @@ def infllmv2_attn_with_kvcache(
     ws_bytes = int(lib.ifv2_decode_workspace_bytes(batch, nheads, d, max_blocks))
     ws = torch.empty(max(ws_bytes, 16), dtype=torch.uint8, device=q.device)
     with _on(q.device):
-        _lib.call("ifv2_decode_paged", q2.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(),
-                  k.contiguous().data_ptr() if k is not None else None,
-                  v.contiguous().data_ptr() if v is not None else None, out.data_ptr(),
-                  lse.data_ptr(), mask.data_ptr() if mask is not None else None,
-                  mask.shape[-1] if mask is not None else 0, cache_seqlens.data_ptr(), batch,
-                  nheads, nheads_k, d, cap, k_cache.stride(0), bt_ptr, bt_stride, page_size,
-                  cache_batch_idx.contiguous().data_ptr() if cache_batch_idx is not None else None,
-                  cache_leftpad.contiguous().data_ptr() if cache_leftpad is not None else None,
-                  float(softmax_scale), ws.data_ptr(), ws_bytes, _stream(q.device))
+        _lib.call("ifv2_decode_prepared", q2.data_ptr(), ptr(q_rot), k_cache.data_ptr(), v_cache.data_ptr(), ptr(k), ptr(v),
+                  rotary_cos.data_ptr() if rotate else None, rotary_sin.data_ptr() if rotate else None,
+                  2 * rotary_cos.shape[1] if rotate else 0, rotary_cos.shape[0] if rotate else 0,
+                  int(bool(rotary_interleaved)), ptr(lists), lists.shape[-1] if lists is not None else 0, out.data_ptr(),
+                  lse.data_ptr(), ptr(mask), mask.shape[-1] if mask is not None else 0, cache_seqlens.data_ptr(), batch,
+                  nheads, nheads_k, d, cap, k_cache.stride(0), bt_ptr, bt_stride, page_size, ptr(cache_batch_idx),
+                  ptr(cache_leftpad), float(softmax_scale), ws.data_ptr(), ws_bytes, _stream(q.device))
     out = out.view(batch, 1, nheads, d)
     return (out, lse.view(batch, nheads, 1)) if return_softmax_lse else out

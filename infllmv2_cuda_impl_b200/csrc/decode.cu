@@ -558,6 +558,80 @@ __global__ void decode_rotary_kernel(const __nv_bfloat16* __restrict__ q, const 
   }
 }
 
+// What a decode step with given block lists does before the attention, in one launch: pack the lists into
+// mask rows, rotate the query and the new key, append the new key and value.  One CTA per (sequence, KV
+// head).  Three launches of 2-6 us (and three calls from the host, which bounds such a step) otherwise;
+// the arithmetic is that of topk_to_uint64_kernel, decode_rotary_kernel and decode_append_kernel.
+struct PrepareParams {
+  const __nv_bfloat16* q;          // (batch, heads_q, 128), rotated into q_out; null = no rotation
+  __nv_bfloat16* q_out;
+  const __nv_bfloat16* k_new;      // (batch, heads_k, 128) or null = no append
+  const __nv_bfloat16* v_new;
+  const __nv_bfloat16* cos_t;      // (seqlen_ro, rotary_dim / 2)
+  const __nv_bfloat16* sin_t;
+  const int32_t* topk_idx;         // (batch, heads_k, topk) or null
+  unsigned long long* mask;        // (batch, heads_k, words)
+  int topk, words, rotary_dim, seqlen_ro, interleaved;
+};
+
+__device__ __forceinline__ void rotate_pair(const PrepareParams& r, const __nv_bfloat16* src, __nv_bfloat16* dst, int i,
+                                            int64_t pos) {
+  const int half = r.rotary_dim / 2;
+  const bool in = i < half;                             // (features past rotary_dim pass through, two at a time)
+  const int i0 = in ? (r.interleaved ? 2 * i : i) : r.rotary_dim + 2 * (i - half);
+  const int i1 = in && !r.interleaved ? i + half : i0 + 1;
+  float x0 = __bfloat162float(src[i0]), x1 = __bfloat162float(src[i1]);
+  if (in) {
+    const float c = __bfloat162float(r.cos_t[pos * half + i]), sn = __bfloat162float(r.sin_t[pos * half + i]);
+    const float re = x0 * c - x1 * sn, im = x0 * sn + x1 * c;
+    x0 = re;
+    x1 = im;
+  }
+  dst[i0] = __float2bfloat16_rn(x0);
+  dst[i1] = __float2bfloat16_rn(x1);
+}
+
+__global__ void __launch_bounds__(256) decode_prepare_kernel(const PrepareParams r, __nv_bfloat16* k_cache,
+                                                             __nv_bfloat16* v_cache, const int32_t* cache_seqlens,
+                                                             int heads_k, int64_t capacity, int64_t batch_stride,
+                                                             const int32_t* block_table, int bt_stride, int page_size,
+                                                             const int32_t* cache_batch_idx) {
+  extern __shared__ unsigned long long row_words[];
+  const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+  const int64_t pair = (int64_t)b * heads_k + h;
+  const int64_t len = cache_seqlens[b];
+  const int64_t ro = r.q != nullptr ? min(max(len, (int64_t)0), (int64_t)r.seqlen_ro - 1) : 0;
+  if (r.topk_idx != nullptr) {
+    for (int w = tid; w < r.words; w += 256) row_words[w] = 0ull;
+    __syncthreads();
+    for (int i = tid; i < r.topk; i += 256) {
+      const int v = r.topk_idx[pair * r.topk + i];
+      if (v >= 0 && v < r.words * 64) atomicOr(&row_words[v >> 6], 1ull << (v & 63));
+    }
+  }
+  if (r.q != nullptr)
+    for (int i = tid; i < kGroup * (kHeadDim / 2); i += 256) {
+      const int64_t row = (pair * kGroup + i / (kHeadDim / 2)) * kHeadDim;
+      rotate_pair(r, r.q + row, r.q_out + row, i % (kHeadDim / 2), ro);
+    }
+  if (r.k_new != nullptr && len >= 0 && len < capacity) {        // no room: the host documents this as an error
+    const int slot = cache_batch_idx ? cache_batch_idx[b] : b;
+    const int64_t off = cache_row_offset(block_table, bt_stride, page_size, batch_stride, (int64_t)heads_k * kHeadDim, b,
+                                         slot, len) + (int64_t)h * kHeadDim;
+    if (r.q != nullptr) {
+      if (tid < kHeadDim / 2) rotate_pair(r, r.k_new + pair * kHeadDim, k_cache + off, tid, ro);
+    } else if (tid < kHeadDim / 8) {
+      reinterpret_cast<uint4*>(k_cache + off)[tid] = reinterpret_cast<const uint4*>(r.k_new + pair * kHeadDim)[tid];
+    }
+    if (tid >= 64 && tid < 64 + kHeadDim / 8)
+      reinterpret_cast<uint4*>(v_cache + off)[tid - 64] = reinterpret_cast<const uint4*>(r.v_new + pair * kHeadDim)[tid - 64];
+  }
+  if (r.topk_idx != nullptr) {
+    __syncthreads();
+    for (int w = tid; w < r.words; w += 256) r.mask[pair * r.words + w] = row_words[w];
+  }
+}
+
 static int decode_impl(const void* q, void* k_cache, void* v_cache, const void* k_new,
                        const void* v_new, void* out, float* lse, const int64_t* mask,
                        int mask_words, const int32_t* cache_seqlens, int batch, int heads_q,
@@ -565,7 +639,7 @@ static int decode_impl(const void* q, void* k_cache, void* v_cache, const void* 
                        int64_t cache_batch_stride, const int32_t* block_table,
                        int block_table_stride, int page_size, const int32_t* cache_batch_idx,
                        const int32_t* cache_leftpad, float softmax_scale, void* workspace,
-                       int64_t workspace_bytes, void* stream) {
+                       int64_t workspace_bytes, void* stream, const PrepareParams* prepare = nullptr) {
   IFV2_REQUIRE(head_dim == kHeadDim, IFV2_ERR_UNSUPPORTED, "decode: head_dim %d not supported (only 128)",
                head_dim);
   IFV2_REQUIRE(heads_k >= 1 && heads_q == heads_k * kGroup, IFV2_ERR_UNSUPPORTED,
@@ -594,7 +668,14 @@ static int decode_impl(const void* q, void* k_cache, void* v_cache, const void* 
                "decode: workspace must be 16-byte aligned");
   IFV2_REQUIRE(batch <= 65535 && heads_k <= 65535, IFV2_ERR_TOO_LARGE, "decode: batch or heads_k > 65535");
   cudaStream_t st = (cudaStream_t)stream;
-  if (k_new != nullptr) {
+  if (prepare != nullptr) {
+    decode_prepare_kernel<<<dim3(heads_k, batch), 256, prepare->topk_idx ? (size_t)prepare->words * 8 : 0, st>>>(
+        *prepare, static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), cache_seqlens, heads_k,
+        cache_capacity, cache_batch_stride, block_table, block_table_stride, page_size > 0 ? page_size : 1, cache_batch_idx);
+    int rc = check_launch("decode_prepare");
+    if (rc) return rc;
+    if (prepare->q != nullptr) q = prepare->q_out;
+  } else if (k_new != nullptr) {
     decode_append_kernel<<<batch, 128, 0, st>>>(
         static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache),
         static_cast<const __nv_bfloat16*>(k_new), static_cast<const __nv_bfloat16*>(v_new),
@@ -694,6 +775,46 @@ extern "C" int ifv2_decode_paged(const void* q, void* k_cache, void* v_cache, co
                      batch, heads_q, heads_k, head_dim, cache_capacity, cache_batch_stride, block_table,
                      block_table_stride, page_size, cache_batch_idx, cache_leftpad, softmax_scale,
                      workspace, workspace_bytes, stream);
+}
+
+extern "C" int ifv2_decode_prepared(const void* q, void* q_rotated, void* k_cache, void* v_cache,
+                                    const void* k_new, const void* v_new, const void* rotary_cos,
+                                    const void* rotary_sin, int rotary_dim, int seqlen_ro, int interleaved,
+                                    const int32_t* topk_idx, int topk, void* out, float* lse, int64_t* mask,
+                                    int mask_words, const int32_t* cache_seqlens, int batch, int heads_q,
+                                    int heads_k, int head_dim, int64_t cache_capacity,
+                                    int64_t cache_batch_stride, const int32_t* block_table,
+                                    int block_table_stride, int page_size, const int32_t* cache_batch_idx,
+                                    const int32_t* cache_leftpad, float softmax_scale, void* workspace,
+                                    int64_t workspace_bytes, void* stream) {
+  const bool rotate = rotary_cos != nullptr;
+  IFV2_REQUIRE(rotate == (rotary_sin != nullptr) &&
+                   (!rotate || batch == 0 || (q_rotated && k_new && q_rotated != q && seqlen_ro >= 1)), IFV2_ERR_INVALID_ARG,
+               "decode_prepared: rotation takes both tables, a new key and a buffer of its own for the query");
+  IFV2_REQUIRE(!rotate || (rotary_dim >= 0 && rotary_dim <= kHeadDim && rotary_dim % 16 == 0), IFV2_ERR_INVALID_ARG,
+               "decode_prepared: rotary_dim must be a multiple of 16 and <= head_dim");
+  IFV2_REQUIRE(topk_idx == nullptr || (mask != nullptr && topk >= 0 && mask_words >= 1), IFV2_ERR_INVALID_ARG,
+               "decode_prepared: block lists need a mask buffer");
+  IFV2_REQUIRE(topk_idx == nullptr || mask_words <= 4096, IFV2_ERR_TOO_LARGE,
+               "decode_prepared: more than 4096 mask words (use ifv2_topk_to_uint64)");
+  PrepareParams r;
+  r.q = rotate ? static_cast<const __nv_bfloat16*>(q) : nullptr;
+  r.q_out = static_cast<__nv_bfloat16*>(q_rotated);
+  r.k_new = static_cast<const __nv_bfloat16*>(k_new);
+  r.v_new = static_cast<const __nv_bfloat16*>(v_new);
+  r.cos_t = static_cast<const __nv_bfloat16*>(rotary_cos);
+  r.sin_t = static_cast<const __nv_bfloat16*>(rotary_sin);
+  r.topk_idx = topk_idx;
+  r.mask = reinterpret_cast<unsigned long long*>(mask);
+  r.topk = topk;
+  r.words = mask_words;
+  r.rotary_dim = rotary_dim;
+  r.seqlen_ro = seqlen_ro;
+  r.interleaved = interleaved ? 1 : 0;
+  return decode_impl(q, k_cache, v_cache, k_new, v_new, out, lse, mask, mask_words, cache_seqlens,
+                     batch, heads_q, heads_k, head_dim, cache_capacity, cache_batch_stride, block_table,
+                     block_table_stride, page_size, cache_batch_idx, cache_leftpad, softmax_scale,
+                     workspace, workspace_bytes, stream, topk_idx || k_new ? &r : nullptr);
 }
 
 extern "C" int ifv2_decode_rotary(const void* q, const void* k_new, void* q_out, void* k_out,

@@ -244,3 +244,52 @@ def test_decode_block_lists(n_blk, picks):
     mx, mr = err_stats(out, ref)
     assert mx <= MAX_ABS and mr <= MEAN_REL, (mx, mr)
     assert (lse.view(hk, 16) - s.logsumexp(-1)).abs().max() < 2e-2
+
+
+@pytest.mark.parametrize("lists", [None, 1, 16, 300])
+@pytest.mark.parametrize("rotary,interleaved", [(None, True), (0, True), (16, False), (96, True), (128, True), (128, False)])
+@pytest.mark.parametrize("paged", [False, True])
+def test_decode_prepares_in_one_launch(lists, rotary, interleaved, paged):
+    """Packing the block lists, rotating query and key and appending, in the launch in front of the
+    attention, against the separate operators; a full and an over-full sequence take no new key."""
+    b, hk, d, page, pages = 5, 3, 128, 64, 4
+    cap = page * pages
+    g = torch.Generator(device=DEV).manual_seed(7)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV, dtype=torch.bfloat16)
+    q, kn, vn = rand(b, 1, 16 * hk, d), rand(b, 1, hk, d), rand(b, 1, hk, d)
+    lens = torch.tensor([0, 63, 200, cap, cap + 3], dtype=torch.int32, device=DEV)
+    shape = (b * pages, page) if paged else (b, cap)
+    table = torch.randperm(b * pages, generator=g, device=DEV).view(b, pages).to(torch.int32) if paged else None
+    caches = rand(*shape, hk, d), rand(*shape, hk, d)
+    idx = None
+    if lists:
+        idx = torch.randint(-1, pages, (b, hk, 1, lists), generator=g, device=DEV, dtype=torch.int32)
+    kw = {}
+    if rotary is not None:
+        ang = torch.rand(200, rotary // 2, generator=g, device=DEV) * 6.28           # positions past the table use its end
+        kw = dict(rotary_cos=ang.cos().to(torch.bfloat16), rotary_sin=ang.sin().to(torch.bfloat16), rotary_interleaved=interleaved)
+    kc, vc = (c.clone() for c in caches)
+    out, lse = infllm_v2.infllmv2_attn_with_kvcache(q, kc, vc, kn, vn, cache_seqlens=lens, block_table=table, topk_idx=idx,
+                                                    return_softmax_lse=True, **kw)
+    # the parts: rotation in fp32 with one rounding, plain indexing for the append, a packed mask
+    q2, k2 = q[:, 0], kn[:, 0]
+    if rotary:
+        at = lens.clamp(0, 199).long()
+        cs, sn = kw["rotary_cos"][at][:, None], kw["rotary_sin"][at][:, None]
+        q2 = oracle.apply_rotary(q2.cpu(), cs.cpu(), sn.cpu(), interleaved).to(DEV).to(torch.bfloat16)
+        k2 = oracle.apply_rotary(k2.cpu(), cs.cpu(), sn.cpu(), interleaved).to(DEV).to(torch.bfloat16)
+    ke, ve = (c.clone() for c in caches)
+    for i, n in enumerate(lens.tolist()):
+        if n < cap:
+            row = (int(table[i, n // page]), n % page) if paged else (i, n)
+            ke[row], ve[row] = k2[i], vn[i, 0]
+    assert torch.equal(vc, ve)
+    assert (kc.float() - ke.float()).abs().max() <= 2.0 ** -7 * 4                    # (an fp32 product contracted or not: one bf16 step)
+    words = infllm_v2.topk_to_uint64(idx, cap, 64)[0] if lists else None
+    exp, exp_lse = infllm_v2.infllmv2_attn_with_kvcache(q2[:, None], kc, vc, cache_seqlens=(lens + 1).clamp(max=cap),
+                                                        block_table=table, block_mask=words, return_softmax_lse=True)
+    seen = torch.isfinite(exp_lse)
+    assert torch.equal(torch.isfinite(lse), seen)
+    assert (lse[seen] - exp_lse[seen]).abs().max() < 2e-2 if seen.any() else True
+    mx, mr = err_stats(out, exp)
+    assert mx <= MAX_ABS and mr <= MEAN_REL, (mx, mr)
