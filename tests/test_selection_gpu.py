@@ -289,3 +289,21 @@ def test_topk_ties_are_taken_lowest_index_first(n, k):
     only, _ = infllm_v2.infllmv2_topk_mask(y.to(DEV), k, 64 * n, cache_len=64 * (n - 1))
     words = torch.from_numpy(oracle.topk_to_uint64(exp.numpy(), 64 * n, 64)[0])
     assert torch.equal(idx.cpu(), exp) and torch.equal(mask.cpu(), words) and torch.equal(only.cpu(), words)
+
+
+@pytest.mark.parametrize("kl", [255, 256, 257, 1023, 1024, 1025, 1032, 2047, 2049])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_pool_across_the_scores_of_a_batch(kl, dtype):
+    """The vector path takes 256 scores per step and 1024 per batch of loads: windows that reach over
+    those borders, negative scores and -inf, rows of a padded buffer."""
+    pad = (kl + 7) // 8 * 8 + 8
+    g = torch.Generator().manual_seed(kl)
+    buf = (torch.randn(3, 10, pad, generator=g) * 2 - 3).to(dtype)
+    buf[:, ::3, ::7] = float("-inf")
+    for at in (255, 256, 1023, 1024):                        # the largest score sits on either side of a border
+        if at < kl:
+            buf[:, 1::4, at] = 5.0
+    cache = 16 * kl
+    exp = oracle.max_pooling_1d(buf[:, :, :kl].contiguous(), cache, 1, 1)
+    got = infllm_v2.max_pooling_1d(buf.to(DEV)[:, :, :kl], cache, 1, 1)
+    assert torch.equal(got.cpu(), exp)
