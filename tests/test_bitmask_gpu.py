@@ -73,3 +73,16 @@ def test_transpose_blockmask(hk, t, kb):
     b = infllm_v2.uint64_to_bool(torch.from_numpy(fwd).to(DEV), kb).transpose(1, 2).contiguous()
     ref_path, _ = infllm_v2.blockmask_to_uint64(b)
     assert torch.equal(ref_path, got)
+
+
+@pytest.mark.parametrize("k", [1, 4, 7, 64, 130])
+def test_topk_to_uint64_runs_and_duplicates(k):
+    # runs inside one half word, across halves and words, repeated entries and gaps between them
+    n = 300
+    rows = [np.arange(k), np.arange(k) + 30, np.arange(k)[::-1] + 60, np.full(k, 31), np.full(k, -1), np.arange(k) * 32 % n,
+            np.where(np.arange(k) % 3 == 1, -1, 95 + np.arange(k)), np.repeat(np.arange((k + 1) // 2) + 62, 2)[:k],
+            n - 1 - np.arange(k) % 5, np.arange(k) + 64 * ((n + 63) // 64) - 2]                # the last runs past the mask
+    idx = np.stack(rows).astype(np.int32)[None]
+    exp, _ = oracle.topk_to_uint64(np.where(idx < (n + 63) // 64 * 64, idx, -1), 64 * n, 64)
+    got, _ = infllm_v2.topk_to_uint64(torch.from_numpy(idx).to(DEV), 64 * n, 64)
+    assert np.array_equal(got.cpu().numpy(), exp)
