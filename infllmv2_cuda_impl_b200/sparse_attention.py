@@ -140,11 +140,14 @@ class SparseAttention:
             kc, cu_c = self.compress(k.detach(), cu_seqlens, seqlens)
             if c.coarse_lse:
                 kc2, cu_c2 = self.compress(k.detach(), cu_seqlens, seqlens, coarse=True)
-        mask = None
+        idx = mask = None
         if max_seqlen > c.dense_len and max_c > 0:
-            mask = self._select_mask(q.detach(), kc, cu_seqlens, cu_c, max_seqlen, max_c, kc2, cu_c2)
+            if getattr(self.select, "__func__", None) is SparseAttention.select:
+                mask = self._select_mask(q.detach(), kc, cu_seqlens, cu_c, max_seqlen, max_c, kc2, cu_c2)
+            else:                                  # a selection of the caller's own
+                idx = self.select(q.detach(), kc, cu_seqlens, cu_c, max_seqlen, max_c, kc2, cu_c2)
         out = infllmv2_attn_varlen_func(q, k, v, cu_seqlens, cu_seqlens, max_seqlen, max_seqlen,
-                                        softmax_scale=softmax_scale, causal=True, block_mask=mask)
+                                        softmax_scale=softmax_scale, causal=True, topk_idx=idx, block_mask=mask)
         if cache is not None:
             cache.fill(k.detach(), v.detach(), kc, cu_seqlens, cu_c, max_seqlen, kc2, cu_c2)
         return out

@@ -340,3 +340,24 @@ def test_graph_step_takes_inputs_of_any_form(form):
              "offset": lambda t: torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)}[given]
         outs.append([step(*(x(t) for t in step_in)).clone(), cache.k.clone(), cache.v.clone()])
     assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
+def test_prefill_uses_a_selection_of_the_callers_own():
+    # prefill packs its own selection at once; an overridden `select` still decides
+    cfg, n = _config(topk=2, local_blocks=0, init_blocks=0), 500
+    q, k, v = (det_tensor((n, h, D), 110 + i, 0.25, device=DEV) for i, h in enumerate((HQ, HK, HK)))
+    idx = torch.full((HK, n, 2), -1, dtype=torch.int32, device=DEV)
+    idx[..., 0] = 0
+
+    class First(infllm_v2.SparseAttention):
+        def select(self, *args, **kwargs):
+            return idx
+
+    got = First(cfg).prefill(q, k, v, cu([n], DEV), n, seqlens=[n])
+    exp = infllm_v2.infllmv2_attn_varlen_func(q, k, v, cu([n], DEV), cu([n], DEV), n, n, causal=True, topk_idx=idx)
+    own = infllm_v2.SparseAttention(cfg)
+    kc, cu_c = own.compress(k, cu([n], DEV), [n])
+    sel = own.select(q, kc, cu([n], DEV), cu_c, n, cfg.windows(n))
+    assert torch.equal(got, exp)
+    assert torch.equal(own.prefill(q, k, v, cu([n], DEV), n, seqlens=[n]),
+                       infllm_v2.infllmv2_attn_varlen_func(q, k, v, cu([n], DEV), cu([n], DEV), n, n, causal=True, topk_idx=sel))
