@@ -518,8 +518,11 @@ class Infllmv2AttnVarlenFunc(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout, *args):
         q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, fwd_mask = ctx.saved_tensors
-        backward = (_varlen_backward if _plain_eager(dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, fwd_mask)
-                    else _infllmv2_attn_varlen_backward)
+        # With create_graph=True autograd runs this with gradients enabled.  The registered operator then
+        # refuses a second backward, as it has no derivative; the body would return the gradients as
+        # constants, and a term of the loss that depends on them would be lost without a word.
+        direct = not torch.is_grad_enabled() and _plain_eager(dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, fwd_mask)
+        backward = _varlen_backward if direct else _infllmv2_attn_varlen_backward
         dq, dk, dv = backward(
             dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, ctx.max_seqlen_q,
             ctx.max_seqlen_k, ctx.softmax_scale, ctx.causal, fwd_mask)

@@ -114,3 +114,18 @@ def test_bwd_odd_and_even_block_counts(n_sel, len_k):
     # the dQ kernel takes blocks in pairs and keeps up to three pairs of key tiles in flight
     _check([24], [len_k], n_sel, True, shared=True, seed=60 + n_sel)
     _check([13], [len_k], n_sel, False, seed=70 + n_sel)
+
+
+def test_bwd_second_order_is_refused():
+    # a gradient penalty needs a second derivative, which the operator does not have: an error, not a
+    # penalty that is silently constant
+    hq, hk, d, n = 32, 2, 128, 70
+    q, k, v = (det_tensor((n, h, d), 90 + i, 0.25, device=DEV).requires_grad_(True) for i, h in enumerate((hq, hk, hk)))
+    args = (cu([n], DEV), cu([n], DEV), n, n)
+    out = infllm_v2.infllmv2_attn_varlen_func(q, k, v, *args, causal=True)
+    plain = torch.autograd.grad(out.float().sum(), (q, k, v))
+    out = infllm_v2.infllmv2_attn_varlen_func(q, k, v, *args, causal=True)
+    grads = torch.autograd.grad(out.float().sum(), (q, k, v), create_graph=True)
+    assert all(torch.equal(a, b) for a, b in zip(grads, plain))          # the first order is what it always is
+    with pytest.raises(RuntimeError, match="no autograd formula"):
+        (out.float().sum() + grads[0].float().pow(2).sum()).backward()
