@@ -407,12 +407,13 @@ def _bwd(dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_
 
 
 def _plain_eager(*tensors) -> bool:
-    """True when nothing watches the operators that are called: no compilation or trace, no dispatch
-    mode, no function transform, no tensor subclass.  The bodies of the two registered operators below
+    """True when nothing watches the operators that are called: no compilation or trace, no dispatch or
+    function mode, no profiler, no function transform, no tensor subclass.  The bodies of the two registered operators below
     are then called as they are; going through the registration costs 50-70 us of host time per call,
     more than the kernels of a short prefill."""
     return (not torch.compiler.is_compiling() and not torch.jit.is_tracing()
-            and torch._C._len_torch_dispatch_stack() == 0
+            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+            and not torch.autograd._profiler_enabled()
             and torch._C._functorch.peek_interpreter_stack() is None
             and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors if t is not None))
 

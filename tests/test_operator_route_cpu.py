@@ -46,3 +46,20 @@ def test_backward_that_is_differentiated_takes_the_operator(calls):
     q, out = _call()
     torch.autograd.grad(out.sum(), q, create_graph=True)
     assert calls == ["forward body", "backward operator"]
+
+
+def test_function_modes_and_profilers_see_the_operators(calls):
+    from torch.overrides import TorchFunctionMode
+
+    class Pass(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    with Pass():
+        _call()
+    assert calls == ["forward operator"]
+    calls.clear()
+    with torch.autograd.profiler.profile(use_kineto=False, use_device=None):
+        q, out = _call()
+        torch.autograd.grad(out.sum(), q)
+    assert calls == ["forward operator", "backward operator"]

@@ -169,3 +169,22 @@ def test_registered_operators_are_used_when_something_traces(packed):
     assert all(torch.equal(a, b) for a, b in zip(*res))
     assert any("_infllmv2_attn_varlen_forward" in s for s in seen)
     # (the engine runs the backward in a thread of its own, which the mode does not cover)
+
+
+def test_function_mode_sees_the_forward_operator():
+    from torch.overrides import TorchFunctionMode
+    seen = []
+
+    class Recorder(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    hq, hk, d, n = 32, 2, 128, 90
+    q, k, v = (det_tensor((n, h, d), 88 + i, 0.25, device=DEV) for i, h in enumerate((hq, hk, hk)))
+    args = (cu([n], DEV), cu([n], DEV), n, n)
+    plain = infllm_v2.infllmv2_attn_varlen_func(q, k, v, *args, causal=True)
+    with Recorder():
+        out = infllm_v2.infllmv2_attn_varlen_func(q, k, v, *args, causal=True)
+    assert torch.equal(out, plain)
+    assert any("_infllmv2_attn_varlen_forward" in s for s in seen)
