@@ -14,7 +14,7 @@ from typing import Optional, Tuple, Union
 import torch
 
 from . import _lib
-from .ops import _on, _stream, topk_to_uint64, transpose_blockmask
+from .ops import _on, _plain_eager, _stream, topk_to_uint64, transpose_blockmask
 
 BLOCK_N = 64      # tokens per KV block (the reference's N_BLOCK_DIM)
 GROUP = 16        # query heads per KV head (the reference's m_block_dim)
@@ -406,16 +406,11 @@ def _bwd(dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_
     return dq, dk, dv
 
 
-def _plain_eager(*tensors) -> bool:
-    """True when nothing watches the operators that are called: no compilation or trace, no dispatch or
-    function mode, no profiler, no function transform, no tensor subclass.  The bodies of the two registered operators below
-    are then called as they are; going through the registration costs 50-70 us of host time per call,
-    more than the kernels of a short prefill."""
-    return (not torch.compiler.is_compiling() and not torch.jit.is_tracing()
-            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
-            and not torch.autograd._profiler_enabled()
-            and torch._C._functorch.peek_interpreter_stack() is None
-            and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors if t is not None))
+def _direct(*tensors) -> bool:
+    """True when the bodies of the two registered operators below may be called as they are: going through
+    the registration costs 50-70 us of host time per call, more than the kernels of a short prefill.  A
+    profiler's trace holds the operators' names."""
+    return not torch.autograd._profiler_enabled() and _plain_eager(*tensors)
 
 
 def _varlen_forward(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softmax_scale,
@@ -504,7 +499,7 @@ class Infllmv2AttnVarlenFunc(torch.autograd.Function):
                       "infllmv2_attn_varlen_func")
         if softmax_scale is None:
             softmax_scale = q.shape[-1] ** (-0.5)
-        forward = (_varlen_forward if _plain_eager(q, k, v, cu_seqlens_q, cu_seqlens_k, topk_idx, block_mask)
+        forward = (_varlen_forward if _direct(q, k, v, cu_seqlens_q, cu_seqlens_k, topk_idx, block_mask)
                    else _infllmv2_attn_varlen_forward)
         out, lse, fwd_mask = forward(
             q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, softmax_scale, causal,
@@ -522,7 +517,7 @@ class Infllmv2AttnVarlenFunc(torch.autograd.Function):
         # With create_graph=True autograd runs this with gradients enabled.  The registered operator then
         # refuses a second backward, as it has no derivative; the body would return the gradients as
         # constants, and a term of the loss that depends on them would be lost without a word.
-        direct = not torch.is_grad_enabled() and _plain_eager(dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, fwd_mask)
+        direct = not torch.is_grad_enabled() and _direct(dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, fwd_mask)
         backward = _varlen_backward if direct else _infllmv2_attn_varlen_backward
         dq, dk, dv = backward(
             dout, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, ctx.max_seqlen_q,

@@ -26,6 +26,16 @@ def _on(device):
     return _AS_IT_IS if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
+def _plain_eager(*tensors) -> bool:
+    """True when nothing watches the operators that are called: no compilation or trace, no dispatch or
+    function mode, no function transform, no tensor subclass.  Only then may a call that is made of
+    operators go around them."""
+    return (not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0
+            and torch._C._functorch.peek_interpreter_stack() is None
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) for t in tensors if t is not None))
+
+
 def _require_cuda(t: torch.Tensor, name: str):
     if not t.is_cuda:
         raise RuntimeError(f"{name} must be a CUDA tensor (got {t.device}); this library has no CPU path")
@@ -274,8 +284,10 @@ def compressed_lengths(cu_seqlens_k: torch.Tensor, kernel_size: int = 32,
     """Cumulative number of compressed keys per sequence (int32, same device, no host sync):
     a sequence of length L has (L - kernel_size) // kernel_stride + 1 full windows, none when
     L < kernel_size (tests/test_stage1_compressed_lse.py:11-55, calc_chunks_with_stride)."""
-    if (cu_seqlens_k.is_cuda and cu_seqlens_k.dtype == torch.int32 and cu_seqlens_k.dim() == 1
-            and cu_seqlens_k.numel() >= 1 and kernel_size >= 1 and kernel_stride >= 1):
+    # (one launch for a table on the device; the operators below can be traced, compiled and run on fakes)
+    if (_plain_eager(cu_seqlens_k) and cu_seqlens_k.is_cuda and cu_seqlens_k.dtype == torch.int32
+            and cu_seqlens_k.dim() == 1 and cu_seqlens_k.numel() >= 1 and type(kernel_size) is int
+            and type(kernel_stride) is int and 1 <= kernel_size < 2 ** 31 and 1 <= kernel_stride < 2 ** 31):
         cu_seqlens_k = cu_seqlens_k.contiguous()
         cu_c = torch.empty_like(cu_seqlens_k)
         with _on(cu_c.device):

@@ -107,3 +107,21 @@ def test_compressed_lengths(batch, kernel, stride):
         exp.append(exp[-1] + ((l - kernel) // stride + 1 if l >= kernel else 0))
     assert got.cpu().tolist() == exp
     assert infllm_v2.compressed_lengths(cu(lens), kernel, stride).tolist() == exp      # a host table
+
+
+def test_compressed_lengths_can_be_compiled_and_watched():
+    # a device table in one graph without breaks, and under a dispatch mode that sees the operators
+    from torch.utils._python_dispatch import TorchDispatchMode
+    seen = []
+
+    class Recorder(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    table = cu([40, 0, 31, 32, 1000], DEV)
+    exp = infllm_v2.compressed_lengths(table)
+    assert torch.equal(torch.compile(infllm_v2.compressed_lengths, fullgraph=True, backend="eager")(table), exp)
+    with Recorder():
+        got = infllm_v2.compressed_lengths(table)
+    assert torch.equal(got, exp) and any("cumsum" in s for s in seen)

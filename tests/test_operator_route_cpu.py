@@ -63,3 +63,17 @@ def test_function_modes_and_profilers_see_the_operators(calls):
         q, out = _call()
         torch.autograd.grad(out.sum(), q)
     assert calls == ["forward operator", "backward operator"]
+
+
+@pytest.mark.parametrize("sizes", [(32, 16), (128, 64)])
+def test_compressed_lengths_of_a_fake_device_table(sizes):
+    # shape propagation and tracing without a device: the lengths are made of tensor operators then
+    from torch._subclasses import FakeTensorMode
+    from torch.fx.experimental.proxy_tensor import make_fx
+    import infllm_v2
+    with FakeTensorMode():
+        table = torch.empty(6, dtype=torch.int32, device="cuda")
+        got = infllm_v2.compressed_lengths(table, *sizes)
+        assert got.shape == (6,) and got.dtype == torch.int32 and got.device == table.device
+        graph = make_fx(lambda t: infllm_v2.compressed_lengths(t, *sizes))(table)
+    assert any("cumsum" in str(n.target) for n in graph.graph.nodes)
