@@ -142,7 +142,7 @@ class SparseAttention:
                 kc2, cu_c2 = self.compress(k.detach(), cu_seqlens, seqlens, coarse=True)
         idx = mask = None
         if max_seqlen > c.dense_len and max_c > 0:
-            if getattr(self.select, "__func__", None) is SparseAttention.select:
+            if getattr(self.select, "__func__", None) is _OWN_SELECT:
                 mask = self._select_mask(q.detach(), kc, cu_seqlens, cu_c, max_seqlen, max_c, kc2, cu_c2)
             else:                                  # a selection of the caller's own
                 idx = self.select(q.detach(), kc, cu_seqlens, cu_c, max_seqlen, max_c, kc2, cu_c2)
@@ -239,3 +239,8 @@ class SparseAttention:
 
         step.graph, step.inputs = graph, (q_in, k_in, v_in)
         return step
+
+
+# `prefill` packs its own selection at once, but only while `select` is the function above: one that was put
+# in its place, on the class, on a subclass or on an object, decides the blocks.
+_OWN_SELECT = SparseAttention.select

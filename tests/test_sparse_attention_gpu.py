@@ -361,3 +361,19 @@ def test_prefill_uses_a_selection_of_the_callers_own():
     assert torch.equal(got, exp)
     assert torch.equal(own.prefill(q, k, v, cu([n], DEV), n, seqlens=[n]),
                        infllm_v2.infllmv2_attn_varlen_func(q, k, v, cu([n], DEV), cu([n], DEV), n, n, causal=True, topk_idx=sel))
+
+
+@pytest.mark.parametrize("where", ["class", "object"])
+def test_prefill_uses_a_select_that_was_replaced(where, monkeypatch):
+    cfg, n = _config(topk=2, local_blocks=0, init_blocks=0), 500
+    q, k, v = (det_tensor((n, h, D), 120 + i, 0.25, device=DEV) for i, h in enumerate((HQ, HK, HK)))
+    idx = torch.full((HK, n, 2), -1, dtype=torch.int32, device=DEV)
+    idx[..., 0] = 0
+    layer = infllm_v2.SparseAttention(cfg)
+    if where == "class":
+        monkeypatch.setattr(infllm_v2.SparseAttention, "select", lambda self, *args, **kwargs: idx)
+    else:
+        layer.select = lambda *args, **kwargs: idx
+    got = layer.prefill(q, k, v, cu([n], DEV), n, seqlens=[n])
+    exp = infllm_v2.infllmv2_attn_varlen_func(q, k, v, cu([n], DEV), cu([n], DEV), n, n, causal=True, topk_idx=idx)
+    assert torch.equal(got, exp)
