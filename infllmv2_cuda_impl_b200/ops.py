@@ -404,16 +404,20 @@ def cache_fill(src: torch.Tensor, cache: torch.Tensor, cu_seqlens: torch.Tensor,
 
 
 def copy3(pairs) -> None:
-    """dst.copy_(src) for three (dst, src) pairs of equally many elements.  One launch when nothing has
-    to be converted, moved between devices or gathered; `copy_` one by one otherwise."""
+    """dst.copy_(src) for three (dst, src) pairs of equally many elements, as if one after the other.  One
+    launch when nothing has to be converted, moved between devices or gathered and the six buffers lie apart (the
+    one launch copies in no order); `copy_` one by one otherwise."""
     dev = pairs[0][0].device
     if all(s.dtype == d.dtype and s.device == dev and d.device == dev and s.numel() == d.numel() and s.is_contiguous()
            and d.is_contiguous() and not s.requires_grad and type(s) is torch.Tensor and (s.data_ptr() | d.data_ptr()) % 16 == 0
            and s.numel() * s.element_size() % 16 == 0 for d, s in pairs):
         args = [x for d, s in pairs for x in (s.data_ptr(), d.data_ptr(), s.numel() * s.element_size())]
-        with _on(dev):
-            _lib.call("ifv2_copy3", *args, _stream(dev))
-        return
+        s0, d0, n0, s1, d1, n1, s2, d2, n2 = args
+        a, b, c, d, e, f = sorted(((s0, s0 + n0), (d0, d0 + n0), (s1, s1 + n1), (d1, d1 + n1), (s2, s2 + n2), (d2, d2 + n2)))
+        if a[1] <= b[0] and b[1] <= c[0] and c[1] <= d[0] and d[1] <= e[0] and e[1] <= f[0]:
+            with _on(dev):
+                _lib.call("ifv2_copy3", *args, _stream(dev))
+            return
     for d, s in pairs:
         d.copy_(s.reshape(d.shape))
 

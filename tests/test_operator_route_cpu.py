@@ -77,3 +77,38 @@ def test_compressed_lengths_of_a_fake_device_table(sizes):
         assert got.shape == (6,) and got.dtype == torch.int32 and got.device == table.device
         graph = make_fx(lambda t: infllm_v2.compressed_lengths(t, *sizes))(table)
     assert any("cumsum" in str(n.target) for n in graph.graph.nodes)
+
+
+@pytest.mark.parametrize("case", ["apart", "neighbours", "onto itself", "swapped", "handed on", "one buffer", "shifted"])
+def test_three_copies_in_one_launch_only_when_their_order_does_not_matter(case, monkeypatch):
+    """A captured step shows its input buffers, so a caller may pass one of them as another input.  The
+    launch is replaced by copies in the opposite order, which differ from the ordered ones if it matters."""
+    import contextlib
+    import ctypes
+    from infllmv2_cuda_impl_b200 import ops
+    launched = []
+
+    def launch(name, *args):
+        launched.append(name)
+        for i in (6, 3, 0):
+            ctypes.memmove(args[i + 1], args[i], args[i + 2])
+
+    monkeypatch.setattr(ops._lib, "call", launch)
+    monkeypatch.setattr(ops, "_on", lambda device: contextlib.nullcontext())
+    monkeypatch.setattr(ops, "_stream", lambda device: 0)
+    # (destination, source) offsets of the three copies of 16 elements
+    offsets = {"apart": ((0, 64), (16, 96), (32, 128)), "neighbours": ((0, 48), (16, 64), (32, 80)),
+               "onto itself": ((0, 0), (16, 96), (32, 32)), "swapped": ((0, 64), (16, 32), (32, 16)),
+               "handed on": ((0, 64), (16, 0), (32, 16)), "one buffer": ((0, 64), (0, 96), (32, 128)),
+               "shifted": ((0, 8), (32, 96), (64, 128))}[case]
+    pairs = lambda buf: [(buf[d:d + 16], buf[s:s + 16]) for d, s in offsets]
+    got, exp = (torch.arange(256, dtype=torch.int32) for _ in range(2))
+    if case == "shifted":                          # refused by copy_
+        with pytest.raises(RuntimeError):
+            ops.copy3(pairs(got))
+    else:
+        ops.copy3(pairs(got))
+        for d, s in pairs(exp):
+            d.copy_(s)
+        assert torch.equal(got, exp)
+    assert launched == (["ifv2_copy3"] if case in ("apart", "neighbours") else [])

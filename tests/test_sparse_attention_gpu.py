@@ -377,3 +377,24 @@ def test_prefill_uses_a_select_that_was_replaced(where, monkeypatch):
     got = layer.prefill(q, k, v, cu([n], DEV), n, seqlens=[n])
     exp = infllm_v2.infllmv2_attn_varlen_func(q, k, v, cu([n], DEV), cu([n], DEV), n, n, causal=True, topk_idx=idx)
     assert torch.equal(got, exp)
+
+
+def test_graph_step_takes_its_own_input_buffers():
+    # the step shows its input buffers (query, key, value); given as inputs, they are copied in this order
+    cfg, b = _config(), 3
+    q, kn, vn = (det_tensor((b, h, D), 130 + i, 0.25, device=DEV) for i, h in enumerate((HQ, HK, HK)))
+    outs = []
+    for own in (True, False):
+        cache = infllm_v2.DecodeCache(b, 300, HK, cfg, DEV)
+        step = infllm_v2.SparseAttention(cfg).capture_decode(cache)
+        step(q, kn, vn)
+        given = step.inputs if own else (q, kn, vn)
+        for of_key, of_value in ((2, None), (1, 2), (2, 1)):
+            key, value = given[of_key], kn if of_value is None else given[of_value]
+            if not own:                            # what the buffers hold after the step
+                given = (q, key, key if of_value == 1 else value)
+                value = given[2]
+            outs.append(step(given[0], key, value).clone())
+        outs += [cache.k.clone(), cache.v.clone()]
+    n = len(outs) // 2
+    assert all(torch.equal(a, b) for a, b in zip(outs[:n], outs[n:]))
