@@ -450,6 +450,10 @@ int ifv2_decode_prepared(const void* q, void* q_rotated, void* k_cache, void* v_
                          const int32_t* cache_batch_idx, const int32_t* cache_leftpad, float softmax_scale,
                          void* workspace, int64_t workspace_bytes, void* stream);
 
+/* How the decode entries lay a step of this size out on the SMs (host only, no launch): plan[0] = CTAs
+ * that share one (sequence, KV head), plan[1] = resident CTAs per SM of the kernel variant. */
+int ifv2_decode_plan(int batch, int heads_k, int32_t* plan);
+
 /* ---------------------------------------------------------------- self-tests -------------- */
 /* Test infrastructure shipped in the library so that a deployment can check the tensor-core
  * building blocks on its own GPU; not part of the attention path.  No counterpart in the

@@ -3,7 +3,7 @@
 // With a single token the query tile is 16 rows, far too small for a tcgen05 tile, and the work
 // is HBM-bound: every selected 64-key block is read once (K and V, 32 KB) and used by 16 rows.
 // So this kernel is built around bandwidth: the selected blocks of one (sequence, KV head) are
-// split over several CTAs (as many as fill the SMs in ONE wave, two CTAs per SM), each warp
+// split over several CTAs (as many as fill the SMs in ONE wave, see plan_splits), each warp
 // streams its blocks as 32-key units into swizzled shared memory (K and V of the next unit are
 // fetched as soon as the current product has consumed its tile), the 16 x 32 products run on
 // mma.sync m16n8k16 (exactly one M tile), and the per-split (max, sum, O) partials are merged by
@@ -29,12 +29,6 @@ constexpr int kMaxSplits = 16;                          // CTAs per (sequence, K
 constexpr int kWarps = 4;
 constexpr int kWarpSmem = 2 * kUnit * 256;              // one K tile + one V tile per warp
 constexpr int kThreads = kWarps * 32;
-// Resident CTAs per SM the split kernel is compiled for, and slots that the split count below fills.  Two
-// (no spills, fewer and longer CTAs) against three: batch 64 at 32k-131k tokens 121.9 us a step against
-// 124.4, batch 12 with 8 KV heads 72.5 / 74.5, paged batch 16 30.6 / 31.5, batch 1 32.4 / 33.4.
-#ifndef IFV2_DECODE_CTAS_PER_SM
-#define IFV2_DECODE_CTAS_PER_SM 2
-#endif
 constexpr int kPartialFloats = kHeadDim + 4;            // O row, running max (log2 units), sum, pad (16-byte rows)
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
@@ -178,8 +172,9 @@ struct BlockList {
   }
 };
 
-template <bool kTma>
-__global__ void __launch_bounds__(kThreads, IFV2_DECODE_CTAS_PER_SM)
+// kResident: CTAs per SM the kernel is compiled for (2: 236 registers, 3: 168 and a few bytes of spills)
+template <bool kTma, int kResident>
+__global__ void __launch_bounds__(kThreads, kResident)
 decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                     const DecodeParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -507,6 +502,36 @@ __global__ void __launch_bounds__(256) decode_combine_kernel(const DecodeParams 
 
 using namespace ifv2;
 
+// How many CTAs share a (sequence, KV head), and how many CTAs per SM the kernel is compiled for.
+//
+// The CTAs of a launch are to fit the SMs all at once: one that spills into another, mostly empty wave
+// takes longer (a step at batch 64 x 2 KV heads, top-64: 2 splits = 256 CTAs on 296 slots 122 us, 4 splits
+// 136, 8 splits 141; batch 16: 8-10 splits 32 us, 4 splits 39, 16 splits 39).
+//
+// Two CTAs per SM (fewer and longer ones, no spills) are the better choice where both counts need the
+// same number of waves: split + combine with 64 of 192 blocks selected, two against three, 64 pairs 43.0 /
+// 45.1 us, 128 pairs 67.6 / 71.6, 512 pairs 190 / 215.  Three are taken where two
+//  - need a wave more: 304 pairs 127.0 us with three, 155.6 with two, 384 pairs 155.6 / 165.9, 600 pairs 227 / 244;
+//  - leave a pair to one CTA while three give it two, so that nothing evens out long and short sequences:
+//    192 pairs of 900-12288 tokens 55.3 us with three, 67.6 with two (all of one length: 92 with either).
+struct SplitPlan { int splits, resident; };
+static SplitPlan plan_splits(int64_t pairs) {
+  const int64_t slots2 = 2 * (int64_t)kNumSMs, slots3 = 3 * (int64_t)kNumSMs;
+  const bool fewer_waves = ceil_div64(pairs, slots3) < ceil_div64(pairs, slots2);
+  const bool two_for_one = slots2 / pairs == 1 && slots3 / pairs == 2;
+  const int resident = fewer_waves || two_for_one ? 3 : 2;
+  const int64_t splits = (resident == 3 ? slots3 : slots2) / pairs;
+  return {(int)(splits < 1 ? 1 : splits > kMaxSplits ? kMaxSplits : splits), resident};
+}
+
+extern "C" int ifv2_decode_plan(int batch, int heads_k, int32_t* plan) {
+  IFV2_REQUIRE(batch >= 1 && heads_k >= 1 && plan != nullptr, IFV2_ERR_INVALID_ARG, "decode_plan: bad argument");
+  const SplitPlan s = plan_splits((int64_t)batch * heads_k);
+  plan[0] = s.splits;
+  plan[1] = s.resident;
+  return IFV2_OK;
+}
+
 extern "C" int64_t ifv2_decode_workspace_bytes(int batch, int heads_q, int head_dim, int max_blocks) {
   (void)max_blocks;
   if (batch < 0 || heads_q < 0 || head_dim != kHeadDim) return 0;
@@ -702,16 +727,8 @@ static int decode_impl(const void* q, void* k_cache, void* v_cache, const void* 
   p.cache_batch_idx = cache_batch_idx;
   p.leftpad = cache_leftpad;
   p.scale_log2 = softmax_scale * kLog2e;
-  // One wave: as many CTAs per (sequence, KV head) as still fit the SMs all at once.  A launch that
-  // spills into a second, mostly empty wave takes longer (a step at batch 64 x 2 KV heads, top-64: 2
-  // splits = 256 CTAs on 296 slots 122 us, 4 splits 136, 8 splits 141; batch 16: 8-10 splits 32 us, 4
-  // splits 39, 16 splits 39).
-  const int64_t slots = (int64_t)kNumSMs * IFV2_DECODE_CTAS_PER_SM;
-  const int64_t pairs = (int64_t)batch * heads_k;
-  int splits = (int)(slots / pairs);
-  if (splits < 1) splits = 1;
-  if (splits > kMaxSplits) splits = kMaxSplits;
-  p.splits = splits;
+  const SplitPlan plan = plan_splits((int64_t)batch * heads_k);
+  p.splits = plan.splits;
   p.partial = static_cast<float*>(workspace);
   p.out = static_cast<__nv_bfloat16*>(out);
   p.lse = lse;
@@ -738,13 +755,11 @@ static int decode_impl(const void* q, void* k_cache, void* v_cache, const void* 
     memset(&map_k, 0, sizeof(map_k));
     memset(&map_v, 0, sizeof(map_v));
   }
-  cudaError_t e = cudaFuncSetAttribute(tma_ok ? decode_split_kernel<true> : decode_split_kernel<false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  auto kernel = plan.resident == 3 ? (tma_ok ? decode_split_kernel<true, 3> : decode_split_kernel<false, 3>)
+                                   : (tma_ok ? decode_split_kernel<true, 2> : decode_split_kernel<false, 2>);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return set_error((int)e, "decode: %s", cudaGetErrorString(e));
-  if (tma_ok)
-    decode_split_kernel<true><<<dim3(p.splits, heads_k, batch), kThreads, smem, st>>>(map_k, map_v, p);
-  else
-    decode_split_kernel<false><<<dim3(p.splits, heads_k, batch), kThreads, smem, st>>>(map_k, map_v, p);
+  kernel<<<dim3(p.splits, heads_k, batch), kThreads, smem, st>>>(map_k, map_v, p);
   int rc = check_launch("decode_split");
   if (rc) return rc;
   decode_combine_kernel<<<dim3(heads_k, batch), 256, 0, st>>>(p);

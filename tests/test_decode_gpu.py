@@ -293,3 +293,29 @@ def test_decode_prepares_in_one_launch(lists, rotary, interleaved, paged):
     assert (lse[seen] - exp_lse[seen]).abs().max() < 2e-2 if seen.any() else True
     mx, mr = err_stats(out, exp)
     assert mx <= MAX_ABS and mr <= MEAN_REL, (mx, mr)
+
+
+@pytest.mark.parametrize("tma", [True, False])
+@pytest.mark.parametrize("batch,hk", [(1, 2), (37, 4), (149, 1), (37, 6), (223, 1), (37, 8), (297, 1), (111, 4), (445, 1), (593, 1)])
+def test_decode_at_the_borders_of_the_split_plan(batch, hk, tma):
+    """The last pair count of one layout and the first of the next, ragged lengths down to nothing, caches
+    that a tensor map describes and caches (an odd batch stride) that it does not."""
+    cap, d = 200, 128
+    g = torch.Generator(device=DEV).manual_seed(batch)
+    row = cap * hk * d + (0 if tma else 8)
+    # values of at most ~2.5: rounding P and the result to bf16 costs 2 x 2^-9 of that, half of MAX_ABS
+    caches = [torch.randn(batch * row, generator=g, device=DEV, dtype=torch.bfloat16).mul_(scale)
+              .as_strided((batch, cap, hk, d), (row, hk * d, d, 1)) for scale in (1.0, 0.5)]
+    q = torch.randn(batch, 1, 16 * hk, d, generator=g, device=DEV, dtype=torch.bfloat16)
+    lens = torch.randint(0, cap + 1, (batch,), generator=g, device=DEV, dtype=torch.int32)
+    lens[0] = 0 if batch > 1 else cap
+    out, lse = infllm_v2.infllmv2_attn_with_kvcache(q, *caches, cache_seqlens=lens, return_softmax_lse=True)
+    s = torch.einsum("bhgd,bnhd->bhgn", q.view(batch, hk, 16, d).float(), caches[0].float()) * d ** -0.5
+    s = s.masked_fill(torch.arange(cap, device=DEV) >= lens[:, None, None, None], float("-inf"))
+    p = torch.nan_to_num(s.softmax(-1))                      # (a sequence without keys gives zeros)
+    ref = torch.einsum("bhgn,bnhd->bhgd", p, caches[1].float()).reshape(out.shape)
+    mx, mr = err_stats(out, ref)
+    assert mx <= MAX_ABS and mr <= MEAN_REL, (mx, mr)
+    seen = lens > 0
+    assert (lse.view(batch, -1)[seen] - s.logsumexp(-1).reshape(batch, -1)[seen]).abs().max() < 2e-2
+    assert torch.isinf(lse.view(batch, -1)[~seen]).all()
