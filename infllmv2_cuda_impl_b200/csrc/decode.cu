@@ -9,7 +9,7 @@
 // mma.sync m16n8k16 (exactly one M tile), and the per-split (max, sum, O) partials are merged by
 // a small second kernel.
 //
-// Launches: [append new K/V in place] -> split kernel -> combine kernel.
+// Launches: [prepare: block lists, rotation, append in place] -> split kernel -> combine kernel.
 //
 // Tile loads: when the cache rows can be described by one tensor map (16-byte aligned base, batch
 // stride a whole number of rows) a warp's K and V tiles arrive as two TMA boxes each ({64 d, 1 head,
@@ -84,29 +84,6 @@ __device__ __forceinline__ int64_t cache_row_offset(const int32_t* block_table, 
     return ((int64_t)page * page_size + pos % page_size) * row_stride;
   }
   return slot * batch_stride + pos * row_stride;
-}
-
-__global__ void decode_append_kernel(__nv_bfloat16* k_cache, __nv_bfloat16* v_cache,
-                                     const __nv_bfloat16* k_new, const __nv_bfloat16* v_new,
-                                     const int32_t* cache_seqlens, int heads_k, int64_t capacity,
-                                     int64_t batch_stride, const int32_t* block_table, int bt_stride,
-                                     int page_size, const int32_t* cache_batch_idx) {
-  const int b = blockIdx.x;
-  const int64_t pos = cache_seqlens[b];
-  if (pos < 0 || pos >= capacity) return;           // no room: the host documents this as an error
-  const int n = heads_k * kHeadDim / 8;             // 16-byte vectors per token
-  const int64_t row_stride = (int64_t)heads_k * kHeadDim;
-  const int slot = cache_batch_idx ? cache_batch_idx[b] : b;
-  const int64_t off = cache_row_offset(block_table, bt_stride, page_size, batch_stride, row_stride, b,
-                                       slot, pos);
-  const uint4* ks = reinterpret_cast<const uint4*>(k_new + (int64_t)b * heads_k * kHeadDim);
-  const uint4* vs = reinterpret_cast<const uint4*>(v_new + (int64_t)b * heads_k * kHeadDim);
-  uint4* kd = reinterpret_cast<uint4*>(k_cache + off);
-  uint4* vd = reinterpret_cast<uint4*>(v_cache + off);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    kd[i] = ks[i];
-    vd[i] = vs[i];
-  }
 }
 
 // The selected blocks of one (sequence, KV head), lowest first, looked up by a whole warp that takes
@@ -538,55 +515,10 @@ extern "C" int64_t ifv2_decode_workspace_bytes(int batch, int heads_q, int head_
   return (int64_t)batch * heads_q * kMaxSplits * kPartialFloats * 4 + 256;
 }
 
-// Rotary embedding of the decode step's new key and of its query, both at the position the key is
-// appended at (the reference rotates them while it copies them, flash_fwd_kernel.h:787-930 with
-// rotary.h): interleaved pairs (2i, 2i+1) or halves (i, i + rotary_dim/2); features past rotary_dim
-// pass through; fp32 arithmetic, one rounding.  One thread per (row, pair).
-__global__ void decode_rotary_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_new,
-                                     __nv_bfloat16* __restrict__ q_out, __nv_bfloat16* __restrict__ k_out,
-                                     const __nv_bfloat16* __restrict__ cos_t, const __nv_bfloat16* __restrict__ sin_t,
-                                     const int32_t* __restrict__ cache_seqlens, int batch, int heads_q,
-                                     int heads_k, int rotary_dim, int seqlen_ro, int interleaved) {
-  const int rows = heads_q + heads_k;                  // per sequence: query heads, then key heads
-  const int64_t n = (int64_t)batch * rows * (kHeadDim / 2);
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(idx % (kHeadDim / 2));
-    const int r = (int)((idx / (kHeadDim / 2)) % rows);
-    const int b = (int)(idx / ((int64_t)(kHeadDim / 2) * rows));
-    const bool is_q = r < heads_q;
-    const __nv_bfloat16* src = is_q ? q + ((int64_t)b * heads_q + r) * kHeadDim
-                                    : k_new + ((int64_t)b * heads_k + (r - heads_q)) * kHeadDim;
-    __nv_bfloat16* dst = is_q ? q_out + ((int64_t)b * heads_q + r) * kHeadDim
-                              : k_out + ((int64_t)b * heads_k + (r - heads_q)) * kHeadDim;
-    const int half = rotary_dim / 2;
-    // the two features this thread owns
-    int i0, i1;
-    if (i < half) {
-      i0 = interleaved ? 2 * i : i;
-      i1 = interleaved ? 2 * i + 1 : i + half;
-    } else {                                            // pass-through part, two features per thread
-      i0 = rotary_dim + 2 * (i - half);
-      i1 = i0 + 1;
-    }
-    float x0 = __bfloat162float(src[i0]), x1 = __bfloat162float(src[i1]);
-    if (i < half) {
-      const int pos = min(max(cache_seqlens[b], 0), seqlen_ro - 1);
-      const float c = __bfloat162float(cos_t[(int64_t)pos * half + i]);
-      const float sn = __bfloat162float(sin_t[(int64_t)pos * half + i]);
-      const float re = x0 * c - x1 * sn, im = x0 * sn + x1 * c;
-      x0 = re;
-      x1 = im;
-    }
-    dst[i0] = __float2bfloat16_rn(x0);
-    dst[i1] = __float2bfloat16_rn(x1);
-  }
-}
-
 // What a decode step with given block lists does before the attention, in one launch: pack the lists into
-// mask rows, rotate the query and the new key, append the new key and value.  One CTA per (sequence, KV
-// head).  Three launches of 2-6 us (and three calls from the host, which bounds such a step) otherwise;
-// the arithmetic is that of topk_to_uint64_kernel, decode_rotary_kernel and decode_append_kernel.
+// mask rows, rotate the query and the new key, append the new key and value, whichever of them there are.
+// One CTA per (sequence, KV head).  Three launches of 2-6 us (and three calls from the host, which bounds
+// such a step) otherwise.
 struct PrepareParams {
   const __nv_bfloat16* q;          // (batch, heads_q, 128), rotated into q_out; null = no rotation
   __nv_bfloat16* q_out;
@@ -599,6 +531,10 @@ struct PrepareParams {
   int topk, words, rotary_dim, seqlen_ro, interleaved;
 };
 
+// Rotary embedding of the two features that number i of a row's 64 threads owns, at table position pos (the
+// reference rotates the new key and the query while it copies them, flash_fwd_kernel.h:787-930 with
+// rotary.h): interleaved pairs (2i, 2i+1) or halves (i, i + rotary_dim/2); features past rotary_dim pass
+// through; fp32 arithmetic, one rounding.
 __device__ __forceinline__ void rotate_pair(const PrepareParams& r, const __nv_bfloat16* src, __nv_bfloat16* dst, int i,
                                             int64_t pos) {
   const int half = r.rotary_dim / 2;
@@ -657,6 +593,23 @@ __global__ void __launch_bounds__(256) decode_prepare_kernel(const PrepareParams
   }
 }
 
+// The rotation alone, into buffers of the caller's.  One thread per (row, pair of features).
+__global__ void decode_rotary_kernel(const PrepareParams r, __nv_bfloat16* __restrict__ k_out,
+                                     const int32_t* __restrict__ cache_seqlens, int batch, int heads_q, int heads_k) {
+  const int rows = heads_q + heads_k;                  // per sequence: query heads, then key heads
+  const int64_t n = (int64_t)batch * rows * (kHeadDim / 2);
+  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n;
+       idx += (int64_t)gridDim.x * blockDim.x) {
+    const int i = (int)(idx % (kHeadDim / 2));
+    const int row = (int)((idx / (kHeadDim / 2)) % rows);
+    const int b = (int)(idx / ((int64_t)(kHeadDim / 2) * rows));
+    const int64_t pos = min(max(cache_seqlens[b], 0), r.seqlen_ro - 1);
+    const int64_t q_off = ((int64_t)b * heads_q + row) * kHeadDim, k_off = ((int64_t)b * heads_k + (row - heads_q)) * kHeadDim;
+    if (row < heads_q) rotate_pair(r, r.q + q_off, r.q_out + q_off, i, pos);
+    else rotate_pair(r, r.k_new + k_off, k_out + k_off, i, pos);
+  }
+}
+
 static int decode_impl(const void* q, void* k_cache, void* v_cache, const void* k_new,
                        const void* v_new, void* out, float* lse, const int64_t* mask,
                        int mask_words, const int32_t* cache_seqlens, int batch, int heads_q,
@@ -693,6 +646,12 @@ static int decode_impl(const void* q, void* k_cache, void* v_cache, const void* 
                "decode: workspace must be 16-byte aligned");
   IFV2_REQUIRE(batch <= 65535 && heads_k <= 65535, IFV2_ERR_TOO_LARGE, "decode: batch or heads_k > 65535");
   cudaStream_t st = (cudaStream_t)stream;
+  PrepareParams append{};
+  if (prepare == nullptr && k_new != nullptr) {
+    append.k_new = static_cast<const __nv_bfloat16*>(k_new);
+    append.v_new = static_cast<const __nv_bfloat16*>(v_new);
+    prepare = &append;
+  }
   if (prepare != nullptr) {
     decode_prepare_kernel<<<dim3(heads_k, batch), 256, prepare->topk_idx ? (size_t)prepare->words * 8 : 0, st>>>(
         *prepare, static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), cache_seqlens, heads_k,
@@ -700,14 +659,6 @@ static int decode_impl(const void* q, void* k_cache, void* v_cache, const void* 
     int rc = check_launch("decode_prepare");
     if (rc) return rc;
     if (prepare->q != nullptr) q = prepare->q_out;
-  } else if (k_new != nullptr) {
-    decode_append_kernel<<<batch, 128, 0, st>>>(
-        static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache),
-        static_cast<const __nv_bfloat16*>(k_new), static_cast<const __nv_bfloat16*>(v_new),
-        cache_seqlens, heads_k, cache_capacity, cache_batch_stride, block_table, block_table_stride,
-        page_size, cache_batch_idx);
-    int rc = check_launch("decode_append");
-    if (rc) return rc;
   }
   DecodeParams p;
   p.q = static_cast<const __nv_bfloat16*>(q);
@@ -849,10 +800,16 @@ extern "C" int ifv2_decode_rotary(const void* q, const void* k_new, void* q_out,
   const int64_t n = (int64_t)batch * (heads_q + heads_k) * (kHeadDim / 2);
   int64_t blocks = ceil_div64(n, 256);
   if (blocks > (int64_t)kNumSMs * 8) blocks = (int64_t)kNumSMs * 8;
-  decode_rotary_kernel<<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(
-      static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k_new),
-      static_cast<__nv_bfloat16*>(q_out), static_cast<__nv_bfloat16*>(k_out),
-      static_cast<const __nv_bfloat16*>(rotary_cos), static_cast<const __nv_bfloat16*>(rotary_sin),
-      cache_seqlens, batch, heads_q, heads_k, rotary_dim, seqlen_ro, interleaved ? 1 : 0);
+  PrepareParams r{};
+  r.q = static_cast<const __nv_bfloat16*>(q);
+  r.q_out = static_cast<__nv_bfloat16*>(q_out);
+  r.k_new = static_cast<const __nv_bfloat16*>(k_new);
+  r.cos_t = static_cast<const __nv_bfloat16*>(rotary_cos);
+  r.sin_t = static_cast<const __nv_bfloat16*>(rotary_sin);
+  r.rotary_dim = rotary_dim;
+  r.seqlen_ro = seqlen_ro;
+  r.interleaved = interleaved ? 1 : 0;
+  decode_rotary_kernel<<<(int)blocks, 256, 0, (cudaStream_t)stream>>>(r, static_cast<__nv_bfloat16*>(k_out), cache_seqlens,
+                                                                      batch, heads_q, heads_k);
   return check_launch("decode_rotary");
 }

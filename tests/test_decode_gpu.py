@@ -319,3 +319,61 @@ def test_decode_at_the_borders_of_the_split_plan(batch, hk, tma):
     seen = lens > 0
     assert (lse.view(batch, -1)[seen] - s.logsumexp(-1).reshape(batch, -1)[seen]).abs().max() < 2e-2
     assert torch.isinf(lse.view(batch, -1)[~seen]).all()
+
+
+@pytest.mark.parametrize("rotary,interleaved", [(None, True), (0, True), (16, False), (128, True)])
+@pytest.mark.parametrize("form", ["dense", "paged", "batch_idx"])
+def test_decode_separate_c_entries(form, rotary, interleaved):
+    """ifv2_topk_to_uint64, ifv2_decode_rotary and ifv2_decode / ifv2_decode_paged one after the other, as a
+    C caller has them, give what infllmv2_attn_with_kvcache gives in one call, bit for bit; the rotation is
+    the oracle's.  A full and an over-full sequence take no new key."""
+    from infllmv2_cuda_impl_b200 import _lib
+    b, hk, d, page, pages = 5, 3, 128, 64, 4
+    cap, hq = page * pages, 16 * hk
+    g = torch.Generator(device=DEV).manual_seed(11)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV, dtype=torch.bfloat16)
+    q, kn, vn = rand(b, 1, hq, d), rand(b, 1, hk, d), rand(b, 1, hk, d)
+    lens = torch.tensor([0, 63, 200, cap, cap + 3], dtype=torch.int32, device=DEV)
+    paged = form == "paged"
+    caches = [rand(*((b * pages, page) if paged else (b + 2, cap)), hk, d) for _ in range(2)]
+    table = torch.randperm(b * pages, generator=g, device=DEV).view(b, pages).to(torch.int32) if paged else None
+    slots = torch.tensor([6, 0, 3, 2, 5], dtype=torch.int32, device=DEV) if form == "batch_idx" else None
+    pad = torch.tensor([0, 10, 65, 0, 1], dtype=torch.int32, device=DEV) if form == "batch_idx" else None
+    idx = torch.randint(-1, pages, (b, hk, 1, 3), generator=g, device=DEV, dtype=torch.int32)
+    kw = {}
+    if rotary is not None:
+        ang = torch.rand(150, rotary // 2, generator=g, device=DEV) * 6.28           # positions past the table use its end
+        kw = dict(rotary_cos=ang.cos().to(torch.bfloat16), rotary_sin=ang.sin().to(torch.bfloat16), rotary_interleaved=interleaved)
+    ke, ve = (c.clone() for c in caches)
+    exp, exp_lse = infllm_v2.infllmv2_attn_with_kvcache(
+        q, ke, ve, kn, vn, cache_seqlens=lens, block_table=table, cache_batch_idx=slots, cache_leftpad=pad, topk_idx=idx,
+        return_softmax_lse=True, **kw)
+
+    st = torch.cuda.current_stream().cuda_stream
+    words = torch.empty(b, hk, 1, 1, dtype=torch.int64, device=DEV)
+    _lib.call("ifv2_topk_to_uint64", idx.data_ptr(), words.data_ptr(), b * hk, 3, pages, 1, st)
+    q2, k2 = q, kn
+    if rotary is not None:
+        q2, k2 = torch.empty_like(q), torch.empty_like(kn)
+        cos, sin = kw["rotary_cos"], kw["rotary_sin"]
+        _lib.call("ifv2_decode_rotary", q.data_ptr(), kn.data_ptr(), q2.data_ptr(), k2.data_ptr(), cos.data_ptr() or None,
+                  sin.data_ptr() or None, lens.data_ptr(), b, hq, hk, d, rotary, cos.shape[0], int(interleaved), st)
+        at = lens.clamp(0, 149).long()
+        for got, src in ((q2, q), (k2, kn)):
+            ref = oracle.apply_rotary(src[:, 0].cpu(), cos[at][:, None].cpu(), sin[at][:, None].cpu(), interleaved)
+            # (an fp32 product contracted or not: at most one bf16 step of values below 8)
+            assert (got[:, 0].cpu().float() - ref.float()).abs().max() <= 2.0 ** -8 * 8
+            assert torch.equal(got[:, 0, :, rotary:], src[:, 0, :, rotary:])
+    out, lse = torch.empty_like(q), torch.empty(b, hq, dtype=torch.float32, device=DEV)
+    ws = torch.empty(int(_lib.load().ifv2_decode_workspace_bytes(b, hq, d, pages)), dtype=torch.uint8, device=DEV)
+    kc, vc = (c.clone() for c in caches)
+    ptr = lambda t: t.data_ptr() if t is not None else None
+    head = (q2.data_ptr(), kc.data_ptr(), vc.data_ptr(), k2.data_ptr(), vn.data_ptr(), out.data_ptr(), lse.data_ptr(),
+            words.data_ptr(), 1, lens.data_ptr(), b, hq, hk, d, cap, kc.stride(0))
+    tail = (float(d ** -0.5), ws.data_ptr(), ws.numel(), st)
+    if form == "dense":
+        _lib.call("ifv2_decode", *head, *tail)
+    else:
+        _lib.call("ifv2_decode_paged", *head, ptr(table), pages if paged else 0, page if paged else 0, ptr(slots), ptr(pad), *tail)
+    assert torch.equal(kc, ke) and torch.equal(vc, ve)
+    assert torch.equal(out, exp) and torch.equal(lse, exp_lse.view(b, hq))
