@@ -251,7 +251,8 @@ def test_decode_block_lists(n_blk, picks):
 @pytest.mark.parametrize("paged", [False, True])
 def test_decode_prepares_in_one_launch(lists, rotary, interleaved, paged):
     """Packing the block lists, rotating query and key and appending, in the launch in front of the
-    attention, against the separate operators; a full and an over-full sequence take no new key."""
+    attention, against the oracle's rotation, plain indexing and the attention with a packed mask; a full
+    and an over-full sequence take no new key."""
     b, hk, d, page, pages = 5, 3, 128, 64, 4
     cap = page * pages
     g = torch.Generator(device=DEV).manual_seed(7)

@@ -111,7 +111,8 @@ def test_bwd_column_masks_with_long_empty_stretches():
 @pytest.mark.parametrize("n_sel", [1, 2, 3, 7])
 @pytest.mark.parametrize("len_k", [448, 461])
 def test_bwd_odd_and_even_block_counts(n_sel, len_k):
-    # the dQ kernel takes blocks in pairs and keeps up to three pairs of key tiles in flight
+    # fewer and more blocks than the dQ kernel's rings hold (three K tiles, two V tiles), and both turns of
+    # its softmax warps, with a whole and a ragged last block
     _check([24], [len_k], n_sel, True, shared=True, seed=60 + n_sel)
     _check([13], [len_k], n_sel, False, seed=70 + n_sel)
 

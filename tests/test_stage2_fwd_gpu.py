@@ -113,8 +113,8 @@ def test_fwd_multiword_mask_eight_kv_heads():
 @pytest.mark.parametrize("n_sel", [1, 2, 3, 5])
 @pytest.mark.parametrize("len_k", [320, 333, 384])
 def test_fwd_odd_and_even_block_counts(n_sel, len_k):
-    # blocks are walked in pairs: a last single block, a ragged block as the first or second of a
-    # pair, and tokens of one tile that select different blocks of a pair
+    # scores and P have two buffers: a last block in the first and in the second of them, a ragged block in
+    # either, and tokens of one tile that select different blocks
     hq, hk, d, lq = 32, 2, 128, 21
     q = det_tensor((lq, hq, d), 31, 0.25)
     k = det_tensor((len_k, hk, d), 32, 0.25)
@@ -127,7 +127,7 @@ def test_fwd_odd_and_even_block_counts(n_sel, len_k):
 @pytest.mark.parametrize("jump", [1, 2, 3, 4])
 def test_fwd_reference_moves_at_any_block(jump):
     # the scores of block `jump` (counted in walking order, highest block first) exceed all before it
-    # by ~60 (natural log units): the running reference has to move at the first or second block of a pair
+    # by ~60 (natural log units): the running reference has to move, in either buffer of scores and P
     hq, hk, d, n_blk = 32, 2, 128, 6
     q = torch.zeros(9, hq, d, dtype=torch.bfloat16)
     q[..., 0] = 1.0
@@ -168,7 +168,85 @@ def test_registered_operators_are_used_when_something_traces(packed):
                 res.append(call())
     assert all(torch.equal(a, b) for a, b in zip(*res))
     assert any("_infllmv2_attn_varlen_forward" in s for s in seen)
-    # (the engine runs the backward in a thread of its own, which the mode does not cover)
+    # (the engine runs the backward in a thread of its own, which the mode does not cover; the next test
+    # keeps it in this thread)
+
+
+def test_registered_backward_is_used_under_a_dispatch_mode():
+    from torch.utils._python_dispatch import TorchDispatchMode
+    seen = []
+
+    class Recorder(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    hq, hk, d, n = 32, 2, 128, 130
+    q, k, v = (det_tensor((n, h, d), 84 + i, 0.25, device=DEV).requires_grad_(True) for i, h in enumerate((hq, hk, hk)))
+    dout = det_tensor((n, hq, d), 87, 0.5, device=DEV)
+
+    def grads():
+        out = infllm_v2.infllmv2_attn_varlen_func(q, k, v, cu([n], DEV), cu([n], DEV), n, n, causal=True)
+        return torch.autograd.grad(out, (q, k, v), dout)
+
+    plain = grads()
+    with torch.autograd.set_multithreading_enabled(False), Recorder():
+        watched = grads()
+    assert all(torch.equal(a, b) for a, b in zip(plain, watched))
+    assert any("_infllmv2_attn_varlen_backward" in s for s in seen)
+
+
+@pytest.mark.parametrize("rows", ["all", "some"])
+@pytest.mark.parametrize("keys", [1, 64])
+@pytest.mark.parametrize("bits", [7, 9, 13, 15])
+def test_fwd_scores_rise_to_either_side_of_the_limit(bits, keys, rows):
+    """One or all keys of a later block lie `bits` powers of two above every score before it, for all rows
+    or for some rows of a warp only.  A block's exponentials may sum up to 2^14 before the reference moves:
+    all keys at 7 and one key at 13 stay below, all keys at 9 and one key at 15 are above."""
+    hq, hk, d, n_blk, lq = 32, 2, 128, 5, 9
+    q = torch.zeros(lq, hq, d, dtype=torch.bfloat16)
+    q[..., 0] = 1.0
+    if rows == "some":
+        q[1::2, :, 0] = 0.0
+        q[:, 1::3, 0] = 0.0
+    q[..., 1:9] = det_tensor((lq, hq, 8), 61, 0.25)
+    k = det_tensor((n_blk * 64, hk, d), 62, 0.25)
+    k[..., 0] = 0.0
+    first = (n_blk - 3) * 64                                # the third block of the walk (highest first)
+    k[first + 64 - keys:first + 64, :, 0] = bits * np.log(2.0) * d ** 0.5
+    v = det_tensor((n_blk * 64, hk, d), 63)
+    _check(q, k, v, cu([lq]), cu([n_blk * 64]), None, False)
+
+
+@pytest.mark.parametrize("n_blk,picks", [(2049, "edges"), (2200, "edges"), (2200, "many"), (2200, None), (4200, "edges"), (4200, "many")])
+def test_fwd_block_lists_of_several_chunks_of_words(n_blk, picks):
+    """More than 32 mask words, so that the walk goes over two or three chunks of them: every token with
+    blocks of its own on both sides of the borders, more than 32 visited blocks in `many`, all of them
+    without a mask.  Against the fp32 result over the selected keys."""
+    hk, d, lq, n = 1, 128, 11, n_blk * 64 - 7
+    g = torch.Generator(device=DEV).manual_seed(n_blk)
+    q = torch.randn(lq, 16 * hk, d, generator=g, device=DEV, dtype=torch.bfloat16)
+    k, v = (torch.randn(n, hk, d, generator=g, device=DEV, dtype=torch.bfloat16).mul_(0.5) for _ in range(2))
+    sel, kw = torch.ones(hk, lq, n_blk, dtype=torch.bool, device=DEV), {}
+    if picks is not None:
+        sel.zero_()
+        edges = [b for b in (0, 63, 64, 1983, 1984, 2047, 2048, 2111, 2112, 4095, 4096, n_blk - 2, n_blk - 1) if b < n_blk]
+        for t in range(lq):
+            sel[:, t, [edges[(t + i) % len(edges)] for i in range(5)]] = True
+        if picks == "many":
+            sel |= torch.rand(hk, lq, n_blk, generator=g, device=DEV) < 60 / n_blk
+        kw = dict(block_mask=infllm_v2.blockmask_to_uint64(sel)[0])
+    out, lse, _ = infllm_v2.infllmv2_attn_varlen_func(q, k, v, cu([lq], DEV), cu([n], DEV), lq, n, causal=True,
+                                                      return_attn_probs=True, **kw)
+    infllm_v2.check_device_status()
+    pos = torch.arange(n, device=DEV)
+    seen = sel[:, :, pos // 64] & (pos <= torch.arange(n - lq, n, device=DEV)[:, None])            # (hk, lq, n)
+    s = torch.einsum("thgd,nhd->htgn", q.view(lq, hk, 16, d).float(), k.float()) * d ** -0.5
+    s = s.masked_fill(~seen[:, :, None, :], float("-inf"))
+    ref = torch.einsum("htgn,nhd->thgd", s.softmax(-1), v.float()).reshape(lq, 16 * hk, d)
+    mx, mr = err_stats(out, ref)
+    assert mx <= MAX_ABS and mr <= MEAN_REL, (mx, mr)
+    assert (lse.view(hk, lq, 16) - s.logsumexp(-1)).abs().max() < 2e-2
 
 
 def test_function_mode_sees_the_forward_operator():
