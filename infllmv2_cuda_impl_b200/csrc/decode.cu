@@ -481,24 +481,23 @@ using namespace ifv2;
 
 // How many CTAs share a (sequence, KV head), and how many CTAs per SM the kernel is compiled for.
 //
-// The CTAs of a launch are to fit the SMs all at once: one that spills into another, mostly empty wave
-// takes longer (a step at batch 64 x 2 KV heads, top-64: 2 splits = 256 CTAs on 296 slots 122 us, 4 splits
-// 136, 8 splits 141; batch 16: 8-10 splits 32 us, 4 splits 39, 16 splits 39).
+// Splits: as many as fit the SMs all at once at three CTAs per SM; a launch that spills into another,
+// mostly empty wave takes longer.  The split also decides the last bits of a result: P is rounded to bf16
+// against the largest score of each warp, whose own weight is exactly 1, so fewer splits leave fewer exact
+// weights (filling two CTAs per SM instead: 32 pairs 30.7 us instead of 32.8 and 128 pairs 67.6 instead of
+// 69.6-71.6, but the error against 64 bits 2.66e-3 -> 2.68e-3 at 32 pairs, 2.72e-3 -> 2.75e-3 at others).
 //
-// Two CTAs per SM (fewer and longer ones, no spills) are the better choice where both counts need the
-// same number of waves: split + combine with 64 of 192 blocks selected, two against three, 64 pairs 43.0 /
-// 45.1 us, 128 pairs 67.6 / 71.6, 512 pairs 190 / 215.  Three are taken where two
-//  - need a wave more: 304 pairs 127.0 us with three, 155.6 with two, 384 pairs 155.6 / 165.9, 600 pairs 227 / 244;
-//  - leave a pair to one CTA while three give it two, so that nothing evens out long and short sequences:
-//    192 pairs of 900-12288 tokens 55.3 us with three, 67.6 with two (all of one length: 92 with either).
+// Resident: two CTAs per SM run faster (no spills) wherever the same CTAs need no more waves that way: a
+// step of one sequence 32.4 us against 33.4 with three, 256 ragged pairs 77.8 / 79.8, 512 pairs 190 / 215;
+// three where two need a wave more: 304 pairs 127.0 us against 155.6 with two, 384 pairs 152 / 166, 600
+// pairs 223 / 242.
 struct SplitPlan { int splits, resident; };
 static SplitPlan plan_splits(int64_t pairs) {
   const int64_t slots2 = 2 * (int64_t)kNumSMs, slots3 = 3 * (int64_t)kNumSMs;
-  const bool fewer_waves = ceil_div64(pairs, slots3) < ceil_div64(pairs, slots2);
-  const bool two_for_one = slots2 / pairs == 1 && slots3 / pairs == 2;
-  const int resident = fewer_waves || two_for_one ? 3 : 2;
-  const int64_t splits = (resident == 3 ? slots3 : slots2) / pairs;
-  return {(int)(splits < 1 ? 1 : splits > kMaxSplits ? kMaxSplits : splits), resident};
+  int64_t splits = slots3 / pairs;
+  splits = splits < 1 ? 1 : splits > kMaxSplits ? kMaxSplits : splits;
+  const bool two_fit = ceil_div64(pairs * splits, slots2) <= ceil_div64(pairs * splits, slots3);
+  return {(int)splits, two_fit ? 2 : 3};
 }
 
 extern "C" int ifv2_decode_plan(int batch, int heads_k, int32_t* plan) {
