@@ -13,14 +13,16 @@
 // epilogue.  K and V each have a 2-deep ring; S/P is double-buffered in TMEM so Q.K^T of the
 // next block overlaps the softmax of the current one.  TMEM: 2 x 64 (S/P) + 128 (O) = 256
 // columns, shared memory 96 KB, so two CTAs share an SM and fill each other's bubbles.
-// The reference maximum of a row is raised only when a block's exponentials get large (their sum passes
-// 64 x 2^8): P is a floating-point number, so its relative precision does not depend on the reference,
-// and the final 1/l normalisation makes the result exact.  A block costs no row maximum otherwise.
+// The reference maximum of a row is raised only by a score more than 2^8 above it; that score's weight is
+// then 1, exact in bf16, and the final 1/l normalisation makes the result exact.  Whether a block can hold
+// such a score follows from the sum of its exponentials, so most blocks cost no row maximum.  (Moving the
+// reference at a sum of 64 x 2^8 instead was no faster, 0.999x, and left the weight of a dominating key
+// rounded: 4.5e-3 off in a result near 1, against the 2e-3 of rounding the result.)
 // What bounds a softmax warp (timeline of a build with clock stamps, 65536-token training batch, per
 // 64-key block): ~1000 clocks of exponentials, 2 x 64 x 8 for the two warps that share a special-function
 // unit, ~200 of waiting for the scores, ~180 of loop and selection bookkeeping, ~100 of TMEM traffic.
 // The bookkeeping was 350 clocks while every thread walked the union and its own mask row block by block
-// (block_walk.cuh does it 32 blocks at a time); that and the row maximum gone: 2.80 -> 2.50 ms at 32768
+// (block_walk.cuh does it 32 blocks at a time); that and most row maxima gone: 2.80 -> 2.50 ms at 32768
 // tokens, 2.00 -> 1.79 ms for a 4096-token chunk at 131072, 4.10 -> 3.62 ms for the training batch.
 // Measured and not taken: pairs of blocks (S with N = 128 in one buffer; 20 % fewer tensor clocks, but the
 // chain of a CTA gets longer: 10-20 % slower); a row split over two threads (8 softmax warps, half the
@@ -42,7 +44,7 @@ constexpr uint32_t kQHalfBytes = 128 * 128;   // 128 rows x 64 bf16
 constexpr uint32_t kKVHalfBytes = 64 * 128;   // 64 keys x 64 bf16
 constexpr uint32_t kTmemCols = 256;
 constexpr float kRescaleThreshold = 8.0f;     // log2 units
-constexpr float kSumLimit = 16384.0f;         // 64 scores, each the threshold above the reference
+constexpr float kSumCheck = 128.0f;           // 2^(threshold - 1): a score beyond the threshold exceeds this by itself
 
 struct FwdParams {
   __nv_bfloat16* out;
@@ -319,15 +321,20 @@ sparse_attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q,
           mx4[(c >> 1) & 3] = fmaxf(mx4[(c >> 1) & 3], fmaxf(__uint_as_float(raw[c]), __uint_as_float(raw[c + 1])));
         return (lim > 0) ? fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) : -INFINITY;
       };
-      // The reference maximum has to move only when a score exceeds it by so much that the numbers
-      // get large, which after a row's first block almost never happens: P keeps its relative
-      // precision at any reference.  So once every row of the warp that takes part has a reference,
-      // the exponentials are taken against it and no row maximum is computed at all; a block whose
-      // sum reaches the bound (or is not a number) is redone below with the maximum.
+      // The reference maximum moves when a score exceeds it by more than the threshold, which after a
+      // row's first block almost never happens.  So once every row of the warp that takes part has a
+      // reference, the exponentials are taken against it, and their sum tells whether there can be such a
+      // score at all: below kSumCheck there is none.  Otherwise (or if the sum is not a number) the row
+      // maximum decides; a block that does move some row's reference is redone below.
       bool done = false;
       if (!no_ref || !__any_sync(0xFFFFFFFFu, lim > 0 && m_ref == -INFINITY)) {
         compute_p((lim == 0) ? -INFINITY : -m_ref * p.scale_log2);
-        done = __all_sync(0xFFFFFFFFu, sum < kSumLimit);
+        done = __all_sync(0xFFFFFFFFu, sum < kSumCheck);
+        if (!done) {
+          const float mx = row_max();
+          const bool moves = mx > m_ref && (mx - m_ref) * p.scale_log2 > kRescaleThreshold;
+          done = !__any_sync(0xFFFFFFFFu, moves);
+        }
       }
       if (!done) {
         const float mx = row_max();

@@ -201,8 +201,8 @@ def test_registered_backward_is_used_under_a_dispatch_mode():
 @pytest.mark.parametrize("bits", [7, 9, 13, 15])
 def test_fwd_scores_rise_to_either_side_of_the_limit(bits, keys, rows):
     """One or all keys of a later block lie `bits` powers of two above every score before it, for all rows
-    or for some rows of a warp only.  A block's exponentials may sum up to 2^14 before the reference moves:
-    all keys at 7 and one key at 13 stay below, all keys at 9 and one key at 15 are above."""
+    or for some rows of a warp only: the reference moves beyond 8, and the row maximum that decides it is
+    taken when the exponentials of a block sum up to 2^7, which one key at 7 just does with the others."""
     hq, hk, d, n_blk, lq = 32, 2, 128, 5, 9
     q = torch.zeros(lq, hq, d, dtype=torch.bfloat16)
     q[..., 0] = 1.0
@@ -216,6 +216,24 @@ def test_fwd_scores_rise_to_either_side_of_the_limit(bits, keys, rows):
     k[first + 64 - keys:first + 64, :, 0] = bits * np.log(2.0) * d ** 0.5
     v = det_tensor((n_blk * 64, hk, d), 63)
     _check(q, k, v, cu([lq]), cu([n_blk * 64]), None, False)
+
+
+def test_fwd_weight_of_a_score_far_above_the_rest_is_exact():
+    """A score more than 8 powers of two above everything before it becomes the reference of its row, so that
+    its weight is 1 and takes no rounding to bf16.  Only that key has a value here: what is left is the
+    rounding of the result, 2^-9 in [0.5, 1), and fp32 arithmetic; a rounded weight would add up to 2^-9."""
+    hq, hk, d, n_blk, lq = 32, 2, 128, 5, 21
+    q = torch.zeros(lq, hq, d)
+    q[..., 0] = torch.linspace(0.7, 1.0, lq * hq).view(lq, hq)
+    k, v = torch.zeros(n_blk * 64, hk, d), torch.zeros(n_blk * 64, hk, d)
+    key = (n_blk - 3) * 64 + 17                             # in the third block of the walk (highest first)
+    k[key, :, 0] = 13.5 * np.log(2.0) * d ** 0.5            # 9.4 .. 13.5 powers of two for the rows above
+    v[key] = 1.0
+    q, k, v = (t.to(torch.bfloat16) for t in (q, k, v))
+    out, _ = _run(q, k, v, cu([lq]), cu([n_blk * 64]), None, False)
+    w = (q[..., 0].double() * k[key, 0, 0].double() * d ** -0.5).exp()
+    ref = (w / (w + n_blk * 64 - 1))[..., None].expand(-1, -1, d)
+    assert ref.min() > 0.5 and (out.double() - ref).abs().max() <= 2.0 ** -9 + 1e-5
 
 
 @pytest.mark.parametrize("n_blk,picks", [(2049, "edges"), (2200, "edges"), (2200, "many"), (2200, None), (4200, "edges"), (4200, "many")])
