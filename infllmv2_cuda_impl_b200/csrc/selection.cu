@@ -46,28 +46,81 @@ __device__ __forceinline__ int block_of(int64_t x, int d) {
   return (x == (int64_t)(int)x) ? (int)x / d : (int)(x / d);
 }
 
-template <bool kVarlen>
+// kNarrow: the division through block_of (where a row holds enough work to hide its branch)
+template <bool kVarlen, bool kNarrow = false>
 __device__ __forceinline__ void row_geometry(const PoolParams& p, int64_t q, int& k_len, int& bq) {
+  int64_t pos = q + p.cache_len;
   if constexpr (kVarlen) {
     const int b = find_sequence(p.cu_q, p.batch, (int)q);
     k_len = min(p.cu_k[b + 1] - p.cu_k[b], p.k_len);
-    bq = block_of(q - p.cu_q[b] + p.cache_lens[b], p.block_size);
+    pos = q - p.cu_q[b] + p.cache_lens[b];
   } else {
     k_len = p.k_len;
-    bq = block_of(q + p.cache_len, p.block_size);
   }
+  bq = kNarrow ? block_of(pos, p.block_size) : (int)(pos / p.block_size);
 }
 
 // Fast path: kernel 5 / stride 4 / padding 1 (block 64 over compression stride 16) and 16-byte
 // aligned rows.  A lane loads 8 consecutive scores and produces the two block scores whose
-// windows they cover: block 2m <- x[8m-1 .. 8m+3], block 2m+1 <- x[8m+3 .. 8m+7].  A warp fetches
-// kPoolBatch x 256 scores of its row before it uses the first (the kernel is bound by HBM, and one load
-// at a time per warp does not keep it busy); the score before a lane's eight comes from its neighbour or
-// from the end of the 256 before.  65536 rows of 2047 scores: 80.0 -> 63.6 us (5.3 TB/s); 63260 rows of
-// 1023: 43.1 -> 37.0 us.
-constexpr int kPoolBatch = 4;
+// windows they cover: block 2m <- x[8m-1 .. 8m+3], block 2m+1 <- x[8m+3 .. 8m+7].
+// One load at a time per warp, 28-30 registers: rows of up to 768 scores, or with few of them to a block
+// score, are bound by latency and issue, and more of them in flight count (8 heads x 4096 rows of 255 scores
+// to 64 blocks: 8.6 us, 14.8 with the kernel below).
 template <typename T, bool kVarlen>
 __global__ void __launch_bounds__(kThreads) max_pool_k5s4_kernel(const PoolParams p) {
+  using N = Num<T>;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t rows = (int64_t)p.heads * p.total_q;
+  const T* in = static_cast<const T*>(p.in);
+  T* out = static_cast<T*>(p.out);
+  const float ninf = -INFINITY;
+  for (int64_t row = (int64_t)blockIdx.x * kWarps + warp; row < rows;
+       row += (int64_t)gridDim.x * kWarps) {
+    int k_len, bq;
+    row_geometry<kVarlen>(p, row % p.total_q, k_len, bq);
+    const T* x = in + row * p.in_row_stride;
+    T* y = out + row * p.out_len;
+    for (int m0 = 0; 2 * m0 < p.out_len; m0 += 32) {     // warp-uniform trip count (shuffles inside)
+      const int m = m0 + lane, e0 = 8 * m;
+      float v[8];
+      if (e0 < k_len) {
+        const uint4 raw = __ldg(reinterpret_cast<const uint4*>(x + e0));
+        const T* t = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = (e0 + j < k_len) ? N::to_f(t[j]) : ninf;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = ninf;
+      }
+      float prev = __shfl_up_sync(0xFFFFFFFFu, v[7], 1);
+      // (lane 0 re-reads its neighbour's last score; it is in L1)
+      if (lane == 0) prev = (e0 >= 1 && e0 - 1 < k_len) ? N::to_f(ldg16(x + e0 - 1)) : ninf;
+      float r0 = fmaxf(fmaxf(prev, v[0]), fmaxf(fmaxf(v[1], v[2]), v[3]));
+      float r1 = fmaxf(fmaxf(v[3], v[4]), fmaxf(fmaxf(v[5], v[6]), v[7]));
+      const int b0 = 2 * m, b1 = b0 + 1;
+      if (b0 >= p.out_len) continue;
+      if (b0 < p.init_blocks || (bq >= b0 && bq <= b0 + p.local_blocks)) r0 = INFINITY;
+      if (b1 < p.init_blocks || (bq >= b1 && bq <= b1 + p.local_blocks)) r1 = INFINITY;
+      if ((p.out_len & 1) == 0) {
+        typename N::T2 pr;
+        pr.x = N::from_f(r0);
+        pr.y = N::from_f(r1);
+        *reinterpret_cast<typename N::T2*>(y + b0) = pr;
+      } else {
+        y[b0] = N::from_f(r0);
+        if (b1 < p.out_len) y[b1] = N::from_f(r1);
+      }
+    }
+  }
+}
+
+// Long rows, bound by HBM, which one load at a time per warp does not keep busy: a warp fetches kPoolBatch x
+// 256 scores of its row before it uses the first; the score before a lane's eight comes from its neighbour or
+// from the end of the 256 before.  44-64 registers.  65536 rows of 2047 scores to 512 blocks: 73.8 -> 61.5 us
+// against the kernel above (5.5 TB/s), 63260 ragged rows of at most 1023: 41.9 -> 36.3 us.
+constexpr int kPoolBatch = 4;
+template <typename T, bool kVarlen>
+__global__ void __launch_bounds__(kThreads) max_pool_k5s4_long_kernel(const PoolParams p) {
   using N = Num<T>;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const T* in = static_cast<const T*>(p.in);
@@ -79,7 +132,7 @@ __global__ void __launch_bounds__(kThreads) max_pool_k5s4_kernel(const PoolParam
   for (int64_t q = (int64_t)blockIdx.x * kWarps + warp; q < p.total_q; q += (int64_t)gridDim.x * kWarps) {
     const int64_t row = head_row + q;
     int k_len, bq;
-    row_geometry<kVarlen>(p, q, k_len, bq);
+    row_geometry<kVarlen, true>(p, q, k_len, bq);
     const T* x = in + row * p.in_row_stride;
     T* y = out + row * p.out_len;
     float before = ninf;                                 // the score in front of the next 256
@@ -93,6 +146,7 @@ __global__ void __launch_bounds__(kThreads) max_pool_k5s4_kernel(const PoolParam
       }
 #pragma unroll
       for (int u = 0; u < kPoolBatch; ++u) {
+        if (2 * (m0 + 32 * u) >= p.out_len) break;       // (the last batch of a row is seldom full)
         const int m = m0 + 32 * u + lane, e0 = 8 * m;
         const T* t = reinterpret_cast<const T*>(&raw[u]);
         float v[8];
@@ -160,12 +214,17 @@ int launch_pool(const PoolParams& p, cudaStream_t st) {
   const bool fast = p.kernel == 5 && p.stride == 4 && p.padding == 1 &&
                     (p.in_row_stride % 8 == 0) && (reinterpret_cast<uintptr_t>(p.in) % 16 == 0) &&
                     (reinterpret_cast<uintptr_t>(p.out) % 4 == 0);
-  if (fast) {
+  // The long kernel where its four loads have a whole row of scores to fetch (more than three times 256) and
+  // the block scores ask for them; rows with far more blocks than scores only pay for its empty steps (1023
+  // scores to 812 blocks: 84.5 us above, 89.8 below).  It was nowhere slower than the other within this line.
+  if (fast && p.k_len > 768 && p.out_len > 192 && 2 * (int64_t)p.k_len >= 3 * (int64_t)p.out_len) {
     const int64_t gy = p.heads < 65535 ? p.heads : 65535;
     int64_t gx = ceil_div64(p.total_q, kWarps);
     const int64_t most = ceil_div64(cap, gy);
     if (gx > most) gx = most;
-    max_pool_k5s4_kernel<T, kVarlen><<<dim3((unsigned)gx, (unsigned)gy), kThreads, 0, st>>>(p);
+    max_pool_k5s4_long_kernel<T, kVarlen><<<dim3((unsigned)gx, (unsigned)gy), kThreads, 0, st>>>(p);
+  } else if (fast) {
+    max_pool_k5s4_kernel<T, kVarlen><<<(int)blocks, kThreads, 0, st>>>(p);
   } else
     max_pool_generic_kernel<T, kVarlen><<<(int)blocks, kThreads, 0, st>>>(p);
   return check_launch("max_pooling_1d");

@@ -307,3 +307,25 @@ def test_pool_across_the_scores_of_a_batch(kl, dtype):
     exp = oracle.max_pooling_1d(buf[:, :, :kl].contiguous(), cache, 1, 1)
     got = infllm_v2.max_pooling_1d(buf.to(DEV)[:, :, :kl], cache, 1, 1)
     assert torch.equal(got.cpu(), exp)
+
+
+@pytest.mark.parametrize("kl,out_len", [(768, 256), (769, 192), (769, 193), (769, 512), (769, 513), (1032, 257), (1040, 260), (2049, 193)])
+def test_pool_at_the_line_between_the_two_vector_kernels(kl, out_len):
+    """Rows just short and just long enough for the kernel that fetches 1024 scores at a time, with more and
+    with fewer blocks than the scores fill, one sequence and ragged ones (down to no score at all)."""
+    g = torch.Generator().manual_seed(kl + out_len)
+    t, pad = 13, (kl + 7) // 8 * 8
+    buf = (torch.randn(3, t, pad, generator=g) * 2 - 3).to(torch.bfloat16)
+    buf[:, ::4, ::5] = float("-inf")
+    cache = 64 * out_len - t
+    exp = oracle.max_pooling_1d(buf[:, :, :kl].contiguous(), cache, 2, 1)
+    got = infllm_v2.max_pooling_1d(buf.to(DEV)[:, :, :kl], cache, 2, 1)
+    assert got.shape[-1] == out_len and torch.equal(got.cpu(), exp)
+
+    lens_q, lens_k = [5, 1, 7], [kl, 0, kl // 3]
+    cuq, cuk = (torch.tensor([0] + l, dtype=torch.int32).cumsum(0).to(torch.int32) for l in (lens_q, lens_k))
+    cl = torch.tensor([64 * out_len - 7, 100, 31], dtype=torch.int32)
+    got = infllm_v2.max_pooling_1d_varlen(buf.to(DEV)[:, :, :kl], cuq.to(DEV), cuk.to(DEV), cl.to(DEV), 7, kl, 2, 1,
+                                          max_cache_len=64 * out_len - 7)
+    exp = oracle.max_pooling_1d_varlen(buf[:, :, :kl], cuq, cuk, cl, 7, kl, 2, 1)
+    assert got.shape[-1] == out_len and torch.equal(got.cpu(), exp)
