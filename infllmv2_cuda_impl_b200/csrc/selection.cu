@@ -577,8 +577,11 @@ void launch_topk_iters(const TopkParams& p, cudaStream_t st) {
   // One wave: every warp strides over the rows, so a second, partly filled wave would leave SMs idle
   // (2048 blocks: 2.28 -> 2.22 ms of 1 M rows; 512 blocks, with 5 instead of 3 CTAs per SM: 0.101 ->
   // 0.094 ms of 65536).  Rows of at most 256 blocks are so short that a row per warp and more CTAs than
-  // fit are better (64 blocks, 8192 rows: 12.4 us against 14.4).
-  int64_t cap = (int64_t)kNumSMs * (kIters == 1 ? 8 : kTopkResident<kIters>) / gy;
+  // fit are better (64 blocks, 8192 rows: 12.4 us against 14.4).  Above 4096 blocks one CTA of eight warps
+  // fills an SM, rows that have to be redone over their full width take twice as long as others, and CTAs
+  // that are handed out as SMs become free even that out: 32768 rows of 6000 blocks, all redone, 935 us
+  // against 1524 with one wave, none redone 653 against 880.
+  int64_t cap = (int64_t)kNumSMs * (kIters == 1 || kIters == 32 ? 8 : kTopkResident<kIters>) / gy;
   if (cap < 1) cap = 1;
   int64_t gx = ceil_div64(p.total_q, kWarps);
   if (gx > cap) gx = cap;
