@@ -93,6 +93,25 @@ __global__ void __launch_bounds__(kThreads) cache_fill_kernel(const FillParams p
       g.seqlens_out[b] = (int32_t)min((int64_t)(g.cu[b + 1] - g.cu[b]), g.cap);
 }
 
+// One tensor of up to kSmallFill vectors, a vector per thread: with so few CTAs the bisections of a thread's
+// four vectors, one after the other, are what the kernel above waits for (64 sequences of 40 tokens x 2 heads
+// 2.7 us, 4.0 above; 1000 of 7 3.5 / 5.7; 300 of 200 tokens, 1.9 M vectors, 14.5 / 13.9).
+constexpr int64_t kSmallFill = 3 << 19;
+__global__ void __launch_bounds__(kThreads) cache_fill_small_kernel(const FillSegment g, int batch, int heads) {
+  const int64_t row_vecs = (int64_t)heads * kVecPerRow;
+  const int64_t n_vec = g.total * row_vecs;
+  for (int64_t idx = (int64_t)blockIdx.x * kThreads + threadIdx.x; idx < n_vec;
+       idx += (int64_t)gridDim.x * kThreads) {
+    const int64_t t = idx / row_vecs, r = idx % row_vecs;
+    const int b = find_sequence(g.cu, batch, (int)t);
+    const int64_t pos = t - g.cu[b];
+    if (pos < g.cap) g.cache[((int64_t)b * g.cap + pos) * row_vecs + r] = __ldg(g.src + idx);
+  }
+  if (g.seqlens_out != nullptr)
+    for (int64_t b = (int64_t)blockIdx.x * kThreads + threadIdx.x; b < batch; b += (int64_t)gridDim.x * kThreads)
+      g.seqlens_out[b] = (int32_t)min((int64_t)(g.cu[b + 1] - g.cu[b]), g.cap);
+}
+
 struct Copy3Params {
   const uint4* src[3];
   uint4* dst[3];
@@ -211,7 +230,7 @@ __global__ void __launch_bounds__(kThreads) decode_append_kernel(const AppendPar
 using namespace ifv2;
 
 static int fill_segment(FillSegment& g, const void* src, void* cache, const int32_t* cu_seqlens, int32_t* seqlens_out,
-                        int64_t total, int64_t capacity, int heads_k) {
+                        int batch, int64_t total, int64_t capacity, int heads_k) {
   IFV2_REQUIRE(total >= 0 && capacity >= 1, IFV2_ERR_INVALID_ARG, "cache_fill: bad size");
   IFV2_REQUIRE(cu_seqlens != nullptr && cache != nullptr && (src != nullptr || total == 0),
                IFV2_ERR_INVALID_ARG, "cache_fill: null pointer");
@@ -220,7 +239,8 @@ static int fill_segment(FillSegment& g, const void* src, void* cache, const int3
   IFV2_REQUIRE(total <= INT32_MAX, IFV2_ERR_TOO_LARGE, "cache_fill: more than 2^31-1 rows");
   g = FillSegment{static_cast<const uint4*>(src), static_cast<uint4*>(cache), cu_seqlens, seqlens_out, total, capacity, 0};
   g.blocks = ceil_div64(total * heads_k * kVecPerRow, kFillPerThread * kThreads);
-  if (g.blocks < 1) g.blocks = 1;              // (the lengths are written in any case)
+  const int64_t for_lengths = ceil_div64(batch, kThreads);      // (the lengths are written in any case)
+  if (g.blocks < for_lengths) g.blocks = for_lengths;
   return IFV2_OK;
 }
 
@@ -241,8 +261,14 @@ extern "C" int ifv2_cache_fill(const void* src, void* cache, const int32_t* cu_s
   FillParams p{};
   p.batch = batch;
   p.heads = heads_k;
-  int rc = fill_segment(p.seg[0], src, cache, cu_seqlens, seqlens_out, total, capacity, heads_k);
-  return rc ? rc : launch_fill(p, stream);
+  int rc = fill_segment(p.seg[0], src, cache, cu_seqlens, seqlens_out, batch, total, capacity, heads_k);
+  if (rc) return rc;
+  const int64_t n_vec = total * heads_k * kVecPerRow;
+  if (n_vec >= kSmallFill) return launch_fill(p, stream);
+  int64_t blocks = ceil_div64(n_vec > batch ? n_vec : batch, kThreads);
+  if (blocks > (int64_t)kNumSMs * 16) blocks = (int64_t)kNumSMs * 16;
+  cache_fill_small_kernel<<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(p.seg[0], batch, heads_k);
+  return check_launch("cache_fill");
 }
 
 extern "C" int ifv2_cache_fill_kv(const void* k, const void* v, const void* kc, void* k_cache, void* v_cache,
@@ -256,11 +282,11 @@ extern "C" int ifv2_cache_fill_kv(const void* k, const void* v, const void* kc, 
   FillParams p{};
   p.batch = batch;
   p.heads = heads_k;
-  int rc = fill_segment(p.seg[0], k, k_cache, cu_seqlens, seqlens_out, total, capacity, heads_k);
+  int rc = fill_segment(p.seg[0], k, k_cache, cu_seqlens, seqlens_out, batch, total, capacity, heads_k);
   if (rc) return rc;
-  rc = fill_segment(p.seg[1], v, v_cache, cu_seqlens, nullptr, total, capacity, heads_k);
+  rc = fill_segment(p.seg[1], v, v_cache, cu_seqlens, nullptr, batch, total, capacity, heads_k);
   if (rc) return rc;
-  rc = fill_segment(p.seg[2], kc, kc_cache, cu_seqlens_c, n_comp_out, total_c, c_capacity, heads_k);
+  rc = fill_segment(p.seg[2], kc, kc_cache, cu_seqlens_c, n_comp_out, batch, total_c, c_capacity, heads_k);
   return rc ? rc : launch_fill(p, stream);
 }
 

@@ -398,3 +398,31 @@ def test_graph_step_takes_its_own_input_buffers():
         outs += [cache.k.clone(), cache.v.clone()]
     n = len(outs) // 2
     assert all(torch.equal(a, b) for a, b in zip(outs[:n], outs[n:]))
+
+
+@pytest.mark.parametrize("rows", [12287, 12288])
+@pytest.mark.parametrize("batch", [1, 700])
+def test_cache_fill_on_either_side_of_the_small_kernel(rows, batch):
+    # 8 heads x 16 vectors: 12288 rows are the first that take the kernel with four vectors per thread; 700
+    # sequences need more than one CTA for their lengths, and every third of them is empty
+    hk, cap = 8, 40 if batch > 1 else rows
+    g = torch.Generator().manual_seed(batch)
+    lens = torch.randint(1, 80, (batch,), generator=g)
+    lens[::3] = 0
+    lens[-1] = 0
+    lens = lens.tolist()
+    used = sum(lens[:-1])
+    lens[-1] = max(rows - used, 0)
+    src = det_tensor((rows, hk, D), 140, device=DEV)
+    cache = torch.zeros(batch, cap, hk, D, dtype=torch.bfloat16, device=DEV)
+    out = torch.full((batch,), -1, dtype=torch.int32, device=DEV)
+    c = [0]
+    for n in lens:
+        c.append(min(c[-1] + n, rows))
+    infllm_v2.cache_fill(src, cache, torch.tensor(c, dtype=torch.int32, device=DEV), out)
+    exp = torch.zeros_like(cache)
+    for b in range(batch):
+        m = min(c[b + 1] - c[b], cap)
+        exp[b, :m] = src[c[b]:c[b] + m]
+    assert torch.equal(cache, exp)
+    assert out.tolist() == [min(c[b + 1] - c[b], cap) for b in range(batch)]
