@@ -109,6 +109,15 @@ def test_compressed_lengths(batch, kernel, stride):
     assert infllm_v2.compressed_lengths(cu(lens), kernel, stride).tolist() == exp      # a host table
 
 
+@pytest.mark.parametrize("batch", [8191, 8192, 8193, 20000])
+def test_compressed_lengths_of_many_sequences(batch):
+    # the kernel's last sizes and the first that the tensor operators take
+    lens = torch.randint(0, 100, (batch,), generator=torch.Generator().manual_seed(batch))
+    got = infllm_v2.compressed_lengths(cu(lens.tolist(), DEV))
+    n = torch.where(lens >= 32, (lens - 32) // 16 + 1, torch.zeros_like(lens))
+    assert got.dtype == torch.int32 and got[0] == 0 and torch.equal(got[1:].cpu(), n.cumsum(0).to(torch.int32))
+
+
 def test_compressed_lengths_can_be_compiled_and_watched():
     # a device table in one graph without breaks, and under a dispatch mode that sees the operators
     from torch.utils._python_dispatch import TorchDispatchMode
