@@ -425,6 +425,11 @@ decode_split_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_cons
 }
 
 // one CTA per (sequence, KV head): merge the per-split partials, normalise, write bf16 + lse
+// Bound by latency: the loads of kBatch splits are issued together (one by one they were a trip to memory per
+// split, most of this kernel's time with 13-16 splits).  A batch of eight costs 109 registers, two CTAs per SM;
+// the large steps, which have one or two splits, want many small CTAs (1024 pairs of 512 tokens, split +
+// combine: 60.1 us with a batch of eight, 57.6 with two).
+template <int kBatch>
 __global__ void __launch_bounds__(256) decode_combine_kernel(const DecodeParams p) {
   const int h = blockIdx.x, b = blockIdx.y;
   const int row = threadIdx.x >> 4, c0 = (threadIdx.x & 15) * 8;
@@ -436,9 +441,6 @@ __global__ void __launch_bounds__(256) decode_combine_kernel(const DecodeParams 
     mmax = fmaxf(mmax, ms[s]);
   }
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, lsum = 0.f;
-  // bound by latency: the loads of kBatch splits are issued together (one by one they were a trip to
-  // memory per split, most of this kernel's time with 13-16 splits)
-  constexpr int kBatch = 8;
 #pragma unroll
   for (int s0 = 0; s0 < kMaxSplits; s0 += kBatch) {
     if (s0 >= p.splits) break;
@@ -712,7 +714,10 @@ static int decode_impl(const void* q, void* k_cache, void* v_cache, const void* 
   kernel<<<dim3(p.splits, heads_k, batch), kThreads, smem, st>>>(map_k, map_v, p);
   int rc = check_launch("decode_split");
   if (rc) return rc;
-  decode_combine_kernel<<<dim3(heads_k, batch), 256, 0, st>>>(p);
+  if (p.splits <= 2)
+    decode_combine_kernel<2><<<dim3(heads_k, batch), 256, 0, st>>>(p);
+  else
+    decode_combine_kernel<8><<<dim3(heads_k, batch), 256, 0, st>>>(p);
   return check_launch("decode_combine");
 }
 
