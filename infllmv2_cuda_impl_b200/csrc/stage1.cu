@@ -241,47 +241,37 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     }
   } else if (warp <= 2) {
     // ================================================================ MMA issuer of query tile hq
-    // All 32 lanes run the same issue code (descriptors stay in uniform registers); `leader`
-    // enables the MMA / commit instructions in one lane only.
-    if (n_steps > 0) {
-      const int hq = __shfl_sync(0xFFFFFFFFu, warp - 1, 0);
-      const uint32_t leader = (lane == 0) ? 1u : 0u;
+    // One elected thread runs the whole loop.
+    if (n_steps > 0 && elect_one()) {
+      const int hq = warp - 1;
       constexpr uint32_t idesc = umma_idesc_bf16(128, 128, false);
-      const uint64_t q_desc = umma_desc_sw128(smem_u32(sm.q[0][0]), 16, 1024) + (uint32_t)hq * ((2 * kHalfBytes) >> 4);
-      const uint64_t kc_desc0 = umma_desc_sw128(smem_u32(sm.kc[0][0]), 16, 1024);
       constexpr uint32_t kStage = (2 * kHalfBytes) >> 4;      // descriptor address units per ring stage
+      const uint32_t q_lo = umma_desc_lo(smem_u32(sm.q[0][0]), 16) + (uint32_t)hq * kStage;
+      const uint32_t kc_lo0 = umma_desc_lo(smem_u32(sm.kc[0][0]), 16);
       const uint64_t d_ones = umma_desc_noswz16(smem_u32(sm.ones));
       const uint64_t d_rowc = umma_desc_noswz16(smem_u32(sm.rowc[0])) + (uint32_t)hq * (4096u >> 4);
       const uint32_t acc0 = tmem + (uint32_t)hq * 256u;
-      bool ok = __all_sync(0xFFFFFFFFu, mbar_wait(&sm.q_full, 0, abort_flag, p.status, 51));
+      bool ok = mbar_wait(&sm.q_full, 0, abort_flag, p.status, 51);
       for (int t = 0; t < n_steps && ok; ++t) {
         const int s = t % kStages, ab = t & 1;
         const bool pass2 = t >= n_tiles1;
-        bool w = mbar_wait(&sm.kc_full[s], (uint32_t)((t / kStages) & 1), abort_flag, p.status, 52);
-        if (w && t >= 2)
-          w = mbar_wait(&sm.acc_empty[hq][ab], (uint32_t)(((t >> 1) & 1) ^ 1), abort_flag, p.status, 53);
-        if (w && t == n_tiles1) w = mbar_wait(&sm.rowc_ready[hq], 0, abort_flag, p.status, 54);
-        ok = __all_sync(0xFFFFFFFFu, w);
+        ok = mbar_wait(&sm.kc_full[s], (uint32_t)((t / kStages) & 1), abort_flag, p.status, 52);
+        if (ok && t >= 2)
+          ok = mbar_wait(&sm.acc_empty[hq][ab], (uint32_t)(((t >> 1) & 1) ^ 1), abort_flag, p.status, 53);
+        if (ok && t == n_tiles1) ok = mbar_wait(&sm.rowc_ready[hq], 0, abort_flag, p.status, 54);
         if (!ok) break;
         tc_fence_after();
-        const uint64_t kc_desc = kc_desc0 + (uint32_t)s * kStage;
+        const uint32_t kc_lo = kc_lo0 + (uint32_t)s * kStage;
         const uint32_t acc = acc0 + (uint32_t)ab * 128u;
-        if (!pass2) {
+        const uint32_t a_lo = pass2 ? kc_lo : q_lo, b_lo = pass2 ? q_lo : kc_lo;
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            const uint32_t off = ((kk >> 2) * kHalfBytes + (kk & 3) * 32) >> 4;
-            umma_ss_pred(acc, q_desc + off, kc_desc + off, idesc, kk > 0, leader);
-          }
-        } else {
-#pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            const uint32_t off = ((kk >> 2) * kHalfBytes + (kk & 3) * 32) >> 4;
-            umma_ss_pred(acc, kc_desc + off, q_desc + off, idesc, kk > 0, leader);
-          }
-          umma_ss_pred(acc, d_ones, d_rowc, idesc, true, leader);   // + row constant
+        for (int kk = 0; kk < 8; ++kk) {
+          const uint32_t off = ((kk >> 2) * kHalfBytes + (kk & 3) * 32) >> 4;
+          umma_ss_lo(acc, a_lo + off, b_lo + off, idesc, kk > 0);
         }
-        umma_commit_pred(&sm.kc_free[s], leader);
-        umma_commit_pred(&sm.acc_full[hq][ab], leader);
+        if (pass2) umma_ss(acc, d_ones, d_rowc, idesc, true);   // + row constant
+        umma_commit(&sm.kc_free[s]);
+        umma_commit(&sm.acc_full[hq][ab]);
       }
     }
   } else {

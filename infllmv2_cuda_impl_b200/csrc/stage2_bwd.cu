@@ -245,84 +245,74 @@ sparse_attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q,
       }
     }
   } else if (warp == 1) {
-    // S = Q K^T.  All 32 lanes run the same issue code (descriptors stay in uniform registers);
-    // `leader` enables the MMA / commit instructions in one lane only.
-    if (n_blocks > 0) {
-      const uint32_t leader = (lane == 0) ? 1u : 0u;
+    // S = Q K^T.  One elected thread runs the whole loop of each issuing warp.
+    if (n_blocks > 0 && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, false);
-      const uint64_t k_desc0 = umma_desc_sw128(smem_u32(sm.k[0][0]), 16, 1024);
       constexpr uint32_t kStage = (2 * kKVHalfBytes) >> 4;     // descriptor address units per ring stage
+      const uint32_t k_lo0 = umma_desc_lo(smem_u32(sm.k[0][0]), 16);
       // Q and dO are A operands read from TMEM: the Q.K^T and dO.V^T products then fetch only
       // their 2 KB key tiles from shared memory per step instead of 6 KB
-      bool ok = __all_sync(0xFFFFFFFFu, mbar_wait(&sm.qdo_tmem, 0, abort_flag, p.status, 73));
+      bool ok = mbar_wait(&sm.qdo_tmem, 0, abort_flag, p.status, 73);
       tc_fence_after();
       int sk = 0, kround = 0;                       // j % 3, j / 3
       for (int j = 0; j < n_blocks && ok; ++j) {
         const int s = j & 1;
         const uint32_t par = (uint32_t)((j >> 1) & 1);
-        bool w = mbar_wait(&sm.k_full[sk], (uint32_t)(kround & 1), abort_flag, p.status, 74);
+        if (!mbar_wait(&sm.k_full[sk], (uint32_t)(kround & 1), abort_flag, p.status, 74)) break;
         // the S columns were last read by the softmax warps of step j - 2
-        if (w && j >= 2) w = mbar_wait(&sm.s_empty[s], par ^ 1u, abort_flag, p.status, 80);
-        if (!__all_sync(0xFFFFFFFFu, w)) break;
+        if (j >= 2 && !mbar_wait(&sm.s_empty[s], par ^ 1u, abort_flag, p.status, 80)) break;
         tc_fence_after();
-        const uint64_t k_desc = k_desc0 + (uint32_t)sk * kStage;
+        const uint32_t k_lo = k_lo0 + (uint32_t)sk * kStage;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t boff = ((kk >> 2) * kKVHalfBytes + (kk & 3) * 32) >> 4;
-          umma_ts_pred(tmem + s * 128, tmem_q + kk * 8, k_desc + boff, idesc_s, kk > 0, leader);
-        }
-        umma_commit_pred(&sm.s_full[s], leader);
+        for (int kk = 0; kk < 8; ++kk)
+          umma_ts_lo(tmem + s * 128, tmem_q + kk * 8, k_lo + (((kk >> 2) * kKVHalfBytes + (kk & 3) * 32) >> 4), idesc_s, kk > 0);
+        umma_commit(&sm.s_full[s]);
         if (++sk == 3) { sk = 0; ++kround; }
       }
     }
   } else if (warp == 3) {
     // dP = dO V^T, on a warp of its own: one warp issuing S and dP was busy four fifths of a step
-    if (n_blocks > 0) {
-      const uint32_t leader = (lane == 0) ? 1u : 0u;
+    if (n_blocks > 0 && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, false);
-      const uint64_t v_desc0 = umma_desc_sw128(smem_u32(sm.v[0][0]), 16, 1024);
       constexpr uint32_t kStage = (2 * kKVHalfBytes) >> 4;
-      bool ok = __all_sync(0xFFFFFFFFu, mbar_wait(&sm.qdo_tmem, 0, abort_flag, p.status, 67));
+      const uint32_t v_lo0 = umma_desc_lo(smem_u32(sm.v[0][0]), 16);
+      bool ok = mbar_wait(&sm.qdo_tmem, 0, abort_flag, p.status, 67);
       tc_fence_after();
       int sk2 = 1, kround2 = -1;                    // (j - 2) % 3, (j - 2) / 3 (used from j = 2 on)
       for (int j = 0; j < n_blocks && ok; ++j) {
         const int s = j & 1;
         const uint32_t par = (uint32_t)((j >> 1) & 1);
         // the dP columns hold dS of step j - 2 until its dQ product is complete
-        bool w = mbar_wait(&sm.v_full[s], par, abort_flag, p.status, 75);
-        if (w && j >= 2) w = mbar_wait(&sm.dq_done[sk2], (uint32_t)(kround2 & 1), abort_flag, p.status, 68);
-        if (!__all_sync(0xFFFFFFFFu, w)) break;
+        if (!mbar_wait(&sm.v_full[s], par, abort_flag, p.status, 75)) break;
+        if (j >= 2 && !mbar_wait(&sm.dq_done[sk2], (uint32_t)(kround2 & 1), abort_flag, p.status, 68)) break;
         tc_fence_after();
-        const uint64_t v_desc = v_desc0 + (uint32_t)s * kStage;
+        const uint32_t v_lo = v_lo0 + (uint32_t)s * kStage;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t boff = ((kk >> 2) * kKVHalfBytes + (kk & 3) * 32) >> 4;
-          umma_ts_pred(tmem + s * 128 + 64, tmem_do + kk * 8, v_desc + boff, idesc_s, kk > 0, leader);
-        }
-        umma_commit_pred(&sm.dp_full[s], leader);
+        for (int kk = 0; kk < 8; ++kk)
+          umma_ts_lo(tmem + s * 128 + 64, tmem_do + kk * 8, v_lo + (((kk >> 2) * kKVHalfBytes + (kk & 3) * 32) >> 4), idesc_s,
+                     kk > 0);
+        umma_commit(&sm.dp_full[s]);
         if (++sk2 == 3) { sk2 = 0; ++kround2; }
       }
     }
   } else if (warp == 2) {
     // dQ += dS K (dS as bf16 pairs in the step's TMEM buffer, K read along the keys)
-    if (n_blocks > 0) {
-      const uint32_t leader = (lane == 0) ? 1u : 0u;
+    if (n_blocks > 0 && elect_one()) {
       constexpr uint32_t idesc_dq = umma_idesc_bf16(128, 128, true);
-      const uint64_t k_desc0_mn = umma_desc_sw128(smem_u32(sm.k[0][0]), kKVHalfBytes, 1024);
       constexpr uint32_t kStage = (2 * kKVHalfBytes) >> 4;
+      const uint32_t k_lo0 = umma_desc_lo(smem_u32(sm.k[0][0]), kKVHalfBytes);
       int sk = 0, kround = 0;
       for (int i = 0; i < n_blocks; ++i) {
         const int s = i & 1;
-        bool w = mbar_wait(&sm.k_full[sk], (uint32_t)(kround & 1), abort_flag, p.status, 70);
-        if (w) w = mbar_wait(&sm.ds_ready[s], (uint32_t)((i >> 1) & 1), abort_flag, p.status, 76);
-        if (!__all_sync(0xFFFFFFFFu, w)) break;
+        if (!mbar_wait(&sm.k_full[sk], (uint32_t)(kround & 1), abort_flag, p.status, 70)) break;
+        if (!mbar_wait(&sm.ds_ready[s], (uint32_t)((i >> 1) & 1), abort_flag, p.status, 76)) break;
         tc_fence_after();
-        const uint64_t k_mn = k_desc0_mn + (uint32_t)sk * kStage;
+        const uint32_t k_lo = k_lo0 + (uint32_t)sk * kStage;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)      // dS of keys 0-31 sits at columns [64, 80), of keys 32-63 at [96, 112)
-          umma_ts_pred(tmem_dq, tmem + s * 128 + 64 + (kk >> 1) * 32 + (kk & 1) * 8, k_mn + ((kk * 2048) >> 4), idesc_dq,
-                       (i > 0) || (kk > 0), leader);
-        umma_commit_pred(&sm.dq_done[sk], leader);
+          umma_ts_lo(tmem_dq, tmem + s * 128 + 64 + (kk >> 1) * 32 + (kk & 1) * 8, k_lo + ((kk * 2048) >> 4), idesc_dq,
+                     (i > 0) || (kk > 0));
+        umma_commit(&sm.dq_done[sk]);
         if (++sk == 3) { sk = 0; ++kround; }
       }
     }
@@ -382,8 +372,7 @@ sparse_attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q,
       if (!ok) break;
       tc_fence_after();
       uint32_t x[32];
-      tmem_ld32(tmem + lane_off + s * 128 + grp * 32, x);
-      tmem_wait_ld_dep(x);
+      tmem_ld32_wait(tmem + lane_off + s * 128 + grp * 32, x);
       tc_fence_before();
       mbar_arrive_warp(&sm.s_empty[s]);
       {
@@ -403,8 +392,7 @@ sparse_attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q,
       uint32_t packed[16];
       {
         uint32_t dpv[32];
-        tmem_ld32(tmem + lane_off + s * 128 + 64 + grp * 32, dpv);
-        tmem_wait_ld_dep(dpv);
+        tmem_ld32_wait(tmem + lane_off + s * 128 + 64 + grp * 32, dpv);
         const uint64_t md2 = pack_f32x2(-dsum, -dsum);
 #pragma unroll
         for (int c = 0; c < 32; c += 2) {
@@ -676,84 +664,77 @@ sparse_attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q,
       }
     }
   } else if (warp == 1) {
-    // S and dP.  All 32 lanes run the same issue code (descriptors stay in uniform registers);
-    // `leader` enables the MMA / commit instructions in one lane only.
-    if (!never_selected) {
-      const uint32_t leader = (lane == 0) ? 1u : 0u;
+    // S and dP.  One elected thread runs the whole loop of each issuing warp.
+    if (!never_selected && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, false);             // K-major x K-major
-      const uint64_t k_desc = umma_desc_sw128(smem_u32(sm.k[0]), 16, 1024);
-      const uint64_t v_desc = umma_desc_sw128(smem_u32(sm.v[0]), 16, 1024);
-      // ring slot s = slot 0 + s * kRing (plain arithmetic keeps the descriptors in registers)
-      const uint64_t q_desc0 = umma_desc_sw128(smem_u32(sm.q[0][0]), 16, 1024);
-      const uint64_t do_desc0 = umma_desc_sw128(smem_u32(sm.dout[0][0]), 16, 1024);
-      constexpr uint32_t kRing = (2 * kTileHalfBytes) >> 4;
-      bool ok = __all_sync(0xFFFFFFFFu, mbar_wait(&sm.kv_full, 0, abort_flag, p.status, 82));
+      constexpr uint32_t kRing = (2 * kTileHalfBytes) >> 4;                     // descriptor address units per ring slot
+      const uint32_t k_lo = umma_desc_lo(smem_u32(sm.k[0]), 16);
+      const uint32_t v_lo = umma_desc_lo(smem_u32(sm.v[0]), 16);
+      const uint32_t q_lo0 = umma_desc_lo(smem_u32(sm.q[0][0]), 16);
+      const uint32_t do_lo0 = umma_desc_lo(smem_u32(sm.dout[0][0]), 16);
+      bool ok = mbar_wait(&sm.kv_full, 0, abort_flag, p.status, 82);
       // (issuing S(j + 1) ahead of dP(j), so that the exponentials of a step would not wait for its
       // dO tile, measured 12 % slower: dS, dK and with them the Q slots then come later)
       int qs = 0, qround = 0;
       for (int j = 0; ok; ++j) {
         const int bf = j & 1;
         const uint32_t par = (uint32_t)((j >> 1) & 1);
-        bool w = mbar_wait(&sm.q_full[qs], (uint32_t)(qround & 1), abort_flag, p.status, 83);
-        if (!__all_sync(0xFFFFFFFFu, w)) break;
+        if (!mbar_wait(&sm.q_full[qs], (uint32_t)(qround & 1), abort_flag, p.status, 83)) break;
         if (j >= *total_steps) break;
-        if (j >= 2) w = mbar_wait(&sm.sdp_empty[bf], par ^ 1u, abort_flag, p.status, 84);
-        if (!__all_sync(0xFFFFFFFFu, w)) break;
+        if (j >= 2 && !mbar_wait(&sm.sdp_empty[bf], par ^ 1u, abort_flag, p.status, 84)) break;
+        tc_fence_after();
+        const uint32_t q_lo = q_lo0 + qs * kRing, do_lo = do_lo0 + bf * kRing;
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {
+          const uint32_t aoff = ((kk >> 2) * kTileHalfBytes + (kk & 3) * 32) >> 4;
+          const uint32_t boff = ((kk >> 2) * kKVHalfBytes + (kk & 3) * 32) >> 4;
+          umma_ss_lo(tmem + bf * 128, q_lo + aoff, k_lo + boff, idesc_s, kk > 0);
+        }
+        umma_commit(&sm.s_full[bf]);
+        if (!mbar_wait(&sm.do_full[bf], par, abort_flag, p.status, 90)) break;
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk) {
           const uint32_t aoff = ((kk >> 2) * kTileHalfBytes + (kk & 3) * 32) >> 4;
           const uint32_t boff = ((kk >> 2) * kKVHalfBytes + (kk & 3) * 32) >> 4;
-          umma_ss_pred(tmem + bf * 128, q_desc0 + qs * kRing + aoff, k_desc + boff, idesc_s, kk > 0, leader);
+          umma_ss_lo(tmem + bf * 128 + 64, do_lo + aoff, v_lo + boff, idesc_s, kk > 0);
         }
-        umma_commit_pred(&sm.s_full[bf], leader);
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&sm.do_full[bf], par, abort_flag, p.status, 90))) break;
-        tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t aoff = ((kk >> 2) * kTileHalfBytes + (kk & 3) * 32) >> 4;
-          const uint32_t boff = ((kk >> 2) * kKVHalfBytes + (kk & 3) * 32) >> 4;
-          umma_ss_pred(tmem + bf * 128 + 64, do_desc0 + bf * kRing + aoff, v_desc + boff, idesc_s, kk > 0, leader);
-        }
-        umma_commit_pred(&sm.dp_full[bf], leader);
-        umma_commit_pred(&sm.do_free[bf], leader);       // first of the two arrivals that release the dO slot
+        umma_commit(&sm.dp_full[bf]);
+        umma_commit(&sm.do_free[bf]);       // first of the two arrivals that release the dO slot
         if (++qs == 3) { qs = 0; ++qround; }
       }
     }
   } else if (warp == 2) {
     // dV^T (128 d x 64 keys) += dO^T . P ; dK^T += Q^T . dS ; K extent = the 128 tile rows
-    if (!never_selected) {
-      const uint32_t leader = (lane == 0) ? 1u : 0u;
+    if (!never_selected && elect_one()) {
       constexpr uint32_t idesc_t = umma_idesc_bf16(128, 64, true, true);        // MN-major x MN-major
-      const uint64_t p_desc = umma_desc_sw128(smem_u32(sm.pmat), 16, 1024);
-      const uint64_t ds_desc = umma_desc_sw128(smem_u32(sm.dsmat), 16, 1024);
-      const uint64_t q_mn0 = umma_desc_sw128(smem_u32(sm.q[0][0]), kTileHalfBytes, 1024);
-      const uint64_t do_mn0 = umma_desc_sw128(smem_u32(sm.dout[0][0]), kTileHalfBytes, 1024);
       constexpr uint32_t kRing = (2 * kTileHalfBytes) >> 4;
+      const uint32_t p_lo = umma_desc_lo(smem_u32(sm.pmat), 16);
+      const uint32_t ds_lo = umma_desc_lo(smem_u32(sm.dsmat), 16);
+      const uint32_t q_lo0 = umma_desc_lo(smem_u32(sm.q[0][0]), kTileHalfBytes);
+      const uint32_t do_lo0 = umma_desc_lo(smem_u32(sm.dout[0][0]), kTileHalfBytes);
       int qs = 0, qround = 0;
       for (int i = 0;; ++i) {
         const int ds = i & 1;
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&sm.q_full[qs], (uint32_t)(qround & 1), abort_flag, p.status, 94)))
-          break;
+        if (!mbar_wait(&sm.q_full[qs], (uint32_t)(qround & 1), abort_flag, p.status, 94)) break;
         if (i >= *total_steps) break;
         // P of step i follows S of step i, which followed the dO tile's arrival only in program
         // order of the other warp: wait for the tile here too
-        bool w = mbar_wait(&sm.do_full[ds], (uint32_t)((i >> 1) & 1), abort_flag, p.status, 95);
-        if (w) w = mbar_wait(&sm.p_ready, (uint32_t)(i & 1), abort_flag, p.status, 85);
-        if (!__all_sync(0xFFFFFFFFu, w)) break;
+        if (!mbar_wait(&sm.do_full[ds], (uint32_t)((i >> 1) & 1), abort_flag, p.status, 95)) break;
+        if (!mbar_wait(&sm.p_ready, (uint32_t)(i & 1), abort_flag, p.status, 85)) break;
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
-          umma_ss_pred(tmem_dv, do_mn0 + ds * kRing + ((kk * 2048) >> 4), p_desc + ((kk * 2048) >> 4), idesc_t,
-                       (i > 0) || (kk > 0), leader);
-        umma_commit_pred(&sm.do_free[ds], leader);       // second arrival: dO slot and P are free
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&sm.ds_ready, (uint32_t)(i & 1), abort_flag, p.status, 91))) break;
+          umma_ss_lo(tmem_dv, do_lo0 + ds * kRing + ((kk * 2048) >> 4), p_lo + ((kk * 2048) >> 4), idesc_t,
+                     (i > 0) || (kk > 0));
+        umma_commit(&sm.do_free[ds]);       // second arrival: dO slot and P are free
+        if (!mbar_wait(&sm.ds_ready, (uint32_t)(i & 1), abort_flag, p.status, 91)) break;
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
-          umma_ss_pred(tmem_dk, q_mn0 + qs * kRing + ((kk * 2048) >> 4), ds_desc + ((kk * 2048) >> 4), idesc_t,
-                       (i > 0) || (kk > 0), leader);
-        umma_commit_pred(&sm.dk_done[qs], leader);
+          umma_ss_lo(tmem_dk, q_lo0 + qs * kRing + ((kk * 2048) >> 4), ds_lo + ((kk * 2048) >> 4), idesc_t,
+                     (i > 0) || (kk > 0));
+        umma_commit(&sm.dk_done[qs]);
         if (++qs == 3) { qs = 0; ++qround; }
       }
     }
@@ -800,8 +781,7 @@ sparse_attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q,
         uint32_t x[32];                               // P of this thread's 32 columns, fp32 bits
         {
           uint32_t pp[16];
-          tmem_ld32(tmem + lane_off + bf * 128 + grp * 32, x);
-          tmem_wait_ld_dep(x);
+          tmem_ld32_wait(tmem + lane_off + bf * 128 + grp * 32, x);
           const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2), n2 = pack_f32x2(neg_lse, neg_lse);
 #pragma unroll
           for (int c = 0; c < 32; c += 2) {
@@ -831,8 +811,7 @@ sparse_attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q,
         tc_fence_after();
         {
           uint32_t dpv[32], dd[16];
-          tmem_ld32(tmem + lane_off + bf * 128 + 64 + grp * 32, dpv);
-          tmem_wait_ld_dep(dpv);
+          tmem_ld32_wait(tmem + lane_off + bf * 128 + 64 + grp * 32, dpv);
           tc_fence_before();
           mbar_arrive_warp(&sm.sdp_empty[bf]);               // S / dP of this buffer may be overwritten
           const uint64_t md2 = pack_f32x2(-dsum, -dsum);

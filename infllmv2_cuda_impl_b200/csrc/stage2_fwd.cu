@@ -202,33 +202,25 @@ sparse_attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q,
     }
   } else if (warp == 1) {
     // ================================================================ MMA issuer
-    // All 32 lanes run the same issue code (descriptors stay in uniform registers); `leader`
-    // enables the MMA / commit instructions in one lane only.
-    if (n_blocks > 0) {
-      const uint32_t leader = (lane == 0) ? 1u : 0u;
+    // One elected thread runs the whole loop.
+    if (n_blocks > 0 && elect_one()) {
       constexpr uint32_t idesc_qk = umma_idesc_bf16(128, 64, false);
       constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 128, true);
-      const uint64_t q_desc = umma_desc_sw128(smem_u32(sm.q[0]), 16, 1024);
-      // ring stage s = stage 0 + s * kStage: plain arithmetic keeps the descriptors in registers
-      // (a runtime-indexed array of descriptors would live in local memory)
-      const uint64_t k_desc0 = umma_desc_sw128(smem_u32(sm.k[0][0]), 16, 1024);
-      const uint64_t v_desc0 = umma_desc_sw128(smem_u32(sm.v[0][0]), kKVHalfBytes, 1024);
-      constexpr uint32_t kStage = (2 * kKVHalfBytes) >> 4;
-      bool ok = __all_sync(0xFFFFFFFFu, mbar_wait(&sm.q_full, 0, abort_flag, p.status, 21));
+      constexpr uint32_t kStage = (2 * kKVHalfBytes) >> 4;         // descriptor address units per ring stage
+      const uint32_t q_lo = umma_desc_lo(smem_u32(sm.q[0]), 16);
+      const uint32_t k_lo0 = umma_desc_lo(smem_u32(sm.k[0][0]), 16);
+      const uint32_t v_lo0 = umma_desc_lo(smem_u32(sm.v[0][0]), kKVHalfBytes);
+      bool ok = mbar_wait(&sm.q_full, 0, abort_flag, p.status, 21);
       auto issue_qk = [&](int j) -> bool {
         const int s = j & 1;
-        if (!__all_sync(0xFFFFFFFFu, mbar_wait(&sm.k_full[s], (uint32_t)((j >> 1) & 1), abort_flag,
-                                               p.status, 22)))
-          return false;
+        if (!mbar_wait(&sm.k_full[s], (uint32_t)((j >> 1) & 1), abort_flag, p.status, 22)) return false;
         tc_fence_after();
+        const uint32_t k_lo = k_lo0 + s * kStage;
 #pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t qoff = (kk >> 2) * kQHalfBytes + (kk & 3) * 32;
-          const uint32_t koff = (kk >> 2) * kKVHalfBytes + (kk & 3) * 32;
-          umma_ss_pred(tmem + s * 64, q_desc + (qoff >> 4), k_desc0 + s * kStage + (koff >> 4), idesc_qk,
-                       kk > 0, leader);
-        }
-        umma_commit_pred(&sm.qk_done[s], leader);
+        for (int kk = 0; kk < 8; ++kk)
+          umma_ss_lo(tmem + s * 64, q_lo + (((kk >> 2) * kQHalfBytes + (kk & 3) * 32) >> 4),
+                     k_lo + (((kk >> 2) * kKVHalfBytes + (kk & 3) * 32) >> 4), idesc_qk, kk > 0);
+        umma_commit(&sm.qk_done[s]);
         return true;
       };
       if (ok) ok = issue_qk(0);
@@ -238,15 +230,15 @@ sparse_attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q,
         if (i + 1 < n_blocks) ok = issue_qk(i + 1);
         if (!ok) break;
         // (V landed long ago: its wait goes first so that it is not paid after P is ready)
-        ok = __all_sync(0xFFFFFFFFu, mbar_wait(&sm.v_full[s], par, abort_flag, p.status, 24) &&
-                                         mbar_wait(&sm.p_ready[s], par, abort_flag, p.status, 23));
+        ok = mbar_wait(&sm.v_full[s], par, abort_flag, p.status, 24) &&
+             mbar_wait(&sm.p_ready[s], par, abort_flag, p.status, 23);
         if (!ok) break;
         tc_fence_after();
+        const uint32_t v_lo = v_lo0 + s * kStage;
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk)
-          umma_ts_pred(tmem_o, tmem + s * 64 + kk * 8, v_desc0 + s * kStage + ((kk * 2048) >> 4), idesc_pv,
-                       (i > 0) || (kk > 0), leader);
-        umma_commit_pred(&sm.pv_done[s], leader);
+          umma_ts_lo(tmem_o, tmem + s * 64 + kk * 8, v_lo + ((kk * 2048) >> 4), idesc_pv, (i > 0) || (kk > 0));
+        umma_commit(&sm.pv_done[s]);
       }
     }
   } else {
