@@ -30,6 +30,7 @@ struct BlockWalk {
 struct WalkBatch {
   int blk;                 // lane l: number 32 n + l of the walk
   uint32_t sel;            // bit l: this lane's token selected it
+  uint32_t any;            // bit l: one of the warp's tokens did
   // umask: union mask in shared memory; masked: token selections come from row0 / row1 (this warp's two
   // tokens, null = not a token of the sequence), otherwise every block counts as selected
   __device__ void refill(const unsigned long long* umask, int words, int i0, bool masked,
@@ -71,6 +72,7 @@ struct WalkBatch {
     }
     const uint32_t b0 = __ballot_sync(0xFFFFFFFFu, s0), b1 = __ballot_sync(0xFFFFFFFFu, s1);
     sel = lane < 16 ? b0 : b1;
+    any = b0 | b1;
   }
 };
 

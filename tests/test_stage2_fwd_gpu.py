@@ -284,3 +284,18 @@ def test_function_mode_sees_the_forward_operator():
         out = infllm_v2.infllmv2_attn_varlen_func(q, k, v, *args, causal=True)
     assert torch.equal(out, plain)
     assert any("_infllmv2_attn_varlen_forward" in s for s in seen)
+
+
+@pytest.mark.parametrize("lk", [256, 250])
+def test_fwd_blocks_that_one_pair_of_tokens_selects(lk):
+    # a softmax warp owns two of a tile's eight tokens and skips the blocks that only others selected: its
+    # first block, its last one, all but one and, with lk = 250, the ragged block that is never skipped
+    hq, hk, d = 32, 2, 128
+    q, k, v = (det_tensor((n, h, d), 80 + i, 0.5) for i, (n, h) in enumerate(((16, hq), (lk, hk), (lk, hk))))
+    idx = torch.full((hk, 16, 2), -1, dtype=torch.int32)
+    for t in range(16):
+        pair = (t % 8) // 2
+        idx[:, t, 0] = 3 - pair if t < 8 else pair
+        if t % 2 and t >= 8:
+            idx[:, t, 0], idx[:, t, 1] = min(pair, (pair + 1) % 4), max(pair, (pair + 1) % 4)
+    _check(q, k, v, cu([16]), cu([lk]), idx, False)
