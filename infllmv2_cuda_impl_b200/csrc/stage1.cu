@@ -80,6 +80,7 @@ struct Stage1Params {
   const int32_t* leftpad_k;       // scored keys start this many rows into the sequence's extent, or null
   const int32_t* block_table;     // (batch, bt_stride) page of every page_size scored keys, or null
   int bt_stride, page_size;
+  int batch, max_tiles;           // sequences, and the most 16-token tiles of one
   int64_t total_q;
   int heads_q, heads_k;
   int max_seqlen_k;
@@ -101,7 +102,8 @@ struct Smem {
   // kc_free[s]: the products of BOTH query tiles that read key slot s are complete (2 arrivals);
   // per query tile: acc_full[b]: accumulator buffer b holds a step's scores; acc_empty[b]: its 8
   // softmax warps have read it
-  uint64_t q_full, kc_full[kStages], kc_free[kStages], acc_full[2][2], acc_empty[2][2], rowc_ready[2],
+  // q_full[t] / q_free[t]: the item's Q tile t has landed / all its products are complete.
+  uint64_t q_full[2], q_free[2], kc_full[kStages], kc_free[kStages], acc_full[2][2], acc_empty[2][2], rowc_ready[2],
       pool_full[2][3];
   uint32_t tmem_base;
   int abort_flag;
@@ -121,7 +123,87 @@ __device__ __forceinline__ float bf16_round(float x) {
   return __bfloat162float(__float2bfloat16_rn(x));
 }
 
-template <bool kPooled>
+// Barrier of the 256 softmax threads of query tile hq that tells all of them whether one said yes.
+__device__ __forceinline__ bool any_of_tile(int hq, bool yes) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.red.or.pred q, %2, 256, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(any) : "r"((uint32_t)yes), "r"(hq + 1) : "memory");
+  return any != 0;
+}
+
+// One work item: 16 tokens of a sequence and one KV head.
+struct Item {
+  int b, h, q0, lq, k0, lc, v0, lcv, st1, tok0, ntok;
+  int n_tiles1, n_steps;                       // pass-1 key tiles, and with the pass-2 tiles behind them
+
+  __device__ Item(const Stage1Params& p, int b_, int h_, int tile) : b(b_), h(h_) {
+    q0 = __ldg(p.cu_q + b);
+    lq = __ldg(p.cu_q + b + 1) - q0;
+    // scored keys of the sequence: rows [k0, k0 + lc) of a packed tensor (optionally starting
+    // `leftpad_k` rows into the sequence's extent), or positions [0, lc) of a paged cache
+    const int pad = p.leftpad_k ? __ldg(p.leftpad_k + b) : 0;
+    const int first = __ldg(p.cu_k + b), extent = __ldg(p.cu_k + b + 1) - first;
+    k0 = p.block_table ? 0 : first + pad;
+    lc = max(0, (p.seqused_k ? min(__ldg(p.seqused_k + b), extent) : extent) - pad);
+    tok0 = tile * kTokPerCta;
+    ntok = min(kTokPerCta, lq - tok0);
+    // Pass 1 (row sums) runs over the keys given as `v`: the same compressed keys, or a coarser
+    // compression (kernel 128 / stride 64) whose log-sum-exp then normalises the scores of
+    // pass 2 -- the reference switches on the key counts (flash_fwd_kernel.h:1236-1240)
+    v0 = k0;
+    lcv = lc;
+    if (p.cu_v) {
+      v0 = __ldg(p.cu_v + b);
+      lcv = __ldg(p.cu_v + b + 1) - v0;
+      if (p.seqused_v) lcv = max(0, min(__ldg(p.seqused_v + b), lcv));
+    }
+    st1 = (lcv == lc) ? 16 : 64;
+    // (limits grow with the token)
+    n_tiles1 = (visible_limit(tok0 + ntok - 1, lq, lcv, p.causal, st1) + kKeysPerTile - 1) / kKeysPerTile;
+    n_steps = n_tiles1 + (visible_limit(tok0 + ntok - 1, lq, lc, p.causal) + kKeysPerTile - 1) / kKeysPerTile;
+  }
+};
+
+// The items of a CTA, in the order in which every role of it takes them.  Without kStay: the one of its grid
+// position.  With kStay all items are numbered sequence by sequence, long tiles first, KV heads side by side,
+// and dealt out to the CTAs in rounds of gridDim.x, every other round backwards (forwards only, CTA 0 would get
+// the longest tile of every round).
+template <bool kStay>
+struct ItemWalk {
+  int b, count, base, round;                   // sequence, its number of items, number of its first item (an item
+                                               // has at least one query row: 32 bits)
+  __device__ ItemWalk() : b(-1), count(0), base(0), round(0) {}
+  // the next item's sequence is b; its head and tile come back; false when there are no more
+  __device__ bool next(const Stage1Params& p, int& h, int& tile) {
+    if (!kStay) {
+      if (b >= 0) return false;
+      b = blockIdx.y;
+      h = blockIdx.z;
+      tile = p.max_tiles - 1 - (int)blockIdx.x;
+      return true;
+    }
+    const int at = (round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
+    const int w = round * (int)gridDim.x + at;
+    ++round;
+    while (b < 0 || w >= base + count) {
+      base += count;
+      if (++b >= p.batch) return false;
+      count = min((__ldg(p.cu_q + b + 1) - __ldg(p.cu_q + b) + kTokPerCta - 1) / kTokPerCta, p.max_tiles) * p.heads_k;
+    }
+    const int i = w - base;
+    h = i % p.heads_k;
+    tile = count / p.heads_k - 1 - i / p.heads_k;
+    return true;
+  }
+};
+
+// kStay: one CTA per SM takes items until there are none, and every barrier, ring slot and accumulator buffer
+// runs on across them, so that an item's keys and Q arrive, and its first products run, while the softmax warps
+// finish the item before.  (u: steps since the start of the kernel, it: items with steps.)  What a CTA does
+// besides its steps (start, first tiles, change of pass, end) is ~10 us, as much as 7 steps.
+template <bool kPooled, bool kStay>
 __global__ void __launch_bounds__(kThreads, 1)      // 19 warps: at most 96 registers per thread
 stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kc,
               const __grid_constant__ CUtensorMap map_kv, const Stage1Params p) {
@@ -129,62 +211,47 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   Smem& sm = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                       ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.y, h = blockIdx.z;
   // (read beside the sequence tables: one trip to memory in front of a CTA instead of two)
   const int32_t failed = *reinterpret_cast<volatile int32_t*>(p.status);
-  const int q0 = p.cu_q[b], lq = p.cu_q[b + 1] - q0;
-  // scored keys of the sequence: rows [k0, k0 + lc) of a packed tensor (optionally starting
-  // `leftpad_k` rows into the sequence's extent), or positions [0, lc) of a paged cache
-  int k0, lc;
-  {
-    const int pad = p.leftpad_k ? p.leftpad_k[b] : 0;
-    const int extent = p.cu_k[b + 1] - p.cu_k[b];
-    k0 = p.block_table ? 0 : p.cu_k[b] + pad;
-    lc = max(0, (p.seqused_k ? min(p.seqused_k[b], extent) : extent) - pad);
+  ItemWalk<kStay> walk;
+  int h, tile16;
+  if (!kStay) {
+    walk.next(p, h, tile16);
+    if (tile16 * kTokPerCta >= p.cu_q[walk.b + 1] - p.cu_q[walk.b]) return;
   }
-  const int tok0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kTokPerCta;   // long tiles first
-  if (tok0 >= lq) return;
   // an earlier CTA of this launch gave up on a wait: do not pile up more waits
-  if (failed != 0) return;
-  const int ntok = min(kTokPerCta, lq - tok0);
-  const int lim_max = visible_limit(tok0 + ntok - 1, lq, lc, p.causal);    // limits grow with i
-  // Pass 1 (row sums) runs over the keys given as `v`: the same compressed keys, or a coarser
-  // compression (kernel 128 / stride 64) whose log-sum-exp then normalises the scores of
-  // pass 2 -- the reference switches on the key counts (flash_fwd_kernel.h:1236-1240)
-  const int v0 = p.cu_v ? p.cu_v[b] : k0;
-  const int lcv = !p.cu_v ? lc
-                  : p.seqused_v ? max(0, min(p.seqused_v[b], p.cu_v[b + 1] - v0)) : p.cu_v[b + 1] - v0;
-  const int st1 = (lcv == lc) ? 16 : 64;
-  const int lim_max1 = visible_limit(tok0 + ntok - 1, lq, lcv, p.causal, st1);
-  // (read through a warp broadcast: it tells the compiler that the value is warp-uniform, so the
-  //  MMA issuer's descriptor arithmetic stays in uniform registers instead of being moved there
-  //  operand by operand for every MMA)
-  const int n_tiles = __shfl_sync(0xFFFFFFFFu, (lim_max + kKeysPerTile - 1) / kKeysPerTile, 0);
-  const int n_tiles1 = __shfl_sync(0xFFFFFFFFu, (lim_max1 + kKeysPerTile - 1) / kKeysPerTile, 0);
-  const int n_steps = n_tiles1 + n_tiles;      // pass-1 tiles, then pass-2 tiles
+  if (kStay ? __syncthreads_or(failed != 0) : failed != 0) return;
+  // (kStay: nothing of this item is used)
+  const Item own(p, kStay ? 0 : walk.b, kStay ? 0 : h, kStay ? 0 : tile16);
 
-  // copies of step t's key tile into its ring slot (the copy warp's lane 0)
-  auto fetch_keys = [&](int t) {
-    const int s = t % kStages;
-    const bool first_pass = t < n_tiles1;
-    const int pos = (first_pass ? t : t - n_tiles1) * kKeysPerTile;
-    int row = (first_pass ? v0 : k0) + pos;      // (paged: the row sums run over the scored keys themselves)
-    if (p.block_table != nullptr)                // a 128-key tile never straddles a page
-      row = __ldg(p.block_table + (int64_t)b * p.bt_stride + pos / p.page_size) * p.page_size + pos % p.page_size;
-    mbar_expect_tx(&sm.kc_full[s], 2 * kHalfBytes);
-    tma_load_3d(sm.kc[s][0], first_pass ? &map_kv : &map_kc, &sm.kc_full[s], 0, h, row);
-    tma_load_3d(sm.kc[s][1], first_pass ? &map_kv : &map_kc, &sm.kc_full[s], 64, h, row);
+  // copies for the copy warp's lane 0: Q tile `tile` of an item, and the key tile of its step t into ring slot s
+  auto fetch_q = [&](const Item& w, int tile) {
+    mbar_expect_tx(&sm.q_full[tile], 2 * kHalfBytes);
+    for (int dh = 0; dh < 2; ++dh)               // rows past the last token come back as zeros or as
+      tma_load_3d(sm.q[tile][dh], &map_q, &sm.q_full[tile], dh * 64, w.h * kGroup,   // the next sequence's rows; they are
+                  w.q0 + w.tok0 + tile * kTokPerBox);                                // never stored
   };
-  const int n_ahead = min(kStages, n_steps);     // steps whose keys are fetched before the CTA is set up
+  auto fetch_keys = [&](const Item& w, int t, int s) {
+    const bool first_pass = t < w.n_tiles1;
+    const int pos = (first_pass ? t : t - w.n_tiles1) * kKeysPerTile;
+    int row = (first_pass ? w.v0 : w.k0) + pos;      // (paged: the row sums run over the scored keys themselves)
+    if (p.block_table != nullptr)                // a 128-key tile never straddles a page
+      row = __ldg(p.block_table + (int64_t)w.b * p.bt_stride + pos / p.page_size) * p.page_size + pos % p.page_size;
+    mbar_expect_tx(&sm.kc_full[s], 2 * kHalfBytes);
+    tma_load_3d(sm.kc[s][0], first_pass ? &map_kv : &map_kc, &sm.kc_full[s], 0, w.h, row);
+    tma_load_3d(sm.kc[s][1], first_pass ? &map_kv : &map_kc, &sm.kc_full[s], 64, w.h, row);
+  };
+  const int n_ahead = kStay ? 0 : min(kStages, own.n_steps);     // steps whose keys are fetched before the CTA is set up
 
   if (threadIdx.x == 0) {
     sm.abort_flag = 0;
-    mbar_init(&sm.q_full, 1);
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&sm.kc_full[s], 1);
       mbar_init(&sm.kc_free[s], 2);               // one commit per MMA warp
     }
     for (int hq = 0; hq < 2; ++hq) {
+      mbar_init(&sm.q_full[hq], 1);
+      mbar_init(&sm.q_free[hq], 1);
       for (int s = 0; s < 2; ++s) {
         mbar_init(&sm.acc_full[hq][s], 1);
         mbar_init(&sm.acc_empty[hq][s], 8);       // one arrival per softmax warp of the tile
@@ -196,12 +263,10 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     // The first copies leave at once: they fly while TMEM is allocated and the constant tiles are written.
     // With one CTA per SM nothing else covers them (0.910 -> 0.897 ms at 32768 tokens, 0.461 -> 0.453 ms for
     // a ragged batch of 31630, together with the status word read beside the tables).
-    if (n_steps > 0) {
-      mbar_expect_tx(&sm.q_full, 4 * kHalfBytes);
-      for (int tile = 0; tile < 2; ++tile)       // rows past the last token come back as zeros or as
-        for (int dh = 0; dh < 2; ++dh)           // the next sequence's rows; they are never stored
-          tma_load_3d(sm.q[tile][dh], &map_q, &sm.q_full, dh * 64, h * kGroup, q0 + tok0 + tile * kTokPerBox);
-      for (int t = 0; t < n_ahead; ++t) fetch_keys(t);
+    if (n_ahead > 0) {
+      fetch_q(own, 0);
+      fetch_q(own, 1);
+      for (int t = 0; t < n_ahead; ++t) fetch_keys(own, t, t);
     }
   }
   if (warp == 1) {
@@ -223,26 +288,41 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, sm.tmem_base, 0);
   volatile int* abort_flag = &sm.abort_flag;
-
   if (warp == 0) {
     // ================================================================ TMA producer
-    if (lane == 0 && n_steps > 0) {
-      int issued = n_ahead;
-      for (int t = n_ahead; t < n_steps; ++t) {
-        if (!mbar_wait(&sm.kc_free[t % kStages], (uint32_t)((t / kStages - 1) & 1), abort_flag, p.status, 41)) break;
-        fetch_keys(t);
-        issued = t + 1;
+    if (lane == 0) {
+      int u = n_ahead, it = kStay ? 0 : 1;
+      bool ok = true;
+      while (ok && (!kStay || walk.next(p, h, tile16))) {
+        const Item w = kStay ? Item(p, walk.b, h, tile16) : own;
+        for (int t = n_ahead; t < w.n_steps && ok; ++t) {
+          // (two key tiles go ahead of Q: their ring slots are free before the last products of the item before)
+          if (kStay && t == min(2, w.n_steps - 1)) {
+            for (int tile = 0; tile < 2 && ok; ++tile) {
+              if (it > 0) ok = mbar_wait(&sm.q_free[tile], (uint32_t)((it - 1) & 1), abort_flag, p.status, 42);
+              if (ok) fetch_q(w, tile);
+            }
+            if (!ok) break;
+            ++it;
+          }
+          const int s = u % kStages;
+          if (u >= kStages) ok = mbar_wait(&sm.kc_free[s], (uint32_t)((u / kStages - 1) & 1), abort_flag, p.status, 41);
+          if (!ok) break;
+          fetch_keys(w, t, s);
+          ++u;
+        }
+        if (!kStay) break;
       }
       if (*abort_flag) {
-        mbar_wait_drain(&sm.q_full, 0);
-        for (int j = max(0, issued - kStages); j < issued; ++j)
+        for (int tile = 0; tile < 2 && it > 0 && u > 0; ++tile) mbar_wait_drain(&sm.q_full[tile], (uint32_t)((it - 1) & 1));
+        for (int j = max(0, u - kStages); j < u; ++j)
           mbar_wait_drain(&sm.kc_full[j % kStages], (uint32_t)((j / kStages) & 1));
       }
     }
   } else if (warp <= 2) {
     // ================================================================ MMA issuer of query tile hq
     // One elected thread runs the whole loop.
-    if (n_steps > 0 && elect_one()) {
+    if (elect_one()) {
       const int hq = warp - 1;
       constexpr uint32_t idesc = umma_idesc_bf16(128, 128, false);
       constexpr uint32_t kStage = (2 * kHalfBytes) >> 4;      // descriptor address units per ring stage
@@ -251,27 +331,39 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       const uint64_t d_ones = umma_desc_noswz16(smem_u32(sm.ones));
       const uint64_t d_rowc = umma_desc_noswz16(smem_u32(sm.rowc[0])) + (uint32_t)hq * (4096u >> 4);
       const uint32_t acc0 = tmem + (uint32_t)hq * 256u;
-      bool ok = mbar_wait(&sm.q_full, 0, abort_flag, p.status, 51);
-      for (int t = 0; t < n_steps && ok; ++t) {
-        const int s = t % kStages, ab = t & 1;
-        const bool pass2 = t >= n_tiles1;
-        ok = mbar_wait(&sm.kc_full[s], (uint32_t)((t / kStages) & 1), abort_flag, p.status, 52);
-        if (ok && t >= 2)
-          ok = mbar_wait(&sm.acc_empty[hq][ab], (uint32_t)(((t >> 1) & 1) ^ 1), abort_flag, p.status, 53);
-        if (ok && t == n_tiles1) ok = mbar_wait(&sm.rowc_ready[hq], 0, abort_flag, p.status, 54);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t kc_lo = kc_lo0 + (uint32_t)s * kStage;
-        const uint32_t acc = acc0 + (uint32_t)ab * 128u;
-        const uint32_t a_lo = pass2 ? kc_lo : q_lo, b_lo = pass2 ? q_lo : kc_lo;
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint32_t off = ((kk >> 2) * kHalfBytes + (kk & 3) * 32) >> 4;
-          umma_ss_lo(acc, a_lo + off, b_lo + off, idesc, kk > 0);
+      int u = 0, it = 0;
+      bool ok = true;
+      while (ok && (!kStay || walk.next(p, h, tile16))) {
+        const Item w = kStay ? Item(p, walk.b, h, tile16) : own;
+        if (w.n_steps == 0) {
+          if (kStay) continue;
+          break;
         }
-        if (pass2) umma_ss(acc, d_ones, d_rowc, idesc, true);   // + row constant
-        umma_commit(&sm.kc_free[s]);
-        umma_commit(&sm.acc_full[hq][ab]);
+        ok = mbar_wait(&sm.q_full[hq], (uint32_t)(it & 1), abort_flag, p.status, 51);
+        for (int t = 0; t < w.n_steps && ok; ++t, ++u) {
+          const int s = u % kStages, ab = u & 1;
+          const bool pass2 = t >= w.n_tiles1;
+          ok = mbar_wait(&sm.kc_full[s], (uint32_t)((u / kStages) & 1), abort_flag, p.status, 52);
+          if (ok && u >= 2)
+            ok = mbar_wait(&sm.acc_empty[hq][ab], (uint32_t)(((u >> 1) & 1) ^ 1), abort_flag, p.status, 53);
+          if (ok && t == w.n_tiles1) ok = mbar_wait(&sm.rowc_ready[hq], (uint32_t)(it & 1), abort_flag, p.status, 54);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t kc_lo = kc_lo0 + (uint32_t)s * kStage;
+          const uint32_t acc = acc0 + (uint32_t)ab * 128u;
+          const uint32_t a_lo = pass2 ? kc_lo : q_lo, b_lo = pass2 ? q_lo : kc_lo;
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) {
+            const uint32_t off = ((kk >> 2) * kHalfBytes + (kk & 3) * 32) >> 4;
+            umma_ss_lo(acc, a_lo + off, b_lo + off, idesc, kk > 0);
+          }
+          if (pass2) umma_ss(acc, d_ones, d_rowc, idesc, true);   // + row constant
+          umma_commit(&sm.kc_free[s]);
+          umma_commit(&sm.acc_full[hq][ab]);
+          if (kStay && t == w.n_steps - 1) umma_commit(&sm.q_free[hq]);
+        }
+        if (!kStay) break;
+        ++it;
       }
     }
   } else {
@@ -282,216 +374,230 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     const int r = quad * 32 + lane;                  // TMEM lane: pass 1 = query row, pass 2 = key
     const uint32_t lane_off = ((uint32_t)(quad * 32) << 16) + (uint32_t)(hq * 256 + grp * 64);
     const int st = threadIdx.x - 96 - hq * kHalfThreads;   // 0..255 among the tile's softmax threads
-    const int tokh = tok0 + hq * kTokPerBox;         // first token of this tile
-    const int ntokh = min(max(ntok - hq * kTokPerBox, 0), kTokPerBox);
     uint64_t* acc_full = sm.acc_full[hq];
     uint64_t* acc_empty = sm.acc_empty[hq];
     uint64_t* pool_full = sm.pool_full[hq];
     bool ok = true;
+    uint32_t u = 0, pt = 0;                          // steps and pooled tiles since the start of the kernel
 
-    // ---------------- pass 1: sum of this thread's query row over its half of every key tile
-    {
-      const int tl = r >> 4;
-      const int lim_row = (tl < ntokh) ? visible_limit(tokh + tl, lq, lcv, p.causal, st1) : 0;
-      float m = -INFINITY, l = 0.f;
-      for (int t = 0; t < n_tiles1; ++t) {
-        const int ab = t & 1;
-        ok = mbar_wait_warp(&acc_full[ab], (uint32_t)((t >> 1) & 1), abort_flag, p.status, 61);
-        if (!ok) break;
-        tc_fence_after();
-        // visible columns among this group's 64
-        const int lim = min(max(lim_row - t * kKeysPerTile - grp * 64, 0), 64);
-        const bool full = __all_sync(0xFFFFFFFFu, lim == 64);
-        uint32_t x[64];
-        tmem_ld64_wait(tmem + lane_off + ab * 128, x);
-        // the scores are in registers: the accumulator goes back to the MMA warp at once
-        tc_fence_before();
-        mbar_arrive_warp(&acc_empty[ab]);
-        if (!full) {
+    while (ok && (!kStay || walk.next(p, h, tile16))) {
+      const Item w = kStay ? Item(p, walk.b, h, tile16) : own;
+      const int b = w.b, q0 = w.q0, lq = w.lq, lc = w.lc, lcv = w.lcv, st1 = w.st1;
+      const int n_tiles1 = w.n_tiles1, n_tiles = w.n_steps - w.n_tiles1;
+      const int tokh = w.tok0 + hq * kTokPerBox;       // first token of this tile
+      const int ntokh = min(max(w.ntok - hq * kTokPerBox, 0), kTokPerBox);
+      // ---------------- pass 1: sum of this thread's query row over its half of every key tile
+      {
+        const int tl = r >> 4;
+        const int lim_row = (tl < ntokh) ? visible_limit(tokh + tl, lq, lcv, p.causal, st1) : 0;
+        float m = -INFINITY, l = 0.f;
+        for (int t = 0; t < n_tiles1; ++t, ++u) {
+          const uint32_t ab = u & 1;
+          ok = mbar_wait_warp(&acc_full[ab], (u >> 1) & 1, abort_flag, p.status, 61);
+          if (!ok) break;
+          tc_fence_after();
+          // visible columns among this group's 64
+          const int lim = min(max(lim_row - t * kKeysPerTile - grp * 64, 0), 64);
+          const bool full = __all_sync(0xFFFFFFFFu, lim == 64);
+          uint32_t x[64];
+          tmem_ld64_wait(tmem + lane_off + ab * 128, x);
+          // the scores are in registers: the accumulator goes back to the MMA warp at once
+          tc_fence_before();
+          mbar_arrive_warp(&acc_empty[ab]);
+          if (!full) {
 #pragma unroll
-          for (int c = 0; c < 64; ++c)
-            if (c >= lim) x[c] = 0xFF800000u;                             // -inf
-        }
-        if (m == -INFINITY) {            // no visible score yet: the first one fixes the reference point
-          float mx = -INFINITY;
-#pragma unroll
-          for (int c = 0; c < 64; ++c) mx = fmaxf(mx, __uint_as_float(x[c]));
-          m = mx;
-        }
-        if (m > -INFINITY) {
-          float neg = -m * p.scale_log2;
-          const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2), n2 = pack_f32x2(neg, neg);
-          uint64_t s2[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) s2[i] = pack_f32x2(0.f, 0.f);
-#pragma unroll
-          for (int c = 0; c < 64; c += 2) {
-            float a0, a1;
-            unpack_f32x2(fma_f32x2(pack_f32x2(x[c], x[c + 1]), c2, n2), a0, a1);
-            s2[(c >> 1) & 3] = add_f32x2(s2[(c >> 1) & 3], pack_f32x2(exp2_mixed_unbounded(a0, c),
-                                                                      exp2_mixed_unbounded(a1, c + 1)));
+            for (int c = 0; c < 64; ++c)
+              if (c >= lim) x[c] = 0xFF800000u;                             // -inf
           }
-          float lo, hi;
-          unpack_f32x2(add_f32x2(add_f32x2(s2[0], s2[1]), add_f32x2(s2[2], s2[3])), lo, hi);
-          float cs = lo + hi;
-          if (!(cs < kSumLimit)) {       // a score far above the reference point: move the point to the maximum
-            float mx = m;
+          if (m == -INFINITY) {            // no visible score yet: the first one fixes the reference point
+            float mx = -INFINITY;
 #pragma unroll
             for (int c = 0; c < 64; ++c) mx = fmaxf(mx, __uint_as_float(x[c]));
-            l *= exp2f((m - mx) * p.scale_log2);
             m = mx;
-            neg = -m * p.scale_log2;
-            cs = 0.f;
-#pragma unroll
-            for (int c = 0; c < 64; ++c) cs += exp2f(fmaf(__uint_as_float(x[c]), p.scale_log2, neg));
           }
-          l += cs;
-        }
-      }
-      // merge the two key halves of every row, then publish the row constant for pass 2, in
-      // units of the raw score: -(m + log2(l) / c), as three bf16 terms
-      if (grp == 1) sm.stat[hq][r] = make_float2(m, l);
-      if (hq == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
-      else asm volatile("bar.sync 2, 256;" ::: "memory");
-      if (grp == 0) {
-        const float2 o = sm.stat[hq][r];
-        const float mm = fmaxf(m, o.x);
-        if (mm > -INFINITY)
-          l = l * ((m > -INFINITY) ? exp2f((m - mm) * p.scale_log2) : 0.f) +
-              o.y * ((o.x > -INFINITY) ? exp2f((o.x - mm) * p.scale_log2) : 0.f);
-        m = mm;
-        // a row without any visible pass-1 key scores 0 everywhere, as in the reference's oracle
-        // (tests/stage1/complse_online_softmax.py: its NaN row sum is scrubbed to 0)
-        const float rc = (l > 0.f) ? -(m + log2f(l) * p.inv_scale_log2) : -30000.f;
-        const float t0 = bf16_round(rc), t1 = bf16_round(rc - t0), t2 = bf16_round(rc - t0 - t1);
-        uint8_t* rowc = sm.rowc[hq];
-        *reinterpret_cast<__nv_bfloat16*>(rowc + umma_noswz16_off(r, 0)) = __float2bfloat16_rn(t0);
-        *reinterpret_cast<__nv_bfloat16*>(rowc + umma_noswz16_off(r, 1)) = __float2bfloat16_rn(t1);
-        *reinterpret_cast<__nv_bfloat16*>(rowc + umma_noswz16_off(r, 2)) = __float2bfloat16_rn(t2);
-        fence_proxy_async_smem();
-        mbar_arrive_warp(&sm.rowc_ready[hq]);
-      }
-    }
-
-    // ---------------- pass 2: this thread's key against 4 tokens x 16 heads
-    constexpr int kTokPerThread = kTokPerBox / 2;            // tokens grp*4 .. grp*4+3 of the tile
-    int lim_tok[kTokPerThread];
-    const int cache_len = p.cache_lens ? p.cache_lens[b] : p.cache_len;
+          if (m > -INFINITY) {
+            float neg = -m * p.scale_log2;
+            const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2), n2 = pack_f32x2(neg, neg);
+            uint64_t s2[4];
 #pragma unroll
-    for (int j = 0; j < kTokPerThread; ++j) {
-      // a token without any visible row-sum key scores exactly 0 (the huge negative row constant
-      // alone leaves 2^-125 per polynomial exponential)
-      const int tk = tokh + grp * kTokPerThread + j;
-      lim_tok[j] = (grp * kTokPerThread + j < ntokh && visible_limit(tk, lq, lcv, p.causal, st1) > 0)
-                       ? visible_limit(tk, lq, lc, p.causal) : 0;
-    }
-    __nv_bfloat16* out_base =
-        p.out ? p.out + ((int64_t)h * p.total_q + q0 + tokh) * p.out_row_stride : nullptr;
-    __nv_bfloat16* pool_base =
-        kPooled ? p.pooled + ((int64_t)h * p.total_q + q0 + tokh) * p.pooled_len : nullptr;
-    const __nv_bfloat16 ninf_b = __float2bfloat16_rn(-INFINITY);
-    __nv_bfloat16 (*pool)[kTokPerBox][kPoolSlots] = sm.pool[hq];
-    __nv_bfloat16 (*carry)[kTokPerBox] = sm.carry[hq];
-
-    // Max-pool of one finished key tile: 32 blocks x 8 tokens, one per thread.  It runs one tile
-    // late, after the next tile's exponentials, so that no warp waits for the others here.
-    auto pool_tile = [&](int tile) -> bool {
-      if (!mbar_wait_warp(&pool_full[tile % 3], (uint32_t)((tile / 3) & 1), abort_flag, p.status, 63))
-        return false;
-      {
-        const int t8 = st >> 5, bl = st & 31;
-        const int blk = tile * 32 + bl;
-        const __nv_bfloat16* w = &pool[tile % 3][t8][4 * bl];             // slots 4bl .. 4bl+4
-        float mxv = fmaxf(fmaxf(__bfloat162float(w[1]), __bfloat162float(w[2])),
-                          fmaxf(__bfloat162float(w[3]), __bfloat162float(w[4])));
-        float first = -INFINITY;                                          // key 4*blk - 1
-        if (bl > 0) first = __bfloat162float(w[0]);
-        else if (tile > 0) first = __bfloat162float(carry[(tile - 1) & 3][t8]);
-        mxv = fmaxf(mxv, first);
-        const int bq = (tokh + t8 + cache_len) / kBlockN;
-        if (blk < p.init_blocks || (bq >= blk && bq <= blk + p.local_blocks)) mxv = INFINITY;
-        if (t8 < ntokh && blk < p.pooled_len)
-          pool_base[(int64_t)t8 * p.pooled_len + blk] = __float2bfloat16_rn(mxv);
-      }
-      return true;
-    };
-
-    if (ok) {
-      for (int t = n_tiles1; t < n_steps; ++t) {
-        const int ab = t & 1, tile = t - n_tiles1;
-        ok = mbar_wait_warp(&acc_full[ab], (uint32_t)((t >> 1) & 1), abort_flag, p.status, 62);
-        if (!ok) break;
-        tc_fence_after();
-        const int key = tile * kKeysPerTile + r;
-        float val[kTokPerThread];
-        uint32_t x[64];                                   // 4 tokens x 16 heads
-        tmem_ld64_wait(tmem + lane_off + ab * 128, x);
-        // the accumulator is in registers now: hand it back before the arithmetic
-        tc_fence_before();
-        mbar_arrive_warp(&acc_empty[ab]);
-        {
-          const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2);
+            for (int i = 0; i < 4; ++i) s2[i] = pack_f32x2(0.f, 0.f);
 #pragma unroll
-          for (int j = 0; j < kTokPerThread; ++j) {
-            uint64_t a2[2] = {pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f)};
-#pragma unroll
-            for (int g = 0; g < 16; g += 2) {
-              float y0, y1;
-              unpack_f32x2(mul_f32x2(pack_f32x2(x[j * 16 + g], x[j * 16 + g + 1]), c2), y0, y1);
-              a2[(g >> 1) & 1] = add_f32x2(a2[(g >> 1) & 1], pack_f32x2(exp2_mixed(y0, g), exp2_mixed(y1, g + 1)));
+            for (int c = 0; c < 64; c += 2) {
+              float a0, a1;
+              unpack_f32x2(fma_f32x2(pack_f32x2(x[c], x[c + 1]), c2, n2), a0, a1);
+              s2[(c >> 1) & 3] = add_f32x2(s2[(c >> 1) & 3], pack_f32x2(exp2_mixed_unbounded(a0, c),
+                                                                        exp2_mixed_unbounded(a1, c + 1)));
             }
             float lo, hi;
-            unpack_f32x2(add_f32x2(a2[0], a2[1]), lo, hi);
-            val[j] = lo + hi;
-          }
-        }
-        if (kPooled && tile > 0) {
-          ok = pool_tile(tile - 1);
-          if (!ok) break;
-        }
+            unpack_f32x2(add_f32x2(add_f32x2(s2[0], s2[1]), add_f32x2(s2[2], s2[3])), lo, hi);
+            float cs = lo + hi;
+            if (!(cs < kSumLimit)) {       // a score far above the reference point: move the point to the maximum
+              float mx = m;
 #pragma unroll
-        for (int j = 0; j < kTokPerThread; ++j) {
-          const int t8 = grp * kTokPerThread + j;
-          // existing but invisible keys score 0; keys past the sequence do not exist (-inf in the pool)
-          const __nv_bfloat16 vb = __float2bfloat16_rn((key < lim_tok[j]) ? val[j] : 0.f);
-          if (out_base != nullptr && t8 < ntokh && key < p.max_seqlen_k)
-            out_base[(int64_t)t8 * p.out_row_stride + key] = vb;
-          if (kPooled) {
-            const __nv_bfloat16 pv = (key < lc) ? vb : ninf_b;
-            pool[tile % 3][t8][1 + r] = pv;
-            if (r == 127) carry[tile & 3][t8] = pv;
+              for (int c = 0; c < 64; ++c) mx = fmaxf(mx, __uint_as_float(x[c]));
+              l *= exp2f((m - mx) * p.scale_log2);
+              m = mx;
+              neg = -m * p.scale_log2;
+              cs = 0.f;
+#pragma unroll
+              for (int c = 0; c < 64; ++c) cs += exp2f(fmaf(__uint_as_float(x[c]), p.scale_log2, neg));
+            }
+            l += cs;
           }
         }
-        // (after the deferred pooling reads: this arrival is what lets a later tile reuse them)
-        if (kPooled) mbar_arrive_warp(&pool_full[tile % 3]);
-      }
-      if (ok && kPooled && n_tiles > 0) ok = pool_tile(n_tiles - 1);
-      // columns past the last tile are zero (rows are 16-byte aligned: stride % 8 == 0)
-      const int first = n_tiles * kKeysPerTile;
-      if (ok && out_base != nullptr && first < p.max_seqlen_k) {
-        const int vec_per_row = (p.max_seqlen_k - first + 7) / 8;   // may spill into row padding
-        const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-        for (int t8 = 0; t8 < ntokh; ++t8) {
-          uint4* dst = reinterpret_cast<uint4*>(out_base + (int64_t)t8 * p.out_row_stride + first);
-          for (int i = st; i < vec_per_row; i += kHalfThreads) dst[i] = z;
+        if (w.n_steps > 0) {
+        // merge the two key halves of every row, then publish the row constant for pass 2, in
+        // units of the raw score: -(m + log2(l) / c), as three bf16 terms
+        if (grp == 1) sm.stat[hq][r] = make_float2(m, l);
+        if (hq == 0) asm volatile("bar.sync 1, 256;" ::: "memory");
+        else asm volatile("bar.sync 2, 256;" ::: "memory");
+        if (grp == 0) {
+          const float2 o = sm.stat[hq][r];
+          const float mm = fmaxf(m, o.x);
+          if (mm > -INFINITY)
+            l = l * ((m > -INFINITY) ? exp2f((m - mm) * p.scale_log2) : 0.f) +
+                o.y * ((o.x > -INFINITY) ? exp2f((o.x - mm) * p.scale_log2) : 0.f);
+          m = mm;
+          // a row without any visible pass-1 key scores 0 everywhere, as in the reference's oracle
+          // (tests/stage1/complse_online_softmax.py: its NaN row sum is scrubbed to 0)
+          const float rc = (l > 0.f) ? -(m + log2f(l) * p.inv_scale_log2) : -30000.f;
+          const float t0 = bf16_round(rc), t1 = bf16_round(rc - t0), t2 = bf16_round(rc - t0 - t1);
+          uint8_t* rowc = sm.rowc[hq];
+          *reinterpret_cast<__nv_bfloat16*>(rowc + umma_noswz16_off(r, 0)) = __float2bfloat16_rn(t0);
+          *reinterpret_cast<__nv_bfloat16*>(rowc + umma_noswz16_off(r, 1)) = __float2bfloat16_rn(t1);
+          *reinterpret_cast<__nv_bfloat16*>(rowc + umma_noswz16_off(r, 2)) = __float2bfloat16_rn(t2);
+          fence_proxy_async_smem();
+          mbar_arrive_warp(&sm.rowc_ready[hq]);
+        }
         }
       }
-      // block scores past the last tile: their keys are invisible (0) or do not exist (-inf);
-      // the first such block still sees the last key of the last tile
-      if (ok && kPooled) {
-        const int first_blk = n_tiles * 32;
-        for (int t8 = 0; t8 < ntokh; ++t8) {
+
+      // ---------------- pass 2: this thread's key against 4 tokens x 16 heads
+      constexpr int kTokPerThread = kTokPerBox / 2;            // tokens grp*4 .. grp*4+3 of the tile
+      int lim_tok[kTokPerThread];
+      const int cache_len = p.cache_lens ? p.cache_lens[b] : p.cache_len;
+#pragma unroll
+      for (int j = 0; j < kTokPerThread; ++j) {
+        // a token without any visible row-sum key scores exactly 0 (the huge negative row constant
+        // alone leaves 2^-125 per polynomial exponential)
+        const int tk = tokh + grp * kTokPerThread + j;
+        lim_tok[j] = (grp * kTokPerThread + j < ntokh && visible_limit(tk, lq, lcv, p.causal, st1) > 0)
+                         ? visible_limit(tk, lq, lc, p.causal) : 0;
+      }
+      __nv_bfloat16* out_base =
+          p.out ? p.out + ((int64_t)h * p.total_q + q0 + tokh) * p.out_row_stride : nullptr;
+      __nv_bfloat16* pool_base =
+          kPooled ? p.pooled + ((int64_t)h * p.total_q + q0 + tokh) * p.pooled_len : nullptr;
+      const __nv_bfloat16 ninf_b = __float2bfloat16_rn(-INFINITY);
+      __nv_bfloat16 (*pool)[kTokPerBox][kPoolSlots] = sm.pool[hq];
+      __nv_bfloat16 (*carry)[kTokPerBox] = sm.carry[hq];
+
+      // Max-pool of one finished key tile: 32 blocks x 8 tokens, one per thread.  It runs one tile
+      // late, after the next tile's exponentials, so that no warp waits for the others here.
+      auto pool_tile = [&](int tile) -> bool {
+        const uint32_t pn = pt + (uint32_t)tile;                            // (slots run on across items)
+        if (!mbar_wait_warp(&pool_full[pn % 3], (pn / 3) & 1, abort_flag, p.status, 63))
+          return false;
+        {
+          const int t8 = st >> 5, bl = st & 31;
+          const int blk = tile * 32 + bl;
+          const __nv_bfloat16* win = &pool[pn % 3][t8][4 * bl];               // slots 4bl .. 4bl+4
+          float mxv = fmaxf(fmaxf(__bfloat162float(win[1]), __bfloat162float(win[2])),
+                            fmaxf(__bfloat162float(win[3]), __bfloat162float(win[4])));
+          float first = -INFINITY;                                          // key 4*blk - 1
+          if (bl > 0) first = __bfloat162float(win[0]);
+          else if (tile > 0) first = __bfloat162float(carry[(pn - 1) & 3][t8]);
+          mxv = fmaxf(mxv, first);
           const int bq = (tokh + t8 + cache_len) / kBlockN;
-          for (int blk = first_blk + st; blk < p.pooled_len; blk += kHalfThreads) {
-            float v = (4 * blk < lc) ? 0.f : -INFINITY;                   // keys 4blk .. 4blk+3
-            if (blk > 0 && 4 * blk - 1 < lc)                              // key 4blk - 1
-              v = fmaxf(v, (blk == first_blk && n_tiles > 0)
-                               ? __bfloat162float(carry[(n_tiles - 1) & 3][t8]) : 0.f);
-            if (blk < p.init_blocks || (bq >= blk && bq <= blk + p.local_blocks)) v = INFINITY;
-            pool_base[(int64_t)t8 * p.pooled_len + blk] = __float2bfloat16_rn(v);
+          if (blk < p.init_blocks || (bq >= blk && bq <= blk + p.local_blocks)) mxv = INFINITY;
+          if (t8 < ntokh && blk < p.pooled_len)
+            pool_base[(int64_t)t8 * p.pooled_len + blk] = __float2bfloat16_rn(mxv);
+        }
+        return true;
+      };
+
+      if (ok) {
+        for (int tile = 0; tile < n_tiles; ++tile, ++u) {
+          const uint32_t ab = u & 1;
+          ok = mbar_wait_warp(&acc_full[ab], (u >> 1) & 1, abort_flag, p.status, 62);
+          if (!ok) break;
+          tc_fence_after();
+          const int key = tile * kKeysPerTile + r;
+          float val[kTokPerThread];
+          uint32_t x[64];                                   // 4 tokens x 16 heads
+          tmem_ld64_wait(tmem + lane_off + ab * 128, x);
+          // the accumulator is in registers now: hand it back before the arithmetic
+          tc_fence_before();
+          mbar_arrive_warp(&acc_empty[ab]);
+          {
+            const uint64_t c2 = pack_f32x2(p.scale_log2, p.scale_log2);
+#pragma unroll
+            for (int j = 0; j < kTokPerThread; ++j) {
+              uint64_t a2[2] = {pack_f32x2(0.f, 0.f), pack_f32x2(0.f, 0.f)};
+#pragma unroll
+              for (int g = 0; g < 16; g += 2) {
+                float y0, y1;
+                unpack_f32x2(mul_f32x2(pack_f32x2(x[j * 16 + g], x[j * 16 + g + 1]), c2), y0, y1);
+                a2[(g >> 1) & 1] = add_f32x2(a2[(g >> 1) & 1], pack_f32x2(exp2_mixed(y0, g), exp2_mixed(y1, g + 1)));
+              }
+              float lo, hi;
+              unpack_f32x2(add_f32x2(a2[0], a2[1]), lo, hi);
+              val[j] = lo + hi;
+            }
+          }
+          if (kPooled && tile > 0) {
+            ok = pool_tile(tile - 1);
+            if (!ok) break;
+          }
+#pragma unroll
+          for (int j = 0; j < kTokPerThread; ++j) {
+            const int t8 = grp * kTokPerThread + j;
+            // existing but invisible keys score 0; keys past the sequence do not exist (-inf in the pool)
+            const __nv_bfloat16 vb = __float2bfloat16_rn((key < lim_tok[j]) ? val[j] : 0.f);
+            if (out_base != nullptr && t8 < ntokh && key < p.max_seqlen_k)
+              out_base[(int64_t)t8 * p.out_row_stride + key] = vb;
+            if (kPooled) {
+              const __nv_bfloat16 pv = (key < lc) ? vb : ninf_b;
+              pool[(pt + tile) % 3][t8][1 + r] = pv;
+              if (r == 127) carry[(pt + tile) & 3][t8] = pv;
+            }
+          }
+          // (after the deferred pooling reads: this arrival is what lets a later tile reuse them)
+          if (kPooled) mbar_arrive_warp(&pool_full[(pt + tile) % 3]);
+        }
+        if (ok && kPooled && n_tiles > 0) ok = pool_tile(n_tiles - 1);
+        // columns past the last tile are zero (rows are 16-byte aligned: stride % 8 == 0)
+        const int first = n_tiles * kKeysPerTile;
+        if (ok && out_base != nullptr && first < p.max_seqlen_k) {
+          const int vec_per_row = (p.max_seqlen_k - first + 7) / 8;   // may spill into row padding
+          const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+          for (int t8 = 0; t8 < ntokh; ++t8) {
+            uint4* dst = reinterpret_cast<uint4*>(out_base + (int64_t)t8 * p.out_row_stride + first);
+            for (int i = st; i < vec_per_row; i += kHalfThreads) dst[i] = z;
+          }
+        }
+        // block scores past the last tile: their keys are invisible (0) or do not exist (-inf);
+        // the first such block still sees the last key of the last tile
+        if (ok && kPooled) {
+          const int first_blk = n_tiles * 32;
+          for (int t8 = 0; t8 < ntokh; ++t8) {
+            const int bq = (tokh + t8 + cache_len) / kBlockN;
+            for (int blk = first_blk + st; blk < p.pooled_len; blk += kHalfThreads) {
+              float v = (4 * blk < lc) ? 0.f : -INFINITY;                   // keys 4blk .. 4blk+3
+              if (blk > 0 && 4 * blk - 1 < lc)                              // key 4blk - 1
+                v = fmaxf(v, (blk == first_blk && n_tiles > 0)
+                                 ? __bfloat162float(carry[(pt + n_tiles - 1) & 3][t8]) : 0.f);
+              if (blk < p.init_blocks || (bq >= blk && bq <= blk + p.local_blocks)) v = INFINITY;
+              pool_base[(int64_t)t8 * p.pooled_len + blk] = __float2bfloat16_rn(v);
+            }
           }
         }
       }
+      pt += (uint32_t)n_tiles;
+      // The tile's warps part by less than an item: its statistics, windows and carries are reused.  If one of
+      // them gave up on a wait, all of them leave here.
+      if (!kStay) break;
+      ok = !any_of_tile(hq, !ok);
     }
   }
 
@@ -583,6 +689,8 @@ int launch_stage1(const void* q, const void* kc, const void* kv, void* out, void
   p.block_table = block_table;
   p.bt_stride = block_table_stride;
   p.page_size = page_size > 0 ? page_size : 1;
+  p.batch = batch;
+  p.max_tiles = (max_seqlen_q + kTokPerCta - 1) / kTokPerCta;
   p.total_q = total_q;
   p.heads_q = heads_q;
   p.heads_k = heads_k;
@@ -598,21 +706,21 @@ int launch_stage1(const void* q, const void* kc, const void* kv, void* out, void
   p.status = status;
 
   const size_t smem = sizeof(Smem) + 1024;
-  dim3 grid((max_seqlen_q + kTokPerCta - 1) / kTokPerCta, batch, heads_k);
+  // CTAs that stay on their SM pay where a walk is short and lose on long ones (their loops are a few per cent
+  // slower, and the SMs' speeds differ more than a fixed deal allows).  One item a CTA / staying, us:  4096 tokens
+  // 45.9 / 42.5, 9001 + 4096 + 3283 208 / 169, 16384 + 8192 + 5001 + 2053 412 / 294, 32768 927 / 921;
+  // 4096 of 131072 2704 / 2880.  So the line is at the compressed keys of 32768 tokens.
+  const bool stay = max_seqlen_k <= 2048;
+  const int64_t items = (int64_t)p.max_tiles * batch * heads_k;        // at most
+  const dim3 grid = stay ? dim3((unsigned)(items < kNumSMs ? items : kNumSMs))
+                         : dim3((unsigned)p.max_tiles, (unsigned)batch, (unsigned)heads_k);
   rc = clear_launch_status(status, stream, what);
   if (rc) return rc;
-  cudaError_t e;
-  if (pooled != nullptr) {
-    e = cudaFuncSetAttribute(stage1_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    if (e != cudaSuccess) return set_error((int)e, "%s: %s", what, cudaGetErrorString(e));
-    stage1_kernel<true><<<grid, kThreads, smem, (cudaStream_t)stream>>>(map_q, map_kc, map_kv, p);
-  } else {
-    e = cudaFuncSetAttribute(stage1_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    if (e != cudaSuccess) return set_error((int)e, "%s: %s", what, cudaGetErrorString(e));
-    stage1_kernel<false><<<grid, kThreads, smem, (cudaStream_t)stream>>>(map_q, map_kc, map_kv, p);
-  }
+  const auto kernel = pooled != nullptr ? (stay ? stage1_kernel<true, true> : stage1_kernel<true, false>)
+                                        : (stay ? stage1_kernel<false, true> : stage1_kernel<false, false>);
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return set_error((int)e, "%s: %s", what, cudaGetErrorString(e));
+  kernel<<<grid, kThreads, smem, (cudaStream_t)stream>>>(map_q, map_kc, map_kv, p);
   return check_launch(what);
 }
 
