@@ -517,9 +517,10 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       };
 
       if (ok) {
-        for (int tile = 0; tile < n_tiles; ++tile, ++u) {
-          const uint32_t ab = u & 1;
-          ok = mbar_wait_warp(&acc_full[ab], (u >> 1) & 1, abort_flag, p.status, 62);
+        for (int t = n_tiles1; t < w.n_steps; ++t, u += kStay) {
+          const int tile = t - n_tiles1;
+          const uint32_t un = kStay ? u : (uint32_t)t, ab = un & 1;
+          ok = mbar_wait_warp(&acc_full[ab], (un >> 1) & 1, abort_flag, p.status, 62);
           if (!ok) break;
           tc_fence_after();
           const int key = tile * kKeysPerTile + r;
