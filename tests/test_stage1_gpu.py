@@ -213,3 +213,26 @@ def test_stage1_decode_path(lens_c, hk, causal):
                                              cu_c.to(DEV), 2, max_c, causal=False)
         diff = (got.float() - ref[:, :bsz].float()).abs()
         assert (diff <= torch.maximum(torch.tensor(2e-2, device=DEV), ref[:, :bsz].float().abs() * 2.0 ** -7)).all()
+
+
+@pytest.mark.parametrize("lens", [[40] * 130 + [1, 700, 15, 33, 2049], [9000]])
+def test_items_taken_in_turn_match_one_item_per_cta(lens):
+    # up to 2048 compressed keys CTAs stay and take several 16-token items (odd counts, items without a visible
+    # key, one-tile items between long ones); above, each CTA has one: the same scores and block scores, bit for bit
+    hk = 2
+    n = sum(lens)
+    q = det_tensor((n, hk * 16, 128), 21, 0.5).to(DEV)
+    k = det_tensor((n, hk, 128), 22, 0.5).to(DEV)
+    cu_q = cu(lens, DEV)
+    kc, cu_c = infllm_v2.compress_keys(k, cu_q)
+    most = int((cu_c[1:] - cu_c[:-1]).max())
+    a = infllm_v2.infllmv2_attn_stage1(q, kc, kc, cu_q, cu_c, cu_c, max(lens), max(most, 1), causal=True)
+    b = infllm_v2.infllmv2_attn_stage1(q, kc, kc, cu_q, cu_c, cu_c, max(lens), 2049, causal=True)
+    infllm_v2.check_device_status()
+    assert torch.equal(a[..., :most], b[..., :most]) and not b[..., most:].any()
+    blocks = (max(lens) + 63) // 64
+    pa = infllm_v2.infllmv2_stage1_block_scores(q, kc, cu_q, cu_c, max(lens), max(most, 1), 1, 1, causal=True)
+    pb = infllm_v2.infllmv2_stage1_block_scores(q, kc, cu_q, cu_c, max(lens), 2049, 1, 1, causal=True)
+    infllm_v2.check_device_status()
+    shared = min(pa.shape[-1], pb.shape[-1], blocks)
+    assert torch.equal(pa[..., :shared], pb[..., :shared])
