@@ -161,8 +161,12 @@ struct Item {
     }
     st1 = (lcv == lc) ? 16 : 64;
     // (limits grow with the token)
-    n_tiles1 = (visible_limit(tok0 + ntok - 1, lq, lcv, p.causal, st1) + kKeysPerTile - 1) / kKeysPerTile;
-    n_steps = n_tiles1 + (visible_limit(tok0 + ntok - 1, lq, lc, p.causal) + kKeysPerTile - 1) / kKeysPerTile;
+    const int n_tiles = (visible_limit(tok0 + ntok - 1, lq, lc, p.causal) + kKeysPerTile - 1) / kKeysPerTile;
+    // Without a scored key nobody reads the row sums: no steps at all.  (So an item with steps has a pass 2, and
+    // its MMA threads wait for the row constants exactly as often as its softmax warps announce them.)
+    n_tiles1 = n_tiles == 0 ? 0
+               : (visible_limit(tok0 + ntok - 1, lq, lcv, p.causal, st1) + kKeysPerTile - 1) / kKeysPerTile;
+    n_steps = n_tiles1 + n_tiles;
   }
 };
 

@@ -236,3 +236,91 @@ def test_items_taken_in_turn_match_one_item_per_cta(lens):
     infllm_v2.check_device_status()
     shared = min(pa.shape[-1], pb.shape[-1], blocks)
     assert torch.equal(pa[..., :shared], pb[..., :shared])
+
+
+def _many_items(layout, causal, hk=2, seed=3):
+    """About 400 short sequences (more than 1000 items of 16 tokens and a KV head for 148 CTAs), some without scored
+    or without row-sum keys, in the given layout: q, cu_q, keys, their arguments and the packed keys for the oracle."""
+    rng = np.random.default_rng(seed)
+    n = 400
+    lens_q = rng.choice([1, 15, 16, 17, 33, 40, 100], n)
+    lens_c = rng.choice([0, 0, 1, 5, 128, 129, 300], n)
+    lens_v = rng.choice([0, 1, 7, 128, 129, 200], n) if layout.startswith("coarse") else lens_c
+    q = det_tensor((int(lens_q.sum()), hk * 16, 128), seed, 0.5)
+    kc = det_tensor((int(lens_c.sum()), hk, 128), seed + 1, 0.5)
+    kv = det_tensor((int(lens_v.sum()), hk, 128), seed + 2, 0.5)
+    kw = {}
+    if layout == "paged":
+        table = torch.zeros(n, 3, dtype=torch.int32)
+        pages = det_tensor((int((-(-lens_c // 128)).sum()) + 1, 128, hk, 128), seed + 3, 3.0)   # unused rows: large keys
+        free, at = list(rng.permutation(pages.shape[0])), 0
+        for b, l in enumerate(lens_c):
+            for j in range(-(-int(l) // 128)):
+                table[b, j] = int(free.pop())
+                m = min(128, int(l) - 128 * j)
+                pages[table[b, j], :m] = kc[at:at + m]
+                at += m
+        k, kw["block_table"] = pages, table.to(DEV)
+        cu_k = cu(lens_c)
+    elif layout == "leftpad" or layout.startswith("coarse_used"):
+        # extents longer than what is in use: five rows in front, or seven (in some sequences all rows) behind
+        front, behind = (5, 0) if layout == "leftpad" else (0, 7)
+        parts, at = [], 0
+        for b, l in enumerate(lens_c):
+            junk = det_tensor((front + behind, hk, 128), seed + 4, 3.0)
+            parts += [junk[:front], kc[at:at + int(l)], junk[front:]]
+            at += int(l)
+        k, cu_k = torch.cat(parts), cu(lens_c + front + behind)
+        if front:
+            kw["leftpad_k"] = torch.full((n,), front, dtype=torch.int32, device=DEV)
+        else:
+            kw["seqused_k"] = torch.tensor(lens_c, dtype=torch.int32, device=DEV)
+    else:
+        k, cu_k = kc, cu(lens_c)
+    vd, cu_v = None, cu_k
+    if layout.startswith("coarse"):
+        vd, cu_v = kv.to(DEV), cu(lens_v)
+        if layout == "coarse_used_both":
+            used = np.maximum(lens_v - 3, 0)                      # (the oracle gets these rows only)
+            kw["seqused_v"] = torch.tensor(used, dtype=torch.int32, device=DEV)
+            o = np.concatenate([[0], np.cumsum(lens_v)])
+            kv = torch.cat([kv[o[b]:o[b] + int(u)] for b, u in enumerate(used)])
+            lens_v = used
+    k = k.to(DEV)
+    args = dict(q=q.to(DEV), k=k, v=vd if vd is not None else k, cu_q=cu(lens_q, DEV), cu_k=cu_k.to(DEV),
+                cu_v=cu_v.to(DEV), max_q=int(lens_q.max()), kw=kw)
+    return args, oracle.stage1_scores(q, kc, cu(lens_q).tolist(), cu(lens_c).tolist(), 300, causal,
+                                      lse_keys=kv if vd is not None else None, cu_seqlens_v=cu(lens_v).tolist())
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("layout", ["packed", "coarse", "coarse_used", "coarse_used_both", "paged", "leftpad"])
+def test_items_taken_in_turn_in_every_key_layout(layout, causal):
+    # passes of different lengths, and one or both of them empty, between each other on one CTA: an item that sees
+    # row-sum keys but no scored key must not shift the row constants of the next one
+    a, ref = _many_items(layout, causal)
+    coarse = layout.startswith("coarse")
+
+    def scores(max_k):
+        return infllm_v2.infllmv2_attn_stage1(a["q"], a["k"], a["v"], a["cu_q"], a["cu_k"], a["cu_v"], a["max_q"], max_k,
+                                              causal=causal, **a["kw"])
+
+    def blocks(max_k):
+        extra = dict(lse_keys=a["v"], cu_seqlens_v=a["cu_v"]) if coarse else {}
+        return infllm_v2.infllmv2_stage1_block_scores(a["q"], a["k"], a["cu_q"], a["cu_k"], a["max_q"], max_k, 0, 0,
+                                                      max_cache_len=0, cache_len=1100, causal=causal, **extra, **a["kw"])
+    for _ in range(3):
+        got = scores(300)
+        infllm_v2.check_device_status()
+        ok, err = _within(got.float().cpu(), ref)
+        assert ok, err
+    if layout != "paged":                      # (its three pages a sequence cover 384 keys)
+        assert torch.equal(got, scores(2049)[..., :300])          # one item a CTA
+        assert torch.equal(blocks(300), blocks(2049))
+    if layout in ("packed", "coarse"):
+        lens = torch.full((a["cu_q"].numel() - 1,), 1100, dtype=torch.int32, device=DEV)
+        pooled = infllm_v2.max_pooling_1d_varlen(got, a["cu_q"], a["cu_k"], lens, a["max_q"], 300, 0, 0)
+        mine = blocks(300)
+        shared = min(pooled.shape[-1], mine.shape[-1])
+        assert shared > 10 and torch.equal(mine[..., :shared], pooled[..., :shared])
+    infllm_v2.check_device_status()
