@@ -295,19 +295,22 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   if (warp == 0) {
     // ================================================================ TMA producer
     if (lane == 0) {
-      int u = n_ahead, it = kStay ? 0 : 1;
+      int u = n_ahead, nq[2];                      // key tiles, and copies of each Q tile, issued so far
+      nq[0] = nq[1] = n_ahead > 0 ? 1 : 0;
       bool ok = true;
       while (ok && (!kStay || walk.next(p, h, tile16))) {
         const Item w = kStay ? Item(p, walk.b, h, tile16) : own;
         for (int t = n_ahead; t < w.n_steps && ok; ++t) {
           // (two key tiles go ahead of Q: their ring slots are free before the last products of the item before)
           if (kStay && t == min(2, w.n_steps - 1)) {
-            for (int tile = 0; tile < 2 && ok; ++tile) {
-              if (it > 0) ok = mbar_wait(&sm.q_free[tile], (uint32_t)((it - 1) & 1), abort_flag, p.status, 42);
-              if (ok) fetch_q(w, tile);
+#pragma unroll
+            for (int tile = 0; tile < 2; ++tile) {
+              if (nq[tile] > 0) ok = ok && mbar_wait(&sm.q_free[tile], (uint32_t)((nq[tile] - 1) & 1), abort_flag, p.status, 42);
+              if (!ok) break;
+              fetch_q(w, tile);
+              ++nq[tile];
             }
             if (!ok) break;
-            ++it;
           }
           const int s = u % kStages;
           if (u >= kStages) ok = mbar_wait(&sm.kc_free[s], (uint32_t)((u / kStages - 1) & 1), abort_flag, p.status, 41);
@@ -318,7 +321,10 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         if (!kStay) break;
       }
       if (*abort_flag) {
-        for (int tile = 0; tile < 2 && it > 0 && u > 0; ++tile) mbar_wait_drain(&sm.q_full[tile], (uint32_t)((it - 1) & 1));
+        // (the tiles count apart: tile 0 of an item may be on its way when the wait for tile 1's place gives up)
+#pragma unroll
+        for (int tile = 0; tile < 2; ++tile)
+          if (nq[tile] > 0) mbar_wait_drain(&sm.q_full[tile], (uint32_t)((nq[tile] - 1) & 1));
         for (int j = max(0, u - kStages); j < u; ++j)
           mbar_wait_drain(&sm.kc_full[j % kStages], (uint32_t)((j / kStages) & 1));
       }
