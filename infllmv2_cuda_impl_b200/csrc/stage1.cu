@@ -1,8 +1,8 @@
 // Stage-1 scorer: group-summed softmax probabilities of the queries against the compressed keys,
 // optionally max-pooled to 64-token block scores in the same kernel.
 //
-// One CTA (one per SM) owns 16 consecutive tokens x the 16 query heads of one KV head: two 128-row
-// query tiles A and B, each fetched by 3-D TMA boxes from the caller's (token, head, d) layout, and
+// A CTA (one per SM) works on items of 16 consecutive tokens x the 16 query heads of one KV head, one item or, where
+// the sequences are short, one after the other: two 128-row query tiles A and B, each fetched by 3-D TMA boxes from the caller's (token, head, d) layout, and
 // streams 128-key tiles of the compressed keys twice through a 4-slot ring.  Every key tile serves
 // both query tiles, which halves the L2 -> SM key traffic per score against an 8-token CTA:
 //   pass 1:  S = Q_t . Kc^T  (rows = query rows of tile t in TMEM lanes) -> reference point m
@@ -81,6 +81,7 @@ struct Stage1Params {
   const int32_t* block_table;     // (batch, bt_stride) page of every page_size scored keys, or null
   int bt_stride, page_size;
   int batch, max_tiles;           // sequences, and the most 16-token tiles of one
+  int n_items, numbering;         // staying form: numbered tiles x KV heads (at most), and how they are numbered
   int64_t total_q;
   int heads_q, heads_k;
   int max_seqlen_k;
@@ -123,14 +124,19 @@ __device__ __forceinline__ float bf16_round(float x) {
   return __bfloat162float(__float2bfloat16_rn(x));
 }
 
-// Barrier of the 256 softmax threads of query tile hq that tells all of them whether one said yes.
-__device__ __forceinline__ bool any_of_tile(int hq, bool yes) {
+// Barrier of the 256 softmax threads of query tile hq that tells all of them whether one said yes.  (Barrier numbers
+// as constants: from a register ptxas has to take all 16 barriers, and spilled more.)
+template <int kBar>
+__device__ __forceinline__ bool any_of_256(bool yes) {
   uint32_t any;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.red.or.pred q, %2, 256, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}"
-      : "=r"(any) : "r"((uint32_t)yes), "r"(hq + 1) : "memory");
+      : "=r"(any) : "r"((uint32_t)yes), "n"(kBar) : "memory");
   return any != 0;
+}
+__device__ __forceinline__ bool any_of_tile(int hq, bool yes) {
+  return hq == 0 ? any_of_256<1>(yes) : any_of_256<2>(yes);
 }
 
 // One work item: 16 tokens of a sequence and one KV head.
@@ -171,15 +177,25 @@ struct Item {
 };
 
 // The items of a CTA, in the order in which every role of it takes them.  Without kStay: the one of its grid
-// position.  With kStay all items are numbered sequence by sequence, long tiles first, KV heads side by side,
-// and dealt out to the CTAs in rounds of gridDim.x, every other round backwards (forwards only, CTA 0 would get
-// the longest tile of every round).
+// position.  With kStay the tiles of all sequences are numbered through, each sequence's last tile first (the longest
+// walk of keys), and the KV heads of a number lie side by side; the items are dealt out to the CTAs in rounds of
+// gridDim.x, every other round backwards (forwards only, CTA 0 would get the longest tile of every round).
+enum Numbering {
+  kEven,      // max_tiles numbers a sequence: fewest where the lengths are even
+  kAddUp,     // a sequence's tiles follow those of the one before; adding them up takes ~230 clocks a sequence in
+              // every role, which is nothing where an item is seldom more than a few sequences on
+  kSearch     // sequence b's numbers start at cu_q[b] / 16 + b (at most one of them has no tile): a binary search
+};            // finds it (4000 sequences of 3 tokens and one of 8000: 290 us, adding up 546)
 template <bool kStay>
 struct ItemWalk {
-  int b, count, base, round;                   // sequence, its number of items, number of its first item (an item
-                                               // has at least one query row: 32 bits)
-  __device__ ItemWalk() : b(-1), count(0), base(0), round(0) {}
-  // the next item's sequence is b; its head and tile come back; false when there are no more
+  int b, round;                                  // (all that lives on between items: the softmax warps have no register left)
+  __device__ ItemWalk() : b(-1), round(0) {}
+  // item of this CTA in a round
+  __device__ static int number(int r) {
+    return r * (int)gridDim.x + ((r & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+  }
+  // the next item's sequence is b; its head and tile come back (tile: still that of the item before on entry); false
+  // when there are no more
   __device__ bool next(const Stage1Params& p, int& h, int& tile) {
     if (!kStay) {
       if (b >= 0) return false;
@@ -188,25 +204,49 @@ struct ItemWalk {
       tile = p.max_tiles - 1 - (int)blockIdx.x;
       return true;
     }
-    const int at = (round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
-    const int w = round * (int)gridDim.x + at;
-    ++round;
-    while (b < 0 || w >= base + count) {
-      base += count;
-      if (++b >= p.batch) return false;
-      count = min((__ldg(p.cu_q + b + 1) - __ldg(p.cu_q + b) + kTokPerCta - 1) / kTokPerCta, p.max_tiles) * p.heads_k;
+    for (;; ++round) {
+      const int w = number(round);
+      if (w >= p.n_items) return false;          // (later rounds lie behind it)
+      const int s = w / p.heads_k;
+      h = w - s * p.heads_k;
+      if (p.numbering == kAddUp) {
+        int last = b < 0 ? 0 : tile + 1 + number(round - 1) / p.heads_k;       // first number behind sequence b
+        while (s >= last) {
+          if (++b >= p.batch) return false;
+          last += min((__ldg(p.cu_q + b + 1) - __ldg(p.cu_q + b) + kTokPerCta - 1) / kTokPerCta, p.max_tiles);
+        }
+        tile = last - 1 - s;
+        break;
+      }
+      int end;
+      if (p.numbering == kEven) {
+        b = s / p.max_tiles;
+        end = __ldg(p.cu_q + b + 1);
+        tile = p.max_tiles - 1 - (s - b * p.max_tiles);
+      } else {
+        int hi = p.batch;
+        b = 0;
+        while (hi - b > 1) {
+          const int mid = (b + hi) >> 1;
+          if (__ldg(p.cu_q + mid) / kTokPerCta + mid <= s) b = mid; else hi = mid;
+        }
+        end = __ldg(p.cu_q + b + 1);
+        tile = end / kTokPerCta + b - s;
+      }
+      // (below 0: rows of q past the last sequence)
+      if (tile >= 0 && tile < p.max_tiles && tile * kTokPerCta < end - __ldg(p.cu_q + b)) break;
     }
-    const int i = w - base;
-    h = i % p.heads_k;
-    tile = count / p.heads_k - 1 - i / p.heads_k;
+    ++round;
     return true;
   }
 };
 
 // kStay: one CTA per SM takes items until there are none, and every barrier, ring slot and accumulator buffer
 // runs on across them, so that an item's keys and Q arrive, and its first products run, while the softmax warps
-// finish the item before.  (u: steps since the start of the kernel, it: items with steps.)  What a CTA does
-// besides its steps (start, first tiles, change of pass, end) is ~10 us, as much as 7 steps.
+// finish the item before.  (u: steps since the start of the kernel, it: items with steps.)  Against one CTA an item
+// that saves 1-3 us an item (block scores, 2 KV heads: 16 x 2048 tokens, 28 items per SM, 256 -> 197 us; 4 x 8192, 28
+// items, 414 -> 358; 16384, 14 items, 301 -> 264; 4096, 3.5 items, 53 -> 49), and in ragged batches 0.8 us of an SM
+// for every CTA of the other grid that finds no tile (4000 x 3 and 8000 tokens, 27000 per SM: 22.4 ms -> 285 us).
 template <bool kPooled, bool kStay>
 __global__ void __launch_bounds__(kThreads, 1)      // 19 warps: at most 96 registers per thread
 stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kc,
@@ -218,7 +258,7 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   // (read beside the sequence tables: one trip to memory in front of a CTA instead of two)
   const int32_t failed = *reinterpret_cast<volatile int32_t*>(p.status);
   ItemWalk<kStay> walk;
-  int h, tile16;
+  int h, tile16 = 0;
   if (!kStay) {
     walk.next(p, h, tile16);
     if (tile16 * kTokPerCta >= p.cu_q[walk.b + 1] - p.cu_q[walk.b]) return;
@@ -717,13 +757,19 @@ int launch_stage1(const void* q, const void* kc, const void* kv, void* out, void
   p.status = status;
 
   const size_t smem = sizeof(Smem) + 1024;
-  // CTAs that stay on their SM pay where a walk is short and lose on long ones (their loops are a few per cent
-  // slower, and the SMs' speeds differ more than a fixed deal allows).  One item a CTA / staying, us:  4096 tokens
-  // 45.9 / 42.5, 9001 + 4096 + 3283 208 / 169, 16384 + 8192 + 5001 + 2053 412 / 294, 32768 927 / 921;
-  // 4096 of 131072 2704 / 2880.  So the line is at the compressed keys of 32768 tokens.
-  const bool stay = max_seqlen_k <= 2048;
-  const int64_t items = (int64_t)p.max_tiles * batch * heads_k;        // at most
-  const dim3 grid = stay ? dim3((unsigned)(items < kNumSMs ? items : kNumSMs))
+  // CTAs that stay on their SM pay where a walk is short and lose on long ones: their loops spill two to five registers,
+  // and the SMs' speeds differ more than a fixed deal allows.  Block scores with 2 KV heads, one item a CTA / staying,
+  // us:  4096 tokens 53 / 49, 9001 + 4096 + 3283 213 / 174, 16384 + 8192 + 5001 + 2053 502 / 422, 32768 (2047 keys)
+  // 911 / 862, 49152 1841 / 1800, 65536 3096 / 3077, 98304 6577 / 6608, 131072 11330 / 11470;  4096 tokens against 1024 keys
+  // 125 / 123, 2048 217 / 219, 4096 401 / 410, 8192 758 / 776.  The line is where both kinds of call meet.  Nothing can
+  // overlap where no CTA would get a second item (300 tokens 16.3 / 18.3, 1000 18.3 / 20.3) or no item has a step
+  // (without keys; 2000 x 16 tokens 129 / 139).
+  const int64_t even = (int64_t)p.max_tiles * batch, found = total_q / kTokPerCta + batch;
+  const int64_t n_items = (even <= found ? even : found) * heads_k;
+  p.numbering = even <= found ? kEven : 4 * n_items >= (int64_t)batch * kNumSMs ? kAddUp : kSearch;
+  const bool stay = max_seqlen_k > 0 && max_seqlen_k <= 2048 && even * heads_k > kNumSMs && n_items < (1 << 30);
+  p.n_items = (int)n_items;
+  const dim3 grid = stay ? dim3((unsigned)(n_items < kNumSMs ? n_items : kNumSMs))
                          : dim3((unsigned)p.max_tiles, (unsigned)batch, (unsigned)heads_k);
   rc = clear_launch_status(status, stream, what);
   if (rc) return rc;

@@ -324,3 +324,18 @@ def test_items_taken_in_turn_in_every_key_layout(layout, causal):
         shared = min(pooled.shape[-1], mine.shape[-1])
         assert shared > 10 and torch.equal(mine[..., :shared], pooled[..., :shared])
     infllm_v2.check_device_status()
+
+
+@pytest.mark.parametrize("lens", [[16] * 600, [0, 5] * 400 + [1, 0, 0],                       # so many numbers a sequence
+                                  [3000, 0, 17, 1400, 0], [2399, 15], [0, 2385],             # added up
+                                  [0] * 90 + [300] + [0] * 300 + [1, 33] * 90])               # searched for
+def test_numbering_of_the_items(lens):
+    # the three ways in which a staying CTA finds its items, with empty sequences between and at both ends: bit for bit
+    # what one item a CTA gives; rows of q past the last sequence belong to nobody
+    hk, n = 2, sum(lens)
+    q = det_tensor((n + 21, hk * 16, 128), 31, 0.5).to(DEV)
+    kc = det_tensor((3 * len(lens), hk, 128), 32, 0.5).to(DEV)
+    cu_q, cu_k = cu(lens, DEV), cu([3] * len(lens), DEV)
+    a, b = (infllm_v2.infllmv2_attn_stage1(q, kc, kc, cu_q, cu_k, cu_k, max(lens), m, causal=False) for m in (3, 2049))
+    infllm_v2.check_device_status()
+    assert torch.equal(a[:, :n], b[:, :n, :3]) and (a[:, :n].float().sum(-1) - 16).abs().max() < 0.25
