@@ -349,7 +349,8 @@ int64_t ifv2_sparse_attn_bwd_workspace_bytes(int64_t total_q, int heads_q, int h
  * (heads_k, ceil(max_seqlen_k/64), bwd_mask_words = ceil(total_q/64)) from
  * ifv2_transpose_blockmask.  workspace: caller-allocated, 16-byte aligned scratch of at least
  * ifv2_sparse_attn_bwd_workspace_bytes bytes (contents on entry are ignored).  Deterministic:
- * no atomics are used.
+ * no atomics are used, and the gradients of a sequence and KV head are the same bits whatever else
+ * the call holds (other sequences, other heads, a loose max_seqlen_q).
  * Replaces C.varlen_bwd: csrc/entry.cu:209-214 -> mha_varlen_bwd,
  * csrc/flash_attn/flash_api.cpp:1278-1547 (+ the transposes, the Python loop and the
  * synchronisations of infllm_v2/infllmv2_sparse_attention.py:174-263, 343-350). */

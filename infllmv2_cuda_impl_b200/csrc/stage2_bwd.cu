@@ -474,8 +474,7 @@ struct DkvSmem {
 };
 
 // Walk over the token octets [8m, 8m+8) of a sequence in which at least one token selected the
-// key block (bits of the transposed mask row, indexed by GLOBAL token), lowest octet first; of these the
-// CTA takes the octets with m % split == rank (split: 1, 2 or 4).
+// key block (bits of the transposed mask row, indexed by GLOBAL token), lowest octet first.
 // A whole warp walks together: lane l caches words wbase + l and wbase + 32 + l of the row, so a
 // step costs shuffles instead of a round trip to global memory, runs of empty words are skipped
 // with one ballot, and the next 32 words are fetched while the cached ones are in use.
@@ -484,12 +483,12 @@ struct OctetWalk {
   const unsigned long long* row;   // null = dense
   int64_t words, wbase;
   unsigned long long cur, nxt;
-  int q0, lq, m, m_end, lane, rank, split;
+  int q0, lq, m, m_end, lane;
   __device__ unsigned long long fetch(int64_t w) const {
     return (row != nullptr && w < words) ? __ldg(row + w) : 0ull;
   }
-  __device__ OctetWalk(const unsigned long long* r, int64_t w, int q0_, int lq_, int m_lo, int lane_, int rank_, int split_)
-      : row(r), words(w), q0(q0_), lq(lq_), m(m_lo), m_end((lq_ + 7) / 8), lane(lane_), rank(rank_), split(split_) {
+  __device__ OctetWalk(const unsigned long long* r, int64_t w, int q0_, int lq_, int m_lo, int lane_)
+      : row(r), words(w), q0(q0_), lq(lq_), m(m_lo), m_end((lq_ + 7) / 8), lane(lane_) {
     wbase = ((int64_t)q0 + 8 * (int64_t)m_lo) >> 6;
     cur = fetch(wbase + lane);
     nxt = fetch(wbase + 32 + lane);
@@ -507,9 +506,7 @@ struct OctetWalk {
       const uint32_t vmask = (1u << ntok) - 1u;
       if (row == nullptr) {
         bits = vmask;
-        const int at = m++;
-        if ((at & (split - 1)) != rank) continue;
-        return at;
+        return m++;
       }
       const int64_t t = (int64_t)q0 + 8 * (int64_t)m;
       const int64_t w = t >> 6;
@@ -523,11 +520,7 @@ struct OctetWalk {
       unsigned long long lo = here;
       if (sh > 56) lo |= word(w + 1) << (64 - sh);
       bits = (uint32_t)lo & vmask;
-      if (bits) {
-        const int at = m++;
-        if ((at & (split - 1)) != rank) continue;
-        return at;
-      }
+      if (bits) return m++;
       if (here != 0ull) {          // later tokens of this word selected the block
         ++m;
         continue;
@@ -558,24 +551,21 @@ struct OctetWalk {
 // dV and dK: each waits, issues and commits on its own, so neither one's barrier round trips hold
 // up the other's instructions, and the S / dP warp runs up to two steps ahead (two TMEM buffers).
 // Q has three ring slots and dO two.
-// `split` CTAs of a cluster take every split-th octet of the block each and add their fp32 sums up through
-// distributed shared memory at the end (rank r stores its part of dV^T | dK^T): block 0 is selected by every
-// token, and as one CTA's serial walk it was as long as the whole grid in small batches.
 __global__ void __launch_bounds__(kDkvThreads, 1)
 sparse_attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q,
                            const __grid_constant__ CUtensorMap map_do,
                            const __grid_constant__ CUtensorMap map_k,
-                           const __grid_constant__ CUtensorMap map_v, const BwdParams p, const int split) {
+                           const __grid_constant__ CUtensorMap map_v, const BwdParams p) {
   extern __shared__ uint8_t smem_raw[];
   DkvSmem& sm = *reinterpret_cast<DkvSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                             ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // block index slowest: the blocks every token selects (block 0 of each sequence) start first
-  const int rank = (int)(blockIdx.x & (unsigned)(split - 1)), b = (int)(blockIdx.x / (unsigned)split);
-  const int h = blockIdx.y, n = blockIdx.z;
+  const int b = blockIdx.x, h = blockIdx.y, n = blockIdx.z;
   const int q0 = p.cu_q[b], lq = p.cu_q[b + 1] - q0;
   const int k0 = p.cu_k[b], lk = p.cu_k[b + 1] - k0;
-  if (n * kBlockN >= lk) return;                     // (the whole cluster)
+  if (n * kBlockN >= lk) return;
+  if (*reinterpret_cast<volatile int32_t*>(p.status) != 0) return;
   const int shift = lk - lq;
   const int nkeys = min(kBlockN, lk - n * kBlockN);
   // first token that can see key 64n (causal), as an octet index
@@ -583,10 +573,7 @@ sparse_attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q,
   const unsigned long long* mask_row =
       (p.bwd_mask != nullptr && n < p.k_blocks)
           ? p.bwd_mask + ((int64_t)h * p.k_blocks + n) * p.bwd_words : nullptr;
-  // An earlier CTA gave up on a wait: nothing to do either, but no early return, the others of the cluster
-  // write into this CTA's shared memory at the end.
-  const int failed = __syncthreads_or(*reinterpret_cast<volatile int32_t*>(p.status) != 0);
-  const bool never_selected = (p.bwd_mask != nullptr && n >= p.k_blocks) || failed;
+  const bool never_selected = (p.bwd_mask != nullptr && n >= p.k_blocks);
 
   if (threadIdx.x == 0) {
     sm.abort_flag = 0;
@@ -620,8 +607,6 @@ sparse_attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q,
   volatile int* total_steps = &sm.total_steps;
 
   // Step i uses Q slot i % 3, dO slot i & 1, TMEM buffer i & 1.
-  bool ok = true;                                    // (of the softmax warps, with the count of steps)
-  int steps = 0;
   if (warp == 0) {
     // the whole warp walks the octet list; lane 0 waits for ring slots and issues the copies
     if (!never_selected) {
@@ -632,7 +617,7 @@ sparse_attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q,
         tma_load_3d(sm.v[0], &map_v, &sm.kv_full, 0, h, k0 + n * kBlockN);
         tma_load_3d(sm.v[1], &map_v, &sm.kv_full, 64, h, k0 + n * kBlockN);
       }
-      OctetWalk walk(mask_row, p.bwd_words, q0, lq, m_lo, lane, rank, split);
+      OctetWalk walk(mask_row, p.bwd_words, q0, lq, m_lo, lane);
       uint32_t bits;
       int issued_q = 0, issued_do = 0;
       int qs = 0, qround = 0;                      // i % 3, i / 3
@@ -763,6 +748,8 @@ sparse_attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q,
     const int r = quad * 32 + lane;
     const int tl = r >> 4, g = r & 15;
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
+    bool ok = true;
+    int steps = 0;
     // row r of a 128-byte-swizzled tile: 16-byte chunk c sits at chunk (c ^ (r & 7))
     uint8_t* prow = sm.pmat + r * 128;
     uint8_t* drow = sm.dsmat + r * 128;
@@ -848,72 +835,37 @@ sparse_attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap map_q,
         }
       }
     }
-    // (every warp of both turns: the exchange below writes over the Q and dO tiles)
-    if (ok && steps > 0)
+    // the warps of the first turn write the block's gradients
+    if (turn != 0) ok = false;
+    if (ok && steps > 0) {
       ok = __all_sync(0xFFFFFFFFu, mbar_wait(&sm.dk_done[(steps - 1) % 3],
                                              (uint32_t)(((steps - 1) / 3) & 1), abort_flag, p.status, 88));
-  }
-
-  // ---- The warps of the first turn write the block's gradients: of dV^T | dK^T (128 features x 128 columns)
-  // rank r has columns [r * 128 / split, ...), summed over the cluster.  The other ranks' fp32 values come
-  // through the Q and dO rings (160 KB, idle once every CTA is past its walk).
-  const int quad = warp & 3, grp = (warp - 4) >> 2, d = quad * 32 + lane;      // (of the writing warps)
-  const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
-  const int ncols = 128 / split, per_warp = ncols / 2;
-  const bool writer = warp >= 4 && warp < 12 && ok;
-  if (split > 1) {
-    tc_fence_before();
-    cluster_sync();
-    tc_fence_after();
-    if (writer) {
-      for (int to = 0; to < split; ++to) {
-        if (to == rank) continue;
-        const int slot = rank < to ? rank : rank - 1;
-        for (int c = 0; c < per_warp; c += 8) {
-          uint32_t o[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-          if (steps > 0) {
-            tmem_ld8(tmem_dv + lane_off + to * ncols + grp * per_warp + c, o);
-            tmem_wait_ld();
+      tc_fence_after();
+    }
+    if (ok) {
+      // this thread owns feature d = r of dV^T / dK^T; 64 key columns each
+      const int d = r;
+      __nv_bfloat16* dv_base = p.dv + ((int64_t)(k0 + n * kBlockN) * p.heads_k + h) * kHeadDim + d;
+      __nv_bfloat16* dk_base = p.dk + ((int64_t)(k0 + n * kBlockN) * p.heads_k + h) * kHeadDim + d;
+      const int64_t key_stride = (int64_t)p.heads_k * kHeadDim;
+      {
+        const int c0 = grp * 32;
+        uint32_t a[32], bb[32];
+        if (steps > 0) {
+          tmem_ld32x2_wait(tmem_dv + lane_off + c0, a, tmem_dk + lane_off + c0, bb);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) { a[j] = 0u; bb[j] = 0u; }
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          if (c0 + j < nkeys) {
+            dv_base[(int64_t)(c0 + j) * key_stride] = __float2bfloat16_rn(__uint_as_float(a[j]));
+            dk_base[(int64_t)(c0 + j) * key_stride] =
+                __float2bfloat16_rn(__uint_as_float(bb[j]) * p.scale);
           }
-          // [source][group of four columns][feature]: a warp writes 512 contiguous bytes
-          const uint32_t at = smem_u32(sm.q[0][0]) + (uint32_t)((slot * (ncols / 4) + (grp * per_warp + c) / 4) * 128 + d) * 16u;
-          st_cluster_v4(at, (uint32_t)to, o[0], o[1], o[2], o[3]);
-          st_cluster_v4(at + 128 * 16, (uint32_t)to, o[4], o[5], o[6], o[7]);
         }
       }
-    }
-    cluster_sync();
-  } else {
-    tc_fence_after();
-  }
-  if (writer) {
-    const int64_t key_stride = (int64_t)p.heads_k * kHeadDim;
-    const int64_t base = ((int64_t)(k0 + n * kBlockN) * p.heads_k + h) * kHeadDim + d;
-    for (int c = 0; c < per_warp; c += 8) {
-      const int col = rank * ncols + grp * per_warp + c;             // of dV^T | dK^T
-      uint32_t o[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-      if (steps > 0) {
-        tmem_ld8(tmem_dv + lane_off + col, o);
-        tmem_wait_ld();
-      }
-      for (int from = 0; from < split - 1; ++from) {
-        const float4* part = reinterpret_cast<const float4*>(sm.q[0][0]) + (from * (ncols / 4) + (grp * per_warp + c) / 4) * 128 + d;
-        const float4 lo = part[0], hi = part[128];
-        o[0] = __float_as_uint(__uint_as_float(o[0]) + lo.x);
-        o[1] = __float_as_uint(__uint_as_float(o[1]) + lo.y);
-        o[2] = __float_as_uint(__uint_as_float(o[2]) + lo.z);
-        o[3] = __float_as_uint(__uint_as_float(o[3]) + lo.w);
-        o[4] = __float_as_uint(__uint_as_float(o[4]) + hi.x);
-        o[5] = __float_as_uint(__uint_as_float(o[5]) + hi.y);
-        o[6] = __float_as_uint(__uint_as_float(o[6]) + hi.z);
-        o[7] = __float_as_uint(__uint_as_float(o[7]) + hi.w);
-      }
-      const float f = col < kBlockN ? 1.f : p.scale;
-      __nv_bfloat16* dst = (col < kBlockN ? p.dv : p.dk) + base;
-      const int key = col & (kBlockN - 1);
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (key + j < nkeys) dst[(int64_t)(key + j) * key_stride] = __float2bfloat16_rn(__uint_as_float(o[j]) * f);
     }
   }
   tc_fence_before();
@@ -1040,32 +992,8 @@ extern "C" int ifv2_sparse_attn_bwd(const void* dout, const void* q, const void*
     cudaError_t e = cudaFuncSetAttribute(sparse_attn_bwd_dkv_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return set_error((int)e, "sparse_attn_bwd: %s", cudaGetErrorString(e));
-    // Every token selects block 0 of its sequence (and with dense attention the first blocks are everybody's):
-    // as one CTA's walk that is max_seqlen_q / 8 steps, against the steps per SM if all work were spread evenly
-    // (64 blocks an octet or, in shorter sequences, half of the blocks).  Where the longest walk would be more
-    // than half of that, clusters of 2 or 4 CTAs share a block's octets and exchange their sums.  Measured with
-    // 1 / 2 / 4 CTAs (us), and the ratio per_sm / max_seqlen_q:  one sequence of 500 tokens, 2 KV heads 73 / 44 / 30
-    // (0.07), 2000 269 / 150 / 106 (0.23), 4096 with 16 blocks 544 / 293 / 193 (0.45);  12000 1798 / 881 / 1023 (0.86),
-    // 32768 5193 / 4600 / 5476 (0.86), 4096 with 4 KV heads 576 / 559 / 743 (0.89), four of ~3100 tokens
-    // 536 / 474 / 592 (1.35), 9001 + 4096 + 3283 1359 / 1035 / 1312 (1.57);  65536 in four 9300 / 10000 / 12100 (2.3),
-    // 16380 with 4 KV heads 2960 / 3330 / 4040 (3.1).
-    const int64_t per_octet = min(k_blocks / 2 + 1, fwd_mask != nullptr ? 64 : INT_MAX);
-    const int64_t per_sm = total_q * heads_k * per_octet / kNumSMs;      // (in tokens, like the longest walk)
-    const int split = per_sm >= 2 * (int64_t)max_seqlen_q ? 1 : 2 * per_sm >= max_seqlen_q ? 2 : 4;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)split;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)batch * (unsigned)split, heads_k, k_blocks);
-    cfg.blockDim = dim3(kDkvThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, sparse_attn_bwd_dkv_kernel, map_q, map_do, map_k, map_v, p, split);
-    if (e != cudaSuccess) return set_error((int)e, "sparse_attn_bwd_dkv: %s", cudaGetErrorString(e));
+    dim3 grid(batch, heads_k, k_blocks);
+    sparse_attn_bwd_dkv_kernel<<<grid, kDkvThreads, smem, st>>>(map_q, map_do, map_k, map_v, p);
     rc = check_launch("sparse_attn_bwd_dkv");
     if (rc) return rc;
   }

@@ -1,6 +1,6 @@
 // Blackwell (sm_100a) primitives as inline PTX: mbarrier, TMA tiled loads, tcgen05 MMA with
 // TMEM accumulators, and the shared-memory / instruction descriptors they take.
-// No multicast anywhere: every CTA fetches its own tiles.  The one cluster launch (dK / dV) exchanges sums.
+// No cluster launch and no multicast anywhere: every CTA fetches its own tiles.
 #pragma once
 #include <cuda.h>          // CUtensorMap (types only; the encoder is looked up at run time)
 #include "common.cuh"
@@ -449,21 +449,6 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                    smem_u32(bar))
                : "memory");
-}
-
-// ------------------------------------------------------------------ clusters -----------------
-// Every thread of every CTA of the cluster; orders their shared-memory accesses, each other's included.
-__device__ __forceinline__ void cluster_sync() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// 16 bytes into the shared memory of the cluster's CTA `rank`, at the place that has address `at` in this CTA's
-__device__ __forceinline__ void st_cluster_v4(uint32_t at, uint32_t rank, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile(
-      "{\n\t.reg .b32 r;\n\tmapa.shared::cluster.u32 r, %0, %1;\n\t"
-      "st.shared::cluster.v4.b32 [r], {%2, %3, %4, %5};\n\t}"
-      ::"r"(at), "r"(rank), "r"(a), "r"(b), "r"(c), "r"(d)
-      : "memory");
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {

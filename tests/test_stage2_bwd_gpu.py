@@ -133,14 +133,49 @@ def test_bwd_second_order_is_refused():
 
 
 @pytest.mark.parametrize("lens,k_sel,dense", [
-    ([64] * 148 + [5], 1, False),     # many short sequences: one CTA a block
-    ([64] * 74, 1, False),            # two share a block's octets
-    ([700, 9], 4, False),             # four
-    ([520], 0, True), ([15], 0, True),   # four, of which some have fewer steps than others or none
+    ([64] * 148 + [5], 1, False), ([64] * 74, 1, False), ([700, 9], 4, False), ([520], 0, True), ([15], 0, True),
 ])
-def test_bwd_octets_of_a_block_shared_by_a_cluster(lens, k_sel, dense):
-    # dK / dV: how many CTAs share a key block follows from the sizes; the partial sums are exchanged in a
-    # fixed order
+def test_bwd_many_short_and_few_sequences(lens, k_sel, dense):
     a = _check(lens, lens, k_sel, True, dense=dense, seed=40)
     b = _check(lens, lens, k_sel, True, dense=dense, seed=40)
     assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("length", [15, 700, 1501])
+def test_bwd_gradients_of_a_sequence_do_not_depend_on_the_rest_of_the_call(length, dense):
+    # bit for bit the same alone, in a batch, for one KV head of several, and with a loose max_seqlen_q
+    hk, k_sel = 2, 4
+    rest = [64] * 40, [1600, 3]
+    q, k, v, do = (det_tensor((length, n, 128), 50 + i, s) for i, (n, s) in enumerate(((hk * 16, 0.25), (hk, 0.25), (hk, 1.0),
+                                                                                       (hk * 16, 0.5))))
+    idx = None if dense else local_topk(hk, [length], [length], k_sel, 8)
+
+    def grads(before, after, heads, loose):
+        lens = before + [length] + after
+        at, n = sum(before), sum(lens)
+        x = [det_tensor((n, t.shape[1], 128), 60 + i, 0.25) for i, t in enumerate((q, k, v, do))]
+        for full, t in zip(x, (q, k, v, do)):
+            full[at:at + length] = t
+        x = [t[:, h.start * t.shape[1] // hk:h.stop * t.shape[1] // hk].contiguous().to(DEV) for t, h in zip(x, [heads] * 4)]
+        i = None
+        if not dense:
+            i = local_topk(hk, lens, lens, k_sel, 9)
+            i[:, at:at + length] = idx
+            i = i[heads].contiguous().to(DEV)
+        for t in x[:3]:
+            t.requires_grad_(True)
+        out = infllm_v2.infllmv2_attn_varlen_func(x[0], x[1], x[2], cu(lens, DEV), cu(lens, DEV), max(lens) * loose,
+                                                  max(lens), causal=True, topk_idx=i)
+        g = torch.autograd.grad(out, x[:3], x[3])
+        infllm_v2.check_device_status()
+        return [t[at:at + length] for t in g]
+
+    both = slice(0, hk)
+    want = grads([], [], both, 1)
+    for args in ((*rest, both, 1), ([], [], both, 5), (rest[1], rest[0], both, 3)):
+        assert all(torch.equal(a, b) for a, b in zip(grads(*args), want))
+    for h in range(hk):
+        for a, b in zip(grads([], [], slice(h, h + 1), 1), want):
+            n = b.shape[1] // hk
+            assert torch.equal(a, b[:, h * n:(h + 1) * n])
