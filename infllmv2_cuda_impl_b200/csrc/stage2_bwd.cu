@@ -201,9 +201,7 @@ sparse_attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap map_q,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  // (read through a warp broadcast: it tells the compiler that the value is warp-uniform, so the
-  //  MMA issuer's descriptor arithmetic stays in uniform registers instead of being moved there
-  //  operand by operand for every MMA)
+  // (warp broadcasts: they tell the compiler that loop bounds and TMEM addresses are warp-uniform)
   const int n_blocks = __shfl_sync(0xFFFFFFFFu, sm.n_blocks, 0);
   const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, sm.tmem_base, 0);
   const uint32_t tmem_dq = tmem + 256;             // [0,128) buffer 0: S | dP, [128,256) buffer 1

@@ -151,9 +151,7 @@ sparse_attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q,
   __syncthreads();
   tc_fence_after();
 
-  // (warp reductions and broadcasts: they tell the compiler that the values are warp-uniform, so the
-  //  MMA issuer's descriptor arithmetic stays in uniform registers instead of being moved there
-  //  operand by operand for every MMA)
+  // (warp reductions and broadcasts: they tell the compiler that loop bounds and TMEM addresses are warp-uniform)
   int n_blocks = 0;
   for (int w = lane; w < words; w += 32) n_blocks += __popcll(sm.umask[w]);
   n_blocks = __reduce_add_sync(0xFFFFFFFFu, n_blocks);
