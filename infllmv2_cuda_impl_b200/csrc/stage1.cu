@@ -1,10 +1,11 @@
 // Stage-1 scorer: group-summed softmax probabilities of the queries against the compressed keys,
 // optionally max-pooled to 64-token block scores in the same kernel.
 //
-// A CTA (one per SM) works on items of 16 consecutive tokens x the 16 query heads of one KV head, one item or, where
-// the sequences are short, one after the other: two 128-row query tiles A and B, each fetched by 3-D TMA boxes from the caller's (token, head, d) layout, and
-// streams 128-key tiles of the compressed keys twice through a 4-slot ring.  Every key tile serves
-// both query tiles, which halves the L2 -> SM key traffic per score against an 8-token CTA:
+// A CTA (one per SM) works on items of 16 consecutive tokens x the 16 query heads of one KV head, on one item or,
+// where the sequences are short, on one after the other: two 128-row query tiles A and B, each fetched by 3-D TMA
+// boxes from the caller's (token, head, d) layout.  It streams 128-key tiles of the compressed keys twice through
+// a 4-slot ring.  Every key tile serves both query tiles, which halves the L2 -> SM key traffic per score against
+// an 8-token CTA:
 //   pass 1:  S = Q_t . Kc^T  (rows = query rows of tile t in TMEM lanes) -> reference point m
 //            and sum l per row
 //   pass 2:  S^T = Kc . Q_t^T  (rows = keys in TMEM lanes)

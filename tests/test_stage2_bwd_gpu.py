@@ -133,9 +133,14 @@ def test_bwd_second_order_is_refused():
 
 
 @pytest.mark.parametrize("lens,k_sel,dense", [
-    ([64] * 148 + [5], 1, False), ([64] * 74, 1, False), ([700, 9], 4, False), ([520], 0, True), ([15], 0, True),
+    ([64] * 148 + [5], 1, False),     # many short sequences: one CTA a block
+    ([64] * 74, 1, False),            # two share a block's octets
+    ([700, 9], 4, False),             # four
+    ([520], 0, True), ([15], 0, True),   # four, of which some have fewer steps than others or none
 ])
-def test_bwd_many_short_and_few_sequences(lens, k_sel, dense):
+def test_bwd_octets_of_a_block_shared_by_a_cluster(lens, k_sel, dense):
+    # dK / dV: how many CTAs share a key block follows from the sizes; the partial sums are exchanged in a
+    # fixed order
     a = _check(lens, lens, k_sel, True, dense=dense, seed=40)
     b = _check(lens, lens, k_sel, True, dense=dense, seed=40)
     assert all(torch.equal(x, y) for x, y in zip(a, b))
