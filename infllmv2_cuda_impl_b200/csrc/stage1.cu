@@ -267,7 +267,11 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   // an earlier CTA of this launch gave up on a wait: do not pile up more waits
   if (kStay ? __syncthreads_or(failed != 0) : failed != 0) return;
   // (kStay: nothing of this item is used)
-  const Item own(p, kStay ? 0 : walk.b, kStay ? 0 : h, kStay ? 0 : tile16);
+  Item own(p, kStay ? 0 : walk.b, kStay ? 0 : h, kStay ? 0 : tile16);
+  if (!kStay) {                                  // (a warp broadcast tells the compiler that the loop bounds are warp-uniform)
+    own.n_tiles1 = __shfl_sync(0xFFFFFFFFu, own.n_tiles1, 0);
+    own.n_steps = __shfl_sync(0xFFFFFFFFu, own.n_steps, 0);
+  }
 
   // copies for the copy warp's lane 0: Q tile `tile` of an item, and the key tile of its step t into ring slot s
   auto fetch_q = [&](const Item& w, int tile) {
@@ -372,9 +376,14 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     }
   } else if (warp <= 2) {
     // ================================================================ MMA issuer of query tile hq
-    // One elected thread runs the whole loop.
-    if (elect_one()) {
-      const int hq = warp - 1;
+    // Staying CTAs: one elected thread runs the whole loop.  One item a CTA: all 32 lanes run it, and `leader` enables
+    // the MMAs and commits in one of them (its long walks lose to an elected thread and to step counts that are not
+    // known to be warp-uniform).  Block scores, elected / all lanes, us:  the last 4096 of 131072 tokens (8 KV heads)
+    // 2628 / 2611, the last 32768 of 65536 (2 KV heads) 2181 / 2168, 49152 1852 / 1844;  staying, 9001 + 4096 + 3283
+    // tokens 176 / 180, 32768 866 / 876.
+    if (!kStay || elect_one()) {
+      const uint32_t leader = (kStay || lane == 0) ? 1u : 0u;
+      const int hq = kStay ? warp - 1 : __shfl_sync(0xFFFFFFFFu, warp - 1, 0);
       constexpr uint32_t idesc = umma_idesc_bf16(128, 128, false);
       constexpr uint32_t kStage = (2 * kHalfBytes) >> 4;      // descriptor address units per ring stage
       const uint32_t q_lo = umma_desc_lo(smem_u32(sm.q[0][0]), 16) + (uint32_t)hq * kStage;
@@ -391,6 +400,7 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
           break;
         }
         ok = mbar_wait(&sm.q_full[hq], (uint32_t)(it & 1), abort_flag, p.status, 51);
+        if (!kStay) ok = __all_sync(0xFFFFFFFFu, ok);
         for (int t = 0; t < w.n_steps && ok; ++t, ++u) {
           const int s = u % kStages, ab = u & 1;
           const bool pass2 = t >= w.n_tiles1;
@@ -398,6 +408,7 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
           if (ok && u >= 2)
             ok = mbar_wait(&sm.acc_empty[hq][ab], (uint32_t)(((u >> 1) & 1) ^ 1), abort_flag, p.status, 53);
           if (ok && t == w.n_tiles1) ok = mbar_wait(&sm.rowc_ready[hq], (uint32_t)(it & 1), abort_flag, p.status, 54);
+          if (!kStay) ok = __all_sync(0xFFFFFFFFu, ok);
           if (!ok) break;
           tc_fence_after();
           const uint32_t kc_lo = kc_lo0 + (uint32_t)s * kStage;
@@ -406,11 +417,11 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
             const uint32_t off = ((kk >> 2) * kHalfBytes + (kk & 3) * 32) >> 4;
-            umma_ss_lo(acc, a_lo + off, b_lo + off, idesc, kk > 0);
+            umma_ss_lo_pred(acc, a_lo + off, b_lo + off, idesc, kk > 0, leader);
           }
-          if (pass2) umma_ss(acc, d_ones, d_rowc, idesc, true);   // + row constant
-          umma_commit(&sm.kc_free[s]);
-          umma_commit(&sm.acc_full[hq][ab]);
+          if (pass2) umma_ss_pred(acc, d_ones, d_rowc, idesc, true, leader);   // + row constant
+          umma_commit_pred(&sm.kc_free[s], leader);
+          umma_commit_pred(&sm.acc_full[hq][ab], leader);
           if (kStay && t == w.n_steps - 1) umma_commit(&sm.q_free[hq]);
         }
         if (!kStay) break;
