@@ -769,17 +769,25 @@ int launch_stage1(const void* q, const void* kc, const void* kv, void* out, void
   p.status = status;
 
   const size_t smem = sizeof(Smem) + 1024;
-  // CTAs that stay on their SM pay where a walk is short and lose on long ones: their loops spill two to five registers,
-  // and the SMs' speeds differ more than a fixed deal allows.  Block scores with 2 KV heads, one item a CTA / staying,
-  // us:  4096 tokens 53 / 49, 9001 + 4096 + 3283 213 / 174, 16384 + 8192 + 5001 + 2053 502 / 422, 32768 (2047 keys)
-  // 911 / 862, 49152 1841 / 1800, 65536 3096 / 3077, 98304 6577 / 6608, 131072 11330 / 11470;  4096 tokens against 1024 keys
-  // 125 / 123, 2048 217 / 219, 4096 401 / 410, 8192 758 / 776.  The line is where both kinds of call meet.  Nothing can
-  // overlap where no CTA would get a second item (300 tokens 16.3 / 18.3, 1000 18.3 / 20.3) or no item has a step
-  // (without keys; 2000 x 16 tokens 129 / 139).
+  // CTAs that stay on their SM pay where walks are short and items many, and lose where walks are long: their loops spill
+  // two to five registers, and the SMs' speeds differ more than a fixed deal allows.  The mean walk of an item is
+  // max_seqlen_k less half of the keys that the queries themselves bring.  Block scores, one item a CTA / staying, us,
+  // with the mean walk in keys and the items per SM:  2 KV heads, 4096 tokens 55 / 51 (127, 3.5), 9001 + 4096 + 3283
+  // 218 / 180, 16384 + 8192 + 5001 + 2053 510 / 414, 32768 928 / 881 (1023, 28), 49152 1858 / 1826 (1535, 42), 65536
+  // 3102 / 3098 (2047, 55), 98304 6547 / 6635 (3071, 83), 131072 11315 / 11618;  the last 2048 tokens of 16384 76 / 76
+  // (960, 1.7), of 24576 100 / 102 (1472, 1.7), the last 4096 of 8192 84 / 80 (384, 3.5), of 16384 133 / 131 (896, 3.5),
+  // of 24576 180 / 181 (1408, 3.5), of 32768 227 / 231 (1920, 3.5), the last 8192 of 24576 291 / 285 (1280, 7), of 32768
+  // 374 / 373 (1792, 7);  8 KV heads, the last 4096 of 24576 596 / 588 (1408, 14), of 32768 757 / 761 (1920, 14), the last
+  // 16384 of 32768 2422 / 2396 (1536, 55).  Where most tiles of the other grid would be empty, missing them outweighs
+  // that: 2047 keys each, 4096 + 1 x 3 tokens 242 / 230, 4096 + 1 x 100 604 / 292, 1024 x 4 + 1 x 28 287 / 238;  4096 + 2048 +
+  // 1024 + 512, twice as many tiles as real ones, 393 / 394.  Nothing can overlap where no CTA would get a second item (300 tokens
+  // 16.4 / 18.4, 1000 18.4 / 20.5) or no item has a step (without keys).
   const int64_t even = (int64_t)p.max_tiles * batch, found = total_q / kTokPerCta + batch;
   const int64_t n_items = (even <= found ? even : found) * heads_k;
   p.numbering = even <= found ? kEven : 4 * n_items >= (int64_t)batch * kNumSMs ? kAddUp : kSearch;
-  const bool stay = max_seqlen_k > 0 && max_seqlen_k <= 2048 && even * heads_k > kNumSMs && n_items < (1 << 30);
+  const int64_t own_half = causal ? min((int64_t)max_seqlen_q, total_q) / 32 : 0;
+  const int64_t most = even > 2 * found ? 2048 : n_items > 4 * kNumSMs ? 1536 : 1024;
+  const bool stay = max_seqlen_k > 0 && max_seqlen_k - own_half <= most && even * heads_k > kNumSMs && n_items < (1 << 30);
   p.n_items = (int)n_items;
   const dim3 grid = stay ? dim3((unsigned)(n_items < kNumSMs ? n_items : kNumSMs))
                          : dim3((unsigned)p.max_tiles, (unsigned)batch, (unsigned)heads_k);

@@ -339,3 +339,20 @@ def test_numbering_of_the_items(lens):
     a, b = (infllm_v2.infllmv2_attn_stage1(q, kc, kc, cu_q, cu_k, cu_k, max(lens), m, causal=False) for m in (3, 2049))
     infllm_v2.check_device_status()
     assert torch.equal(a[:, :n], b[:, :n, :3]) and (a[:, :n].float().sum(-1) - 16).abs().max() < 0.25
+
+
+@pytest.mark.parametrize("lens,keys,hk", [
+    ([2048], 1088, 2), ([2048], 1089, 2), ([5008], 1692, 2), ([5008], 1693, 2), ([49152], 3071, 1),
+    ([2400, 1, 1], 2123, 2), ([2400, 1, 1], 2124, 2),
+])
+def test_scores_on_both_sides_of_the_line_of_staying_ctas(lens, keys, hk):
+    # whether CTAs stay follows from the mean walk (at most 1024 keys, with more than 4 items per SM 1536, 2048 where most
+    # tiles would be empty) and never shows in the results: a loose max_seqlen_k takes one item a CTA
+    q = det_tensor((sum(lens), hk * 16, 128), 41, 0.5).to(DEV)
+    kc = det_tensor((keys * len(lens), hk, 128), 42, 0.5).to(DEV)
+    cu_q, cu_k = cu(lens, DEV), cu([keys] * len(lens), DEV)
+    cache = 16 * keys + 16 - max(lens)
+    a, b = (infllm_v2.infllmv2_stage1_block_scores(q, kc, cu_q, cu_k, max(lens), m, 1, 1, cache_len=cache, max_cache_len=cache,
+                                                   causal=True) for m in (keys, 5000))
+    infllm_v2.check_device_status()
+    assert torch.equal(a, b) and a.isfinite().any()
