@@ -245,9 +245,9 @@ struct ItemWalk {
 // kStay: one CTA per SM takes items until there are none, and every barrier, ring slot and accumulator buffer
 // runs on across them, so that an item's keys and Q arrive, and its first products run, while the softmax warps
 // finish the item before.  (u: steps since the start of the kernel, it: items with steps.)  Against one CTA an item
-// that saves 1-3 us an item (block scores, 2 KV heads: 16 x 2048 tokens, 28 items per SM, 256 -> 197 us; 4 x 8192, 28
-// items, 414 -> 358; 16384, 14 items, 301 -> 264; 4096, 3.5 items, 53 -> 49), and in ragged batches 0.8 us of an SM
-// for every CTA of the other grid that finds no tile (4000 x 3 and 8000 tokens, 27000 per SM: 22.4 ms -> 285 us).
+// that saves 1-3 us an item (block scores, 2 KV heads: 16 x 2048 tokens, 28 items per SM, 264 -> 201 us; 4 x 8192, 28
+// items, 426 -> 365; 16384, 14 items, 311 -> 277; 4096, 3.5 items, 55 -> 51), and in ragged batches 0.8 us of an SM
+// for every CTA of the other grid that finds no tile (4000 x 3 and 8000 tokens, 27000 per SM: 22.2 ms -> 289 us).
 template <bool kPooled, bool kStay>
 __global__ void __launch_bounds__(kThreads, 1)      // 19 warps: at most 96 registers per thread
 stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_kc,
@@ -379,8 +379,7 @@ stage1_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     // Staying CTAs: one elected thread runs the whole loop.  One item a CTA: all 32 lanes run it, and `leader` enables
     // the MMAs and commits in one of them (its long walks lose to an elected thread and to step counts that are not
     // known to be warp-uniform).  Block scores, elected / all lanes, us:  the last 4096 of 131072 tokens (8 KV heads)
-    // 2628 / 2611, the last 32768 of 65536 (2 KV heads) 2181 / 2168, 49152 1852 / 1844;  staying, 9001 + 4096 + 3283
-    // tokens 176 / 180, 32768 866 / 876.
+    // 2628 / 2611, the last 32768 of 65536 (2 KV heads) 2181 / 2168, 49152 1852 / 1844;  staying, all lanes are 1-2 % slower.
     if (!kStay || elect_one()) {
       const uint32_t leader = (kStay || lane == 0) ? 1u : 0u;
       const int hq = kStay ? warp - 1 : __shfl_sync(0xFFFFFFFFu, warp - 1, 0);
